@@ -234,6 +234,95 @@ std::vector<double> csc_dense(const sse_csc &A, int rows, int cols) {
   return out;
 }
 
+
+// Fixed-point pair tables (KernelArgs::fx) from the FP64 ones: volume pairs
+// ordered by the directions in which S is nonzero, each pair's S / 2 or C / 2
+// as integers with its own factor 2^k, and the incidence lists with k.
+int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vector<double> &vp_S,
+                   const std::vector<double> &C, const std::vector<int> &qflat, const std::vector<int> &fflat) {
+  KernelArgs &ka = s->ka;
+  const int d = s->cfg.d, nq = s->cfg.n_q, nvp = (int)vp_ij.size();
+  auto largest = [](const double *v, size_t n) {
+    double m = 0.0;
+    for (size_t t = 0; t < n; ++t) m = std::isfinite(v[t]) ? std::max(m, std::fabs(v[t])) : INFINITY;
+    return m;
+  };
+  // e with |v / 2| < 2^e
+  auto exponent = [](double m) { return m > 0.0 ? std::ilogb(m) : -1000; };
+  const double mS = largest(vp_S.data(), vp_S.size()), mC = largest(C.data(), C.size());
+  // (pair numbers take 23 bits of the incidence words)
+  if (!(mS > 1e-60 && mS < 1e60) || !(mC < 1e60) || nvp >= 1 << 23 || C.size() >= (size_t)1 << 23) return SSE_OK;
+  FxTables fx{};
+  fx.eS = exponent(mS);
+  fx.eC = mC > 1e-60 ? exponent(mC) : 0;
+  std::vector<int> order(nvp), mask(nvp, 0);
+  for (int t = 0; t < nvp; ++t) {
+    order[t] = t;
+    for (int m = 0; m < d; ++m) mask[t] |= (vp_S[(size_t)t * d + m] != 0.0) << m;
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return mask[a] > mask[b]; });
+  std::vector<int> ij(nvp), inc_flat, inc_ptr(nq + 1, 0);
+  std::vector<Fx> S((size_t)nvp * d), Cx(C.size());
+  std::vector<std::vector<int>> inc(nq);
+  for (int t = 0; t < nvp; ++t) {
+    const double *v = &vp_S[(size_t)order[t] * d];
+    const int k = std::min(kFxMaxK, fx.eS - exponent(largest(v, d)));
+    ij[t] = vp_ij[order[t]];
+    inc[ij[t] & 0xffff].push_back(t << 8 | k << 1 | 1);
+    inc[ij[t] >> 16].push_back(t << 8 | k << 1);
+    for (int m = 0; m < d; ++m) S[(size_t)t * d + m] = fx_split_near(fx_from_double(0.5 * v[m], fx.eS - k));
+  }
+  for (int i = 0; i < nq; ++i) {
+    inc_flat.insert(inc_flat.end(), inc[i].begin(), inc[i].end());
+    inc_ptr[i + 1] = (int)inc_flat.size();
+  }
+  std::vector<int> kC(C.size());
+  for (size_t t = 0; t < C.size(); ++t) {
+    kC[t] = std::min(kFxMaxK, fx.eC - exponent(std::fabs(C[t])));
+    Cx[t] = fx_split_near(fx_from_double(0.5 * C[t], fx.eC - kC[t]));
+  }
+  std::vector<int> q(qflat), f(fflat);
+  for (int &v : q) v = v << 8 | kC[v] << 1;
+  for (int &v : f) v = v << 8 | kC[v] << 1;
+  cudaError_t e;
+  if ((e = upload(s, ij.data(), ij.size(), &fx.vp_ij)) || (e = upload(s, S.data(), S.size(), &fx.vp_S)) ||
+      (e = upload(s, inc_ptr.data(), inc_ptr.size(), &fx.vp_inc_ptr)) ||
+      (e = upload(s, inc_flat.data(), inc_flat.size(), &fx.vp_inc)))
+    return cuda_fail(s, e, "fixed-point pair tables");
+  if (!C.empty() && ((e = upload(s, Cx.data(), Cx.size(), &fx.fp_C)) || (e = upload(s, q.data(), q.size(), &fx.fp_q)) ||
+                     (e = upload(s, f.data(), f.size(), &fx.fp_f))))
+    return cuda_fail(s, e, "fixed-point pair tables");
+  ka.fx = fx;
+  return SSE_OK;
+}
+
+// Fixed-point metric terms, when they take at most a quarter of the free
+// device memory; without them phase B runs in FP64.
+int setup_fx_geometry(sse_solver *s) {
+  KernelArgs &ka = s->ka;
+  const sse_config &c = s->cfg;
+  const size_t ne = c.n_e, nl = ne * c.n_q * c.d * c.d, nh = ne * c.n_q * c.d * c.num_faces, nf = ne * c.n_f * c.d;
+  size_t freeb = 0, totalb = 0;
+  cudaError_t e;
+  if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
+  if ((nl + nh + 2 * nf) * sizeof(Fx) > freeb / 4) return SSE_OK;
+  void *lam, *hnq, *hnf, *bn, *n, *eG;
+  if ((e = alloc(s, nl * sizeof(Fx), &lam)) || (e = alloc(s, nh * sizeof(Fx), &hnq)) ||
+      (e = alloc(s, nf * sizeof(Fx), &hnf)) || (e = alloc(s, nf * sizeof(Fx), &bn)) ||
+      (e = alloc(s, ne * (c.n_q + c.n_f), &n)) || (e = alloc(s, ne * sizeof(int), &eG)) ||
+      (e = launch_fx_geometry(ka, (Fx *)lam, (Fx *)hnq, (Fx *)hnf, (Fx *)bn, (signed char *)n, (int *)eG, s->stream)) ||
+      (e = cudaStreamSynchronize(s->stream)))
+    return cuda_fail(s, e, "fixed-point metric terms");
+  ka.fx.Lam = (const Fx *)lam;
+  ka.fx.hnq = (const Fx *)hnq;
+  ka.fx.hnf = (const Fx *)hnf;
+  ka.fx.bn = (const Fx *)bn;
+  ka.fx.n = (const signed char *)n;
+  ka.fx.eG = (const int *)eG;
+  ka.fx.on = 1;
+  return SSE_OK;
+}
+
 // The one-kernel StandardForm path (std_compact_kernel): StandardForm on
 // elements with at most 32 volume, facet and modal nodes, each face meeting
 // one neighbour element, with the element's dense weight-adjusted mass
@@ -587,10 +676,11 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     if ((e = upload(s, inc_flat.data(), inc_flat.size(), &op.vp_inc)) != cudaSuccess) return cuda_fail(s, e, "upload");
 
     op.nfp = 0;
+    std::vector<double> fp_C;
+    std::vector<int> qflat, fflat;
     if (has_C) {
       const sse_csc &Cm = ops->C;
       std::vector<int> fp_ij;
-      std::vector<double> fp_C;
       std::vector<std::vector<int>> qinc(c.n_q), finc(c.n_f);
       for (int64_t j = 0; j < Cm.n; ++j)
         for (int64_t q = Cm.colptr[j] - 1; q < Cm.colptr[j + 1] - 1; ++q) {
@@ -601,7 +691,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
           qinc[i].push_back(t);
           finc[j].push_back(t);
         }
-      std::vector<int> qptr(c.n_q + 1, 0), qflat, fptr(c.n_f + 1, 0), fflat;
+      std::vector<int> qptr(c.n_q + 1, 0), fptr(c.n_f + 1, 0);
       for (int i = 0; i < c.n_q; ++i) { qflat.insert(qflat.end(), qinc[i].begin(), qinc[i].end()); qptr[i + 1] = (int)qflat.size(); }
       for (int j = 0; j < c.n_f; ++j) { fflat.insert(fflat.end(), finc[j].begin(), finc[j].end()); fptr[j + 1] = (int)fflat.size(); }
       op.nfp = (int)fp_ij.size();
@@ -618,6 +708,12 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       if ((e = upload(s, fptr.data(), fptr.size(), &op.fp_f_ptr)) != cudaSuccess) return cuda_fail(s, e, "upload");
       if ((e = upload(s, fflat.data(), fflat.size(), &op.fp_f)) != cudaSuccess) return cuda_fail(s, e, "upload");
     }
+    // fixed-point pair tables: the two-point flux and its bounds are those of
+    // fx_ec_flux (gamma <= 1.7)
+    ka.fx = FxTables{};
+    if (c.law == SSE_EULER && c.two_point_flux == SSE_EC_FLUX && c.gamma > 1.0 && c.gamma <= 1.7 &&
+        (rc = setup_fx_pairs(s, vp_ij, vp_S, fp_C, qflat, fflat)))
+      return rc;
   }
 
   // ---- geometry
@@ -727,6 +823,31 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     ka.fd_chunk = chunk;
     ka.vdm_zsz = zsz_e;
     layout(chunk);
+    if (ka.fx.vp_ij) {
+      // the same rule for the fixed-point passes, whose second pass has the
+      // interface fluxes too
+      const int nodes = nq + 2 * nf, pairs = std::max(op.nvp, op.nfp + nf), stride = d == 2 ? kFxStride<2> : kFxStride<3>;
+      auto layout_x = [&](int n) {
+        finish(ka.layBx, {nc * nf, nc * nq, std::max(n * nc, final_scratch), d * d * nq,
+                          op.nfp > 0 ? d * c.num_faces * nq : 0, op.nfp > 0 ? d * nf : 0, nodes * stride, 2 * nodes, 4,
+                          (nq + nf + 7) / 8});
+        return ka.layBx.team_doubles;
+      };
+      int n = pairs;
+      if (layout_x(n) > budget) {
+        const int fixed = layout_x(0) - ((std::max(0, final_scratch) + 1) & ~1);
+        const int cap1 = (int)((size_t)220 * 1024 / 8 / epb_for(tpe));
+        int room = budget - fixed;
+        if (room / nc < std::min(tpe, pairs)) room = cap1 - fixed;
+        n = std::max(1, room / nc);
+        if (n >= tpe) n = n / tpe * tpe;
+        n = std::max(1, std::min(n, pairs));
+      }
+      ka.fx_chunk = n;
+      layout_x(n);
+      // no room for the node values: the FP64 passes
+      if ((size_t)epb_for(tpe) * ka.layBx.team_doubles * 8 > (size_t)220 * 1024) ka.fx = FxTables{};
+    }
     // the interface flux of one facet node costs about 0.8 of a volume pair
     // (block timings at p = 4): balance lanes when all pairs are one chunk.
     // Teams narrower than a warp share warps, and a warp waits for its
@@ -783,7 +904,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   if ((size_t)ka.epb_a * ka.layA.team_doubles * 8 > 220 * 1024) ka.epb_a = epb;
   // opt in to large dynamic shared memory for every kernel instantiation used
   size_t smA = (size_t)std::max(epb, ka.epb_a) * ka.layA.team_doubles * 8,
-         smB = (size_t)epb * ka.layB.team_doubles * 8;
+         smB = (size_t)epb * std::max(ka.layB.team_doubles, ka.fx.vp_ij ? ka.layBx.team_doubles : 0) * 8;
   if ((e = sse_set_smem_limits(ka, smA, smB)) != cudaSuccess) return cuda_fail(s, e, "cudaFuncSetAttribute");
 
   // the weight-adjusted mass operator V' diag(J^-1 W) V of every element,
@@ -802,6 +923,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       ka.Ak = (const double *)p;
     }
   }
+  if (ka.fx.vp_ij && (rc = setup_fx_geometry(s))) return rc;
   return setup_compact(s, ops, mapP);
 }
 

@@ -13,6 +13,8 @@
 //          (standard_form_first_order.jl:1-14, flux_differencing_form.jl:190-292)
 // Phase B  fd_time_derivative_kernel   time_derivative! FD (flux_differencing_form.jl:294-347)
 //          std_time_derivative_kernel  time_derivative! StandardForm (standard_form_first_order.jl:16-63)
+#include <algorithm>
+
 #include "sse_device.cuh"
 #include "sse_kernels.cuh"
 #include "sse_tma.cuh"
@@ -287,20 +289,16 @@ __global__ void __launch_bounds__(256) projection_of_one_kernel(KernelArgs ka, d
 // ---------------------------------------------------------------------------
 // Phase B, FluxDifferencingForm
 // ---------------------------------------------------------------------------
+
+// Volume and facet residuals of one element in FP64: r_q at L.off[3], f_f at
+// L.off[2] of layout ka.layB
 template <int D, int NC>
-__global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) {
-  extern __shared__ double smem[];
+__device__ __forceinline__ void fd_fluxes(const KernelArgs &ka, double *base, int kk, int lane, int tpe) {
   const DevOps &op = ka.op;
   const Physics &ph = ka.ph;
   const Layout &L = ka.layB;
-  const int tpe = blockDim.x / ka.epb;
-  const int team = threadIdx.x / tpe, lane = threadIdx.x % tpe;
-  const int k = blockIdx.x * ka.epb + team;
-  const bool live = k < ka.ne;
-  const int kk = live ? k : 0;
-  const int np = op.np, nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf;
+  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf;
   const float rnpf = qrcp(npf > 0 ? npf : 1);
-  double *base = smem + (size_t)team * L.team_doubles;
   double *uq = base + L.off[0], *uf = base + L.off[1], *ff = base + L.off[2], *rq = base + L.off[3],
          *diff = base + L.off[4], *Lam = base + L.off[5], *hnq = base + L.off[6],
          *prim = base + L.off[7];
@@ -561,14 +559,22 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
       __syncthreads();
     }
   }
+}
 
+// The lift, V^T and the mass solve: dudt of one element from r_q and f_f, with
+// scratch space for the modal and nodal buffers and the sum factorisation
+template <int D, int NC>
+__device__ __forceinline__ void fd_tail(const KernelArgs &ka, double *rq, double *ff, double *scratch, int kk,
+                                        bool live, int lane, int tpe) {
+  const DevOps &op = ka.op;
+  const int np = op.np, nq = op.nq;
   // r_q -= R^T f_f
   rt_apply<double, NC>(op, op.Rt_val, ff, lane, tpe, [&](int t, double v) { rq[t] -= v; });
   __syncthreads();
 
   // dudt = V^T r_q ; mass solve  (the pair buffer is free now: it holds the
   // modal and nodal buffers and the sum-factorisation scratch)
-  double *Xm = diff, *Yq = diff + (size_t)NC * np;
+  double *Xm = scratch, *Yq = scratch + (size_t)NC * np;
   double *Z = Yq + (size_t)NC * nq;
   double *Wb = Z + ka.vdm_zsz;
   vdm_tmul<double, D, NC>(op, rq, Xm, Z, Wb, lane, tpe);
@@ -581,6 +587,504 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
       out[t] = Xm[t];
       if (!isfinite(Xm[t])) ka.flag_nonphysical();
     }
+}
+
+template <int D, int NC>
+__global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) {
+  extern __shared__ double smem[];
+  const int tpe = blockDim.x / ka.epb;
+  const int team = threadIdx.x / tpe, lane = threadIdx.x % tpe;
+  const int k = blockIdx.x * ka.epb + team;
+  const bool live = k < ka.ne;
+  const int kk = live ? k : 0;
+  const Layout &L = ka.layB;
+  double *base = smem + (size_t)team * L.team_doubles;
+  fd_fluxes<D, NC>(ka, base, kk, lane, tpe);
+  fd_tail<D, NC>(ka, base + L.off[3], base + L.off[2], base + L.off[4], kk, live, lane, tpe);
+}
+
+// ---------------------------------------------------------------------------
+// Phase B, FluxDifferencingForm with the entropy-conservative flux (Euler),
+// two-point fluxes in block fixed point (sse_fixed.cuh)
+//
+// The FP64 passes are bound by the FP64 pipe (a p = 4 tet has 155 K FP64
+// instructions, 125 K of them in its 1,750 pairs; the pipe was 79 % busy and
+// the issue slots 10 %).  Here the pairs take none: node values are scaled to
+// integers once per element, the pair passes are integer multiply-adds and
+// FP32, and FP64 is left to the node values, the Lax-Friedrichs term and the
+// tail.  24,576 p = 4 tets: 8.86 -> 3.58 ms; 7,986 p = 5 tets 6.5 -> 2.42 ms;
+// 8,192 p = 4 triangles 0.365 -> 0.184 ms.  The error against the
+// extended-precision residual is 0.81 to 1.00 of the FP64 passes' own on 60
+// configurations (modal and nodal, p = 2 to 6, both metrics and interface
+// fluxes).
+// ---------------------------------------------------------------------------
+
+// FP64 value of a fixed-point sum v 2^e with two FMAs: the words of v as the
+// low bits of two doubles, their offsets taken out by exact FMAs
+struct FxUnit {
+  double lo, hi, off;  // 2^e, 2^(e + 32), their offsets
+  __device__ __forceinline__ explicit FxUnit(int e) {
+    lo = fx_pow2(e);
+    hi = fx_pow2(e + 32);
+    off = -(0x1p84 + 0x1p63 + 0x1p52) * lo;
+  }
+  __device__ __forceinline__ double operator()(long long v) const {
+    const double h = __hiloint2double(0x43300000, (int)(v >> 32) ^ 0x80000000);
+    const double l = __hiloint2double(0x43300000, (int)v);
+    return fma(l, lo, fma(h, hi, off));
+  }
+};
+
+// v 2^-s to the nearest integer, 0 <= s < 63
+struct FxShift {
+  int s;
+  long long half;
+  __device__ __forceinline__ explicit FxShift(int s_) : s(s_), half((1LL << s_) >> 1) {}
+  __device__ __forceinline__ long long operator()(long long v) const { return (v + half) >> s; }
+};
+
+__device__ __forceinline__ void fx_copy_async(Fx *dst, const Fx *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// Exponents of an element's units from the extremes of its node values (upper
+// words of the largest density, enthalpy and |velocity component| and
+// 0x7fffffff less that of the smallest density and enthalpy); ok: positive,
+// finite and within a factor 2^4 to 2^5 of each other
+struct FxScale {
+  int eR, eH, eV;
+  bool ok;
+  __device__ __forceinline__ FxScale(const unsigned *key, int eG) {
+    ok = key[0] < 0x7ff00000u && key[1] < 0x7ff00000u && key[2] < 0x7ff00000u;
+    const int r = fx_exponent(key[0]), h = fx_exponent(key[1]), v = fx_exponent(key[2]);
+    ok = ok && r - fx_exponent(0x7fffffffu - key[3]) <= 4 && h - fx_exponent(0x7fffffffu - key[4]) <= 4;
+    ok = ok && abs(r) < 200 && abs(h) < 200 && v < 200 && eG != kFxNone;
+    eR = r + 1;
+    eV = v + 1;
+    eH = max(h + 1, 2 * eV);
+    eV = max(eV, (eH - 40) >> 1);
+  }
+};
+
+template <int D, int NC>
+__global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs ka) {
+  static_assert(NC == D + 2, "Euler");
+  extern __shared__ double smem[];
+  const DevOps &op = ka.op;
+  const Physics &ph = ka.ph;
+  const FxTables &fx = ka.fx;
+  const Layout &L = ka.layBx;
+  const int tpe = blockDim.x / ka.epb;
+  const int team = threadIdx.x / tpe, lane = threadIdx.x % tpe;
+  const int k = blockIdx.x * ka.epb + team;
+  const bool live = k < ka.ne;
+  const int kk = live ? k : 0;
+  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf;
+  constexpr int PS = kFxStride<D>;
+  double *base = smem + (size_t)team * L.team_doubles;
+  double *ff = base + L.off[0], *rq = base + L.off[1];
+  long long *diff = reinterpret_cast<long long *>(base + L.off[2]);
+  long long *rqi = reinterpret_cast<long long *>(rq);
+  Fx *Lam = reinterpret_cast<Fx *>(base + L.off[3]), *hnq = reinterpret_cast<Fx *>(base + L.off[4]),
+     *hnf = reinterpret_cast<Fx *>(base + L.off[5]), *node = reinterpret_cast<Fx *>(base + L.off[6]);
+  double *noded = base + L.off[6];
+  FxPair *pair = reinterpret_cast<FxPair *>(base + L.off[7]);
+  unsigned *key = reinterpret_cast<unsigned *>(base + L.off[8]);
+  signed char *ns = reinterpret_cast<signed char *>(base + L.off[9]);
+
+  // metric terms, landing while the node values are formed
+  {
+    const Fx *g = fx.Lam + (size_t)kk * nq * D * D;
+    for (int t = lane; t < nq * D * D; t += tpe) fx_copy_async(Lam + t, g + t);
+    if (op.nfp > 0) {
+      g = fx.hnq + (size_t)kk * D * nfac * nq;
+      for (int t = lane; t < D * nfac * nq; t += tpe) fx_copy_async(hnq + t, g + t);
+      g = fx.hnf + (size_t)kk * D * nf;
+      for (int t = lane; t < D * nf; t += tpe) fx_copy_async(hnf + t, g + t);
+    }
+  }
+  for (int t = lane; t < nq + nf; t += tpe) ns[t] = fx.n[(size_t)kk * (nq + nf) + t];
+  if (lane < 5) key[lane] = 0u;
+  // FP64 node values [rho, p, h, V] of the volume nodes, the facet nodes and
+  // the facing nodes of the neighbours; the Lax-Friedrichs term of a facet
+  // node from its two states
+  unsigned k0 = 0u, k1 = 0u, k2 = 0u, k3 = 0u, k4 = 0u;
+  auto store_node = [&](int i, const double *u, double rr) {
+    double *P = noded + (size_t)i * PS;
+    double s = 0.0;
+#pragma unroll
+    for (int m = 0; m < D; ++m) {
+      const double v = u[m + 1] * rr;
+      P[3 + m] = v;
+      s = fma(v, v, s);
+      k2 = max(k2, (unsigned)__double2hiint(v) & 0x7fffffffu);
+    }
+    const double p = ph.gm1 * fma(-0.5 * u[0], s, u[D + 1]);
+    const double h = p * (ph.igm1 * rr);
+    P[0] = u[0];
+    P[1] = p;
+    P[2] = h;
+    const unsigned r = (unsigned)__double2hiint(u[0]), e = (unsigned)__double2hiint(h);
+    k0 = max(k0, r);
+    k1 = max(k1, e);
+    k3 = max(k3, 0x7fffffffu - r);
+    k4 = max(k4, 0x7fffffffu - e);
+  };
+  {
+    const double *uqg = ka.u_q + (size_t)kk * NC * nq;
+    for (int i = lane; i < nq; i += tpe) {
+      double u[NC];
+#pragma unroll
+      for (int e = 0; e < NC; ++e) u[e] = uqg[e * nq + i];
+      store_node(i, u, sse_rcp(u[0]));
+    }
+    const double *ufg = ka.u_f + (size_t)kk * NC * nf;
+    for (int j = lane; j < nf; j += tpe) {
+      const int P = ka.geo.mapP[(size_t)kk * nf + j];
+      const int jn = P % nf, kn = P / nf;
+      double ui[NC], uo[NC];
+#pragma unroll
+      for (int e = 0; e < NC; ++e) {
+        ui[e] = ufg[e * nf + j];
+        uo[e] = ka.u_f[((size_t)kn * NC + e) * nf + jn];
+      }
+      const double ri = sse_rcp(ui[0]), ro = sse_rcp(uo[0]);
+      store_node(nq + j, ui, ri);
+      store_node(nq + nf + j, uo, ro);
+      if (ph.nflux == 0) {
+        const double *Pi = noded + (size_t)(nq + j) * PS, *Po = noded + (size_t)(nq + nf + j) * PS;
+        double vni = 0.0, vno = 0.0;
+#pragma unroll
+        for (int m = 0; m < D; ++m) {
+          const double n = ka.geo.n_f[m + D * (j + (size_t)nf * kk)];
+          vni = fma(Pi[3 + m], n, vni);
+          vno = fma(Po[3 + m], n, vno);
+        }
+        const double c = sqrt(ph.gamma * fmax(Pi[1] * ri, Po[1] * ro));
+        const double a = ph.half_lambda * (fmax(fabs(vni), fabs(vno)) + c) * ka.geo.BJf[(size_t)kk * nf + j];
+#pragma unroll
+        for (int e = 0; e < NC; ++e) ff[e * nf + j] = a * (ui[e] - uo[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) ff[e * nf + j] = 0.0;
+      }
+    }
+  }
+  const int width = tpe < 32 ? tpe : 32;
+  for (int o = width >> 1; o > 0; o >>= 1) {
+    k0 = max(k0, __shfl_xor_sync(0xffffffffu, k0, o));
+    k1 = max(k1, __shfl_xor_sync(0xffffffffu, k1, o));
+    k2 = max(k2, __shfl_xor_sync(0xffffffffu, k2, o));
+    k3 = max(k3, __shfl_xor_sync(0xffffffffu, k3, o));
+    k4 = max(k4, __shfl_xor_sync(0xffffffffu, k4, o));
+  }
+  __syncthreads();  // key cleared
+  if ((lane & (width - 1)) == 0) {
+    atomicMax(key + 0, k0);
+    atomicMax(key + 1, k1);
+    atomicMax(key + 2, k2);
+    atomicMax(key + 3, k3);
+    atomicMax(key + 4, k4);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const int eG = fx.eG[kk];
+  const FxScale sc(key, eG);
+  // a block with an element out of range runs in FP64 as a whole
+  if (!__syncthreads_and(sc.ok)) {
+    double *b64 = smem + (size_t)team * ka.layB.team_doubles;
+    fd_fluxes<D, NC>(ka, b64, kk, lane, tpe);
+    fd_tail<D, NC>(ka, b64 + ka.layB.off[3], b64 + ka.layB.off[2], b64 + ka.layB.off[4], kk, live, lane, tpe);
+    return;
+  }
+  const int kappa = sc.eH - 2 * sc.eV, eP = sc.eR + sc.eH - 2;
+  // node values in the element's units, each by the thread that wrote it
+  auto convert = [&](int i) {
+    Fx v[kFxNode<D>];
+    const double *P = noded + (size_t)i * PS;
+    v[0] = fx_split_near(fx_from_double(P[0], sc.eR));
+    v[1] = fx_split_near(fx_from_double(P[1], eP));
+    v[2] = fx_split_near(fx_from_double(P[2], sc.eH));
+#pragma unroll
+    for (int m = 0; m < D; ++m) v[3 + m] = fx_split_near(fx_from_double(P[3 + m], sc.eV));
+    FxPair f;
+    fx_two_floats(v[0], &f.rh, &f.rl);
+    fx_two_floats(v[2], &f.hh, &f.hl);
+    pair[i] = f;
+#pragma unroll
+    for (int m = 0; m < kFxNode<D>; ++m) node[(size_t)i * PS + m] = v[m];
+  };
+  for (int i = lane; i < nq; i += tpe) convert(i);
+  for (int j = lane; j < nf; j += tpe) {
+    convert(nq + j);
+    convert(nq + nf + j);
+  }
+  __syncthreads();
+
+  // volume flux differencing: pass 1 one flux per pair, pass 2 each node's sum
+  // over its pairs (as fd_fluxes, in integers)
+  const int CH = ka.fx_chunk;
+  int cur[kMaxNodeSlots];
+#pragma unroll
+  for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
+    const int i = lane + sl * tpe;
+    cur[sl] = i < nq ? fx.vp_inc_ptr[i] : 0;
+    if (i < nq)
+#pragma unroll
+      for (int e = 0; e < NC; ++e) rqi[e * nq + i] = 0;
+  }
+  for (int c0 = 0; c0 < op.nvp; c0 += CH) {
+    const int c1 = min(op.nvp, c0 + CH);
+    for (int p = c0 + lane; p < c1; p += tpe) {
+      const int ij = fx.vp_ij[p];
+      const int i = ij & 0xffff, j = ij >> 16;
+      FxDot s[D];
+      long long h[D];
+#pragma unroll
+      for (int n = 0; n < D; ++n) { s[n].x = 0; h[n] = 0; }
+#pragma unroll
+      for (int m = 0; m < D; ++m) {
+        const Fx S = fx.vp_S[(size_t)p * D + m];
+        if ((S.lo | S.hi) == 0) continue;
+#pragma unroll
+        for (int n = 0; n < D; ++n) {
+          const Fx l = fx_add(Lam[i + nq * (m + D * n)], Lam[j + nq * (m + D * n)]);
+          s[n].cross(S, l);
+          h[n] = fx_wide(S.hi, l.hi, h[n]);
+        }
+      }
+      Fx G[D];
+#pragma unroll
+      for (int n = 0; n < D; ++n) G[n] = fx_split(h[n] + (s[n].x >> kFxLow));
+      long long out[NC];
+      fx_ec_flux<D>(node + (size_t)i * PS, node + (size_t)j * PS, pair[i], pair[j], G, kappa, out);
+      long long *dp = diff + (size_t)(p - c0) * NC;
+#pragma unroll
+      for (int e = 0; e < NC; ++e) dp[e] = out[e];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
+      const int i = lane + sl * tpe;
+      if (i >= nq) continue;
+      long long acc[NC];
+#pragma unroll
+      for (int e = 0; e < NC; ++e) acc[e] = rqi[e * nq + i];
+      int q = cur[sl];
+      const int qe = fx.vp_inc_ptr[i + 1];
+      for (; q < qe; ++q) {
+        const int inc = fx.vp_inc[q];
+        const int p = inc >> 8;
+        if (p >= c1) break;
+        const FxShift down((inc >> 1 & 127) - ns[i]);
+        const long long *dp = diff + (size_t)(p - c0) * NC;
+        // r_q[i] += -diff if i is the pair's first node, +diff otherwise
+#pragma unroll
+        for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
+      }
+      cur[sl] = q;
+#pragma unroll
+      for (int e = 0; e < NC; ++e) rqi[e * nq + i] = acc[e];
+    }
+    __syncthreads();
+  }
+
+  const FxUnit um(sc.eR + eG + sc.eV - 63), up(eP + eG - 61), ue(eP + eG + sc.eV - 61);
+  // a sum of node t (its unit 2^-n_t smaller) in FP64
+  auto value = [&](int t, int e, long long v) {
+    const double x = e == 0 ? um(v) : (e == D + 1 ? ue(v) : up(v));
+    return v == 0 ? 0.0 : sse_from_bits(sse_bits(x) - ((long long)ns[t] << 52));
+  };
+  // facet correction and interface flux, chunked the same way; the sums are
+  // subtracted from r_q (integers) and f_f (converted, FP64)
+  const float rnpf = qrcp(npf > 0 ? npf : 1);
+#pragma unroll
+  for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
+    const int t = lane + sl * tpe;
+    cur[sl] = op.nfp == 0 ? 0 : (t < nq ? op.fp_q_ptr[t] : (t < nq + nf ? op.fp_f_ptr[t - nq] : 0));
+  }
+  // the pairs nfp .. nfp + nf - 1 are the facet nodes with their facing nodes
+  const int nall = op.nfp + nf;
+  for (int c0 = 0; c0 < nall; c0 += CH) {
+    const int c1 = min(nall, c0 + CH);
+    for (int p = c0 + lane; p < c1; p += tpe) {
+      Fx G[D];
+      int i, j;
+      if (p < op.nfp) {
+        const int ij = op.fp_ij[p];
+        i = ij & 0xffff;
+        const int jf = ij >> 16;
+        j = nq + jf;
+        const int f = qdiv(jf, rnpf);
+        const Fx C = fx.fp_C[p];
+#pragma unroll
+        for (int m = 0; m < D; ++m)
+          G[m] = fx_split(fx_mul(C, fx_add(hnf[m + D * jf], hnq[(f * D + m) * nq + i])));
+      } else {
+        i = nq + p - op.nfp;
+        j = i + nf;
+#pragma unroll
+        for (int m = 0; m < D; ++m) G[m] = fx.bn[m + D * ((i - nq) + (size_t)nf * kk)];
+      }
+      long long out[NC];
+      fx_ec_flux<D>(node + (size_t)i * PS, node + (size_t)j * PS, pair[i], pair[j], G, kappa, out);
+      long long *dp = diff + (size_t)(p - c0) * NC;
+#pragma unroll
+      for (int e = 0; e < NC; ++e) dp[e] = out[e];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
+      const int t = lane + sl * tpe;
+      if (t >= nq + nf) continue;
+      long long acc[NC];
+#pragma unroll
+      for (int e = 0; e < NC; ++e) acc[e] = 0;
+      const bool vol = t < nq;
+      const int r = vol ? t : t - nq;
+      if (op.nfp > 0) {
+        const int *lst = vol ? fx.fp_q : fx.fp_f;
+        const int qe = vol ? op.fp_q_ptr[r + 1] : op.fp_f_ptr[r + 1];
+        int q = cur[sl];
+        for (; q < qe; ++q) {
+          const int p = lst[q] >> 8;
+          if (p >= c1) break;
+          const FxShift down((lst[q] >> 1 & 127) - ns[t]);
+          const long long *dp = diff + (size_t)(p - c0) * NC;
+#pragma unroll
+          for (int e = 0; e < NC; ++e) acc[e] -= down(dp[e]);
+        }
+        cur[sl] = q;
+      }
+      if (vol) {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) rqi[e * nq + r] += acc[e];
+      } else {
+        const int p = op.nfp + r;
+        if (p >= c0 && p < c1) {
+          const long long *dp = diff + (size_t)(p - c0) * NC;
+#pragma unroll
+          for (int e = 0; e < NC; ++e) acc[e] += dp[e];
+        }
+#pragma unroll
+        for (int e = 0; e < NC; ++e) ff[e * nf + r] += value(t, e, acc[e]);
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = lane; i < nq; i += tpe)
+#pragma unroll
+    for (int e = 0; e < NC; ++e) rq[e * nq + i] = value(i, e, rqi[e * nq + i]);
+  __syncthreads();
+  fd_tail<D, NC>(ka, rq, ff, base + L.off[2], kk, live, lane, tpe);
+}
+
+// Fixed-point metric terms of one element per block.  2^eG bounds every
+// pair's |G|_1 2^k (no flux overflows) and keeps the scaled Lambda_q and
+// halfnJ at most 1/2; 2^-n_i bounds the sum of |G|_1 over the pairs of node i
+// in that unit (no sum of fluxes overflows).
+template <int D>
+__global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
+                                                          signed char *on, int *oeG) {
+  __shared__ double sh[3][128];
+  const DevOps &op = ka.op;
+  const FxTables &fx = ka.fx;
+  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf > 0 ? op.npf : 1;
+  const size_t k = blockIdx.x;
+  const double *Lam = ka.geo.Lambda_q + k * nq * D * D, *hnq = ka.geo.halfnJq + k * D * nfac * nq,
+               *hnf = ka.geo.halfnJf + k * D * nf, *BJf = ka.geo.BJf + k * nf, *n_f = ka.geo.n_f + k * D * nf;
+  const int lane = threadIdx.x;
+  double gmax = 0.0, lmax = 0.0, hmax = 0.0;
+  // |G|_1 of a pair; gmax: the largest with the pair's factor 2^k (NaN kept)
+  auto larger = [&](double v) { gmax = v > gmax || !(v >= 0.0) ? v : gmax; };
+  auto volume_norm = [&](int inc) {
+    const int p = inc >> 8, a = fx.vp_ij[p] & 0xffff, b = fx.vp_ij[p] >> 16, kp = inc >> 1 & 127;
+    double s = 0.0;
+    for (int n = 0; n < D; ++n) {
+      double g = 0.0;
+      for (int m = 0; m < D; ++m)
+        g = fma(fx_to_unit_double(fx.vp_S[(size_t)p * D + m]), Lam[a + nq * (m + D * n)] + Lam[b + nq * (m + D * n)], g);
+      s += fabs(g);
+    }
+    s *= fx_pow2(fx.eS);
+    larger(s);
+    return s * fx_pow2(-kp);
+  };
+  auto facet_norm = [&](int inc) {
+    const int p = inc >> 8, i = op.fp_ij[p] & 0xffff, j = op.fp_ij[p] >> 16, f = j / npf, kp = inc >> 1 & 127;
+    double s = 0.0;
+    for (int m = 0; m < D; ++m) s += fabs(fx_to_unit_double(fx.fp_C[p]) * (hnf[m + D * j] + hnq[m + D * (f + nfac * i)]));
+    s *= fx_pow2(fx.eC);
+    larger(s);
+    return s * fx_pow2(-kp);
+  };
+  // the sum over the pairs of node t; and the smallest k among them
+  auto row_norm = [&](int t, int *kmin) {
+    double s = 0.0;
+    *kmin = kFxMaxK;
+    if (t < nq) {
+      for (int q = fx.vp_inc_ptr[t]; q < fx.vp_inc_ptr[t + 1]; ++q) {
+        s += volume_norm(fx.vp_inc[q]);
+        *kmin = min(*kmin, fx.vp_inc[q] >> 1 & 127);
+      }
+    } else {
+      double b = 0.0;
+      for (int m = 0; m < D; ++m) b += fabs(0.5 * BJf[t - nq] * n_f[m + D * (t - nq)]);
+      larger(b);
+      s += b;
+    }
+    if (op.nfp > 0) {
+      const int *ptr = t < nq ? op.fp_q_ptr + t : op.fp_f_ptr + (t - nq), *lst = t < nq ? fx.fp_q : fx.fp_f;
+      for (int q = ptr[0]; q < ptr[1]; ++q) {
+        s += facet_norm(lst[q]);
+        *kmin = min(*kmin, lst[q] >> 1 & 127);
+      }
+    }
+    return s;
+  };
+  int kmin;
+  for (int t = lane; t < nq + nf; t += blockDim.x) row_norm(t, &kmin);
+  for (int t = lane; t < nq * D * D; t += blockDim.x) lmax = fmax(lmax, fabs(Lam[t]));
+  for (int t = lane; t < D * nfac * nq; t += blockDim.x) hmax = fmax(hmax, fabs(hnq[t]));
+  for (int t = lane; t < D * nf; t += blockDim.x) hmax = fmax(hmax, fabs(hnf[t]));
+  sh[0][lane] = gmax;
+  sh[1][lane] = lmax;
+  sh[2][lane] = hmax;
+  __syncthreads();
+  bool bad = false;
+  for (int t = 0; t < (int)blockDim.x; ++t) {
+    const double r = sh[0][t];
+    bad = bad || !(r >= 0.0 && r < 1e60);
+    gmax = fmax(gmax, r);
+    lmax = fmax(lmax, sh[1][t]);
+    hmax = fmax(hmax, sh[2][t]);
+  }
+  bad = bad || !(gmax > 1e-60) || !(lmax < 1e60) || !(hmax < 1e60);
+  auto ex = [](double x) { return fx_exponent((unsigned)__double2hiint(x)); };
+  int eG = ex(gmax * (1.0 + 1e-10));
+  eG = max(eG, ex(fmax(lmax, 1e-60)) + 1 + fx.eS);
+  if (op.nfp > 0) eG = max(eG, ex(fmax(hmax, 1e-60)) + 1 + fx.eC);
+  if (lane == 0) oeG[k] = bad ? kFxNone : eG;
+  if (bad) return;
+  for (int t = lane; t < nq * D * D; t += blockDim.x)
+    oLam[k * nq * D * D + t] = fx_split_near(fx_from_double(Lam[t], eG - fx.eS));
+  for (int t = lane; t < D * nfac * nq; t += blockDim.x) {
+    const int i = t % nq, fm = t / nq, f = fm / D, m = fm - f * D;
+    ohnq[k * D * nfac * nq + t] = fx_split_near(fx_from_double(hnq[m + D * (f + nfac * i)], eG - fx.eC));
+  }
+  for (int t = lane; t < D * nf; t += blockDim.x)
+    ohnf[k * D * nf + t] = fx_split_near(fx_from_double(hnf[t], eG - fx.eC));
+  for (int t = lane; t < nq + nf; t += blockDim.x) {
+    const double s = row_norm(t, &kmin) * (1.0 + 1e-10);
+    const int n = min(kmin, max(-kFxMaxK, s > 1e-60 ? eG - ex(s) : kFxMaxK));
+    on[k * (nq + nf) + t] = (signed char)n;
+    if (t >= nq)
+      for (int m = 0; m < D; ++m) {
+        const int o = m + D * (t - nq);
+        obn[k * D * nf + o] = fx_split_near(fx_from_double(0.5 * BJf[t - nq] * n_f[o], eG - n));
+      }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1593,8 +2097,11 @@ cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
     set((const void *)nodal_values_kernel<D, NC>, smA);
     set((const void *)conservation_kernel<D, NC>, smA);
     if (ka.fd) set((const void *)fd_time_derivative_kernel<D, NC>, smB);
-    else set((const void *)std_time_derivative_kernel<D, NC>, smB);
+    if (!ka.fd) set((const void *)std_time_derivative_kernel<D, NC>, smB);
   });
+  if (ka.fx.vp_ij)
+    set(ka.op.d == 2 ? (const void *)fd_time_derivative_fx_kernel<2, 4>
+                     : (const void *)fd_time_derivative_fx_kernel<3, 5>, smB);
   return e;
 }
 
@@ -1699,11 +2206,24 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
     }
     return cudaGetLastError();
   }
-  if (ka.fd) {
+  // the fixed-point passes wherever their tables exist (the EC flux with
+  // gamma <= 1.7); their blocks choose FP64 for themselves
+  if (ka.fx.on) {
+    sm = (size_t)ka.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
+    if (ka.op.d == 2) fd_time_derivative_fx_kernel<2, 4><<<grid, ka.tpb, sm, st>>>(ka);
+    else fd_time_derivative_fx_kernel<3, 5><<<grid, ka.tpb, sm, st>>>(ka);
+  } else if (ka.fd) {
     SSE_DISPATCH(D, NC, (fd_time_derivative_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka)));
   } else {
     SSE_DISPATCH(D, NC, (std_time_derivative_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka)));
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
+                               cudaStream_t st) {
+  if (ka.op.d == 2) fx_geometry_kernel<2><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
+  else fx_geometry_kernel<3><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
   return cudaGetLastError();
 }
 

@@ -7,6 +7,7 @@
 
 #include "../../include/sse_gb300.h"
 #include "sse_device.cuh"
+#include "sse_fixed.cuh"
 
 namespace sse {
 
@@ -20,11 +21,44 @@ struct Layout {
   int team_doubles;
 };
 
+// Fixed-point copies of the flux-differencing operators and metric terms
+// (sse_fixed.cuh) for the FP64 phase B with the entropy-conservative flux.
+// Volume pairs are ordered by the set of directions m with S_m != 0, so that
+// the lanes of a warp form the same products; their node sums are integer
+// sums, for which any order gives the same bits.
+// The quadrature weights of collapsed elements spread over orders of
+// magnitude, and with them the operator entries: pair p carries its S (or C)
+// times 2^k_p (largest entry in [1/2, 1)), so that its flux has all its bits,
+// and node i sums 2^n_i times its contributions, each shifted down by
+// k_p - n_i >= 0.
+struct FxTables {
+  int on;             // 0: no fixed-point tables, phase B runs in FP64
+  const int *vp_ij;   // i | j << 16
+  const Fx *vp_S;     // nvp x d: S / 2 in units 2^(eS - k)
+  // incident pairs per node: pair << 8 | k << 1 | sign (volume pairs: node is i)
+  const int *vp_inc_ptr, *vp_inc;
+  const Fx *fp_C;     // C / 2 in units 2^(eC - k)
+  const int *fp_q, *fp_f;  // pair << 8 | k << 1, at DevOps::fp_q_ptr, fp_f_ptr
+  int eS, eC;
+  const int *eG;      // per element: metric vectors in units 2^eG (kFxNone: none)
+  const Fx *Lam;      // Lambda_q in units 2^(eG - eS), the layout of Lambda_q
+  const Fx *hnq;      // halfnJq in units 2^(eG - eC), transposed to (f d + m) n_q + i
+  const Fx *hnf;      // halfnJf in units 2^(eG - eC)
+  const Fx *bn;       // BJf n_f / 2 in units 2^(eG - n), d x nf x ne
+  const signed char *n;  // node shifts n_i, (nq + nf) x ne
+};
+constexpr int kFxMaxK = 30;  // largest k_p
+constexpr int kFxNone = -100000;
+
 struct KernelArgs {
   DevOps op;
+  FxTables fx;
   DevGeo geo;
   Physics ph;
   Layout layA, layB;
+  Layout layBx;      // fixed-point phase B: 0 facet fluxes, 1 r_q, 2 pair buffer and tail scratch,
+                     // 3 Lambda_q, 4 halfnJq, 5 halfnJf, 6 node values, 7 float pairs, 8 extremes,
+                     // 9 node shifts
   Layout layBm;      // mixed-form phase B layout, offsets and team size in floats:
                      // 0 volume states (then r_q), 1 facet states, 2 facet fluxes,
                      // 3 mass operator, 4 pair buffer, 5 Lambda_q, 6 halfnJq,
@@ -64,6 +98,7 @@ struct KernelArgs {
   int pair_chunk;    // pairs per shared-memory chunk in the pair-adjoint passes
   int pair_chunk_generic;  // the same for the conservative two-point flux
   int fd_chunk;      // pairs per chunk in the FP64 flux-differencing passes
+  int fx_chunk;      // pairs per chunk in the fixed-point passes
   int vp_split;      // volume pairs per interface lane in the one-chunk pass (0: even split)
   int epb_bm;        // elements per block of the FP32 phase-B kernel (blocks of tpb threads)
   int epb_am;        // elements per block of the mixed phase-A kernel (blocks of tpb threads)
@@ -156,6 +191,9 @@ cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st);
 cudaError_t launch_projection_of_one(const KernelArgs &ka, double *P1, double *RP1, cudaStream_t st);
 cudaError_t sse_set_smem_limits_mixed_a(const KernelArgs &ka);
 cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st);
+// the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG)
+cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
+                               cudaStream_t st);
 cudaError_t launch_mass_operator(const KernelArgs &ka, double *Ak, cudaStream_t st);
 cudaError_t launch_energy(const KernelArgs &ka, const double *u, const double *dudt, double *partial,
                           cudaStream_t st);
