@@ -235,11 +235,17 @@ std::vector<double> csc_dense(const sse_csc &A, int rows, int cols) {
 }
 
 
+// incidence words (pair << 8 | k << 1 | sign) of every volume node's volume
+// pairs, and of every volume and facet node's facet pairs
+struct FxLists {
+  std::vector<std::vector<int>> vol, fac;
+};
+
 // Fixed-point pair tables (KernelArgs::fx) from the FP64 ones: volume pairs
 // ordered by the directions in which S is nonzero, each pair's S / 2 or C / 2
 // as integers with its own factor 2^k, and the incidence lists with k.
 int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vector<double> &vp_S,
-                   const std::vector<double> &C, const std::vector<int> &qflat, const std::vector<int> &fflat) {
+                   const std::vector<double> &C, const std::vector<std::vector<int>> &fp_inc, FxLists *lists) {
   KernelArgs &ka = s->ka;
   const int d = s->cfg.d, nq = s->cfg.n_q, nvp = (int)vp_ij.size();
   auto largest = [](const double *v, size_t n) {
@@ -261,38 +267,59 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
     for (int m = 0; m < d; ++m) mask[t] |= (vp_S[(size_t)t * d + m] != 0.0) << m;
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return mask[a] > mask[b]; });
-  std::vector<int> ij(nvp), inc_flat, inc_ptr(nq + 1, 0);
+  std::vector<int> ij(nvp);
   std::vector<Fx> S((size_t)nvp * d), Cx(C.size());
-  std::vector<std::vector<int>> inc(nq);
+  lists->vol.assign(nq, {});
   for (int t = 0; t < nvp; ++t) {
     const double *v = &vp_S[(size_t)order[t] * d];
     const int k = std::min(kFxMaxK, fx.eS - exponent(largest(v, d)));
     ij[t] = vp_ij[order[t]];
-    inc[ij[t] & 0xffff].push_back(t << 8 | k << 1 | 1);
-    inc[ij[t] >> 16].push_back(t << 8 | k << 1);
+    lists->vol[ij[t] & 0xffff].push_back(t << 8 | k << 1 | 1);
+    lists->vol[ij[t] >> 16].push_back(t << 8 | k << 1);
     for (int m = 0; m < d; ++m) S[(size_t)t * d + m] = fx_split_near(fx_from_double(0.5 * v[m], fx.eS - k));
-  }
-  for (int i = 0; i < nq; ++i) {
-    inc_flat.insert(inc_flat.end(), inc[i].begin(), inc[i].end());
-    inc_ptr[i + 1] = (int)inc_flat.size();
   }
   std::vector<int> kC(C.size());
   for (size_t t = 0; t < C.size(); ++t) {
     kC[t] = std::min(kFxMaxK, fx.eC - exponent(std::fabs(C[t])));
     Cx[t] = fx_split_near(fx_from_double(0.5 * C[t], fx.eC - kC[t]));
   }
-  std::vector<int> q(qflat), f(fflat);
-  for (int &v : q) v = v << 8 | kC[v] << 1;
-  for (int &v : f) v = v << 8 | kC[v] << 1;
+  lists->fac = fp_inc;
+  for (auto &l : lists->fac)
+    for (int &v : l) v = v << 8 | kC[v] << 1;
   cudaError_t e;
   if ((e = upload(s, ij.data(), ij.size(), &fx.vp_ij)) || (e = upload(s, S.data(), S.size(), &fx.vp_S)) ||
-      (e = upload(s, inc_ptr.data(), inc_ptr.size(), &fx.vp_inc_ptr)) ||
-      (e = upload(s, inc_flat.data(), inc_flat.size(), &fx.vp_inc)))
-    return cuda_fail(s, e, "fixed-point pair tables");
-  if (!C.empty() && ((e = upload(s, Cx.data(), Cx.size(), &fx.fp_C)) || (e = upload(s, q.data(), q.size(), &fx.fp_q)) ||
-                     (e = upload(s, f.data(), f.size(), &fx.fp_f))))
+      (!C.empty() && (e = upload(s, Cx.data(), Cx.size(), &fx.fp_C))))
     return cuda_fail(s, e, "fixed-point pair tables");
   ka.fx = fx;
+  return SSE_OK;
+}
+
+// The incidence lists of the fixed-point passes, with each node's range in
+// every chunk of ka.fx_chunk pairs.
+int setup_fx_lists(sse_solver *s, const FxLists &lists) {
+  FxTables &fx = s->ka.fx;
+  const int CH = s->ka.fx_chunk;
+  auto flatten = [&](const std::vector<std::vector<int>> &inc, int pairs, int *chunks, const int **ptr_d,
+                     const int **inc_d) {
+    *chunks = (pairs + CH - 1) / CH;
+    const size_t n = inc.size();
+    std::vector<int> flat, ptr((*chunks + 1) * n);
+    for (size_t t = 0; t < n; ++t) {
+      size_t q = 0;
+      for (int c = 0; c <= *chunks; ++c) {
+        while (q < inc[t].size() && (inc[t][q] >> 8) / CH < c) ++q;
+        ptr[c * n + t] = (int)(flat.size() + q);
+      }
+      flat.insert(flat.end(), inc[t].begin(), inc[t].end());
+    }
+    if (flat.empty()) flat.push_back(0);
+    cudaError_t e = upload(s, ptr.data(), ptr.size(), ptr_d);
+    return e ? e : upload(s, flat.data(), flat.size(), inc_d);
+  };
+  cudaError_t e;
+  if ((e = flatten(lists.vol, s->ka.op.nvp, &fx.vp_chunks, &fx.vp_ptr, &fx.vp_inc)) ||
+      (e = flatten(lists.fac, s->ka.op.nfp + s->ka.op.nf, &fx.fp_chunks, &fx.fp_ptr, &fx.fp_inc)))
+    return cuda_fail(s, e, "fixed-point incidence lists");
   return SSE_OK;
 }
 
@@ -625,6 +652,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   }
 
   // ---- flux-differencing pair tables
+  FxLists fx_lists;
   if (fd) {
     // unique pairs (i < j) over the union of the S_m patterns, ordered by (j, i)
     std::vector<std::pair<int, int>> pairs;
@@ -677,23 +705,22 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
 
     op.nfp = 0;
     std::vector<double> fp_C;
-    std::vector<int> qflat, fflat;
+    std::vector<std::vector<int>> fp_inc(c.n_q + c.n_f);  // of the volume, then the facet nodes
     if (has_C) {
       const sse_csc &Cm = ops->C;
       std::vector<int> fp_ij;
-      std::vector<std::vector<int>> qinc(c.n_q), finc(c.n_f);
       for (int64_t j = 0; j < Cm.n; ++j)
         for (int64_t q = Cm.colptr[j] - 1; q < Cm.colptr[j + 1] - 1; ++q) {
           int i = (int)(Cm.rowval[q] - 1);
           int t = (int)fp_ij.size();
           fp_ij.push_back(i | ((int)j << 16));
           fp_C.push_back(Cm.nzval[q]);
-          qinc[i].push_back(t);
-          finc[j].push_back(t);
+          fp_inc[i].push_back(t);
+          fp_inc[c.n_q + j].push_back(t);
         }
-      std::vector<int> qptr(c.n_q + 1, 0), fptr(c.n_f + 1, 0);
-      for (int i = 0; i < c.n_q; ++i) { qflat.insert(qflat.end(), qinc[i].begin(), qinc[i].end()); qptr[i + 1] = (int)qflat.size(); }
-      for (int j = 0; j < c.n_f; ++j) { fflat.insert(fflat.end(), finc[j].begin(), finc[j].end()); fptr[j + 1] = (int)fflat.size(); }
+      std::vector<int> qptr(c.n_q + 1, 0), qflat, fptr(c.n_f + 1, 0), fflat;
+      for (int i = 0; i < c.n_q; ++i) { qflat.insert(qflat.end(), fp_inc[i].begin(), fp_inc[i].end()); qptr[i + 1] = (int)qflat.size(); }
+      for (int j = 0; j < c.n_f; ++j) { fflat.insert(fflat.end(), fp_inc[c.n_q + j].begin(), fp_inc[c.n_q + j].end()); fptr[j + 1] = (int)fflat.size(); }
       op.nfp = (int)fp_ij.size();
       s->nfpC = fp_C.size();
       if ((e = upload(s, fp_ij.data(), fp_ij.size(), &op.fp_ij)) != cudaSuccess) return cuda_fail(s, e, "upload");
@@ -712,7 +739,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     // fx_ec_flux (gamma <= 1.7)
     ka.fx = FxTables{};
     if (c.law == SSE_EULER && c.two_point_flux == SSE_EC_FLUX && c.gamma > 1.0 && c.gamma <= 1.7 &&
-        (rc = setup_fx_pairs(s, vp_ij, vp_S, fp_C, qflat, fflat)))
+        (rc = setup_fx_pairs(s, vp_ij, vp_S, fp_C, fp_inc, &fx_lists)))
       return rc;
   }
 
@@ -785,6 +812,8 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     for (; i < 12; ++i) L.off[i] = off;
     L.team_doubles = off;
   };
+  Layout fx_layB{};     // FP64 passes inside the fixed-point kernel: layout and chunk
+  int fx_fd_chunk = 0;
   // phase-A layout: X, Y, Z, W, F, lane partials; F holds NC x max(N_p, N_q,
   // N_f) (modal scratch, facet values, or V dudt in the conservation kernel)
   finish(ka.layA, {nc * std::max(np, nq), nc * nq, zsz, wsz, nc * std::max({np, nq, nf}), tpe * (nc + 1)});
@@ -824,29 +853,50 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     ka.vdm_zsz = zsz_e;
     layout(chunk);
     if (ka.fx.vp_ij) {
-      // the same rule for the fixed-point passes, whose second pass has the
-      // interface fluxes too
+      // Fixed-point passes: the second has the interface fluxes too.  A thread
+      // takes about 5.5 pairs in all, as far as blocks of 256 threads allow
+      // (13,182 p = 2 tets, 269 pairs: 64 threads 0.318 ms, 32 0.438, 128 0.397;
+      // 8,192 p = 4 triangles, 190: 32 threads 0.144 ms, 16 0.176, 64 0.155; p = 3,
+      // 108: 16 threads 0.087 ms, 32 0.114).  All pairs at once where two blocks
+      // still fit on an SM (p = 4 tets: three), else chunks for two blocks (7,986
+      // p = 5 tets: chunks of 1,536 of 2,088 pairs 2.02 ms, 512 for three blocks
+      // 2.37), or for one if those were below a third of the pairs (3,072 p = 6
+      // tets: all 3,626 pairs 2.09 ms, chunks of 768 2.57).
+      int tpe_x = 16;
+      while (tpe_x < 256 && (op.nvp + op.nfp + nf) / 5.5 > 1.414 * tpe_x) tpe_x *= 2;
+      while (nq + nf > kMaxNodeSlots * tpe_x) tpe_x *= 2;
+      const int epb_x = tpe_x < 128 ? 128 / tpe_x : 1;
+      ka.epb_bx = epb_x;
+      ka.tpb_bx = epb_x * tpe_x;
+      const int budget = 110 * 1024 / 8 / epb_x;
       const int nodes = nq + 2 * nf, pairs = std::max(op.nvp, op.nfp + nf), stride = d == 2 ? kFxStride<2> : kFxStride<3>;
       auto layout_x = [&](int n) {
-        finish(ka.layBx, {nc * nf, nc * nq, std::max(n * nc, final_scratch), d * d * nq,
-                          op.nfp > 0 ? d * c.num_faces * nq : 0, op.nfp > 0 ? d * nf : 0, nodes * stride, 2 * nodes, 4,
+        finish(ka.layBx, {nc * nf, nc * nq, std::max(n * nc, final_scratch), nodes * stride, 2 * nodes, 4,
                           (nq + nf + 7) / 8});
         return ka.layBx.team_doubles;
       };
       int n = pairs;
       if (layout_x(n) > budget) {
         const int fixed = layout_x(0) - ((std::max(0, final_scratch) + 1) & ~1);
-        const int cap1 = (int)((size_t)220 * 1024 / 8 / epb_for(tpe));
+        const int cap1 = (int)((size_t)220 * 1024 / 8 / epb_x);
         int room = budget - fixed;
-        if (room / nc < std::min(tpe, pairs)) room = cap1 - fixed;
+        if (room / nc < std::max(std::min(tpe_x, pairs), pairs / 3)) room = cap1 - fixed;
         n = std::max(1, room / nc);
-        if (n >= tpe) n = n / tpe * tpe;
+        if (n < pairs && n >= tpe_x) n = n / tpe_x * tpe_x;
         n = std::max(1, std::min(n, pairs));
       }
       ka.fx_chunk = n;
       layout_x(n);
       // no room for the node values: the FP64 passes
-      if ((size_t)epb_for(tpe) * ka.layBx.team_doubles * 8 > (size_t)220 * 1024) ka.fx = FxTables{};
+      if ((size_t)epb_x * ka.layBx.team_doubles * 8 > (size_t)220 * 1024) ka.fx = FxTables{};
+      // the FP64 passes of blocks that leave the fixed-point ones fit in the
+      // same shared memory where chunks of at least one pass of the threads do
+      const Layout one = ka.layB;
+      const int room = (ka.layBx.team_doubles - (layout(0) - ((std::max(0, final_scratch) + 1) & ~1)) - 1) / nc;
+      fx_fd_chunk = std::min(chunk, room >= tpe_x ? room / tpe_x * tpe_x : std::min(tpe_x, max_pairs));
+      layout(fx_fd_chunk);
+      fx_layB = ka.layB;
+      ka.layB = one;
     }
     // the interface flux of one facet node costs about 0.8 of a volume pair
     // (block timings at p = 4): balance lanes when all pairs are one chunk.
@@ -904,7 +954,9 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   if ((size_t)ka.epb_a * ka.layA.team_doubles * 8 > 220 * 1024) ka.epb_a = epb;
   // opt in to large dynamic shared memory for every kernel instantiation used
   size_t smA = (size_t)std::max(epb, ka.epb_a) * ka.layA.team_doubles * 8,
-         smB = (size_t)epb * std::max(ka.layB.team_doubles, ka.fx.vp_ij ? ka.layBx.team_doubles : 0) * 8;
+         smB = (size_t)epb * ka.layB.team_doubles * 8;
+  if (ka.fx.vp_ij)
+    smB = std::max(smB, (size_t)ka.epb_bx * std::max(fx_layB.team_doubles, ka.layBx.team_doubles) * 8);
   if ((e = sse_set_smem_limits(ka, smA, smB)) != cudaSuccess) return cuda_fail(s, e, "cudaFuncSetAttribute");
 
   // the weight-adjusted mass operator V' diag(J^-1 W) V of every element,
@@ -923,7 +975,12 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       ka.Ak = (const double *)p;
     }
   }
-  if (ka.fx.vp_ij && (rc = setup_fx_geometry(s))) return rc;
+  if (ka.fx.vp_ij && ((rc = setup_fx_lists(s, fx_lists)) || (rc = setup_fx_geometry(s)))) return rc;
+  if (ka.fx.on) {
+    ka.layB = fx_layB;
+    ka.fd_chunk = fx_fd_chunk;
+    ka.vp_split = 0;
+  }
   return setup_compact(s, ops, mapP);
 }
 

@@ -612,8 +612,12 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // the issue slots 10 %).  Here the pairs take none: node values are scaled to
 // integers once per element, the pair passes are integer multiply-adds and
 // FP32, and FP64 is left to the node values, the Lax-Friedrichs term and the
-// tail.  24,576 p = 4 tets: 8.86 -> 3.58 ms; 7,986 p = 5 tets 6.5 -> 2.42 ms;
-// 8,192 p = 4 triangles 0.365 -> 0.184 ms.  The error against the
+// tail.  Metric terms are read through L1, which leaves shared memory for
+// three blocks of 256 threads on an SM (80 registers): while one block is in its
+// FP64 part the others keep the integer pipes busy (staged in shared memory,
+// two blocks: 3.58 ms against 2.48).  24,576 p = 4 tets: 8.86 -> 2.48 ms; 7,986
+// p = 5 tets 6.5 -> 2.02 ms; 13,182 p = 2 tets 0.96 -> 0.316 ms; 8,192 p = 4
+// triangles 0.365 -> 0.145 ms.  The error against the
 // extended-precision residual is 0.81 to 1.00 of the FP64 passes' own on 60
 // configurations (modal and nodal, p = 2 to 6, both metrics and interface
 // fluxes).
@@ -643,11 +647,6 @@ struct FxShift {
   __device__ __forceinline__ long long operator()(long long v) const { return (v + half) >> s; }
 };
 
-__device__ __forceinline__ void fx_copy_async(Fx *dst, const Fx *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-
 // Exponents of an element's units from the extremes of its node values (upper
 // words of the largest density, enthalpy and |velocity component| and
 // 0x7fffffff less that of the smallest density and enthalpy); ok: positive,
@@ -667,8 +666,17 @@ struct FxScale {
   }
 };
 
+// the FP64 passes for a block that leaves the fixed-point ones: out of line, so
+// that their registers are not the kernel's
 template <int D, int NC>
-__global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs ka) {
+__device__ __noinline__ void fd_fp64(const KernelArgs &ka, double *base, int kk, bool live, int lane, int tpe) {
+  const Layout &L = ka.layB;
+  fd_fluxes<D, NC>(ka, base, kk, lane, tpe);
+  fd_tail<D, NC>(ka, base + L.off[3], base + L.off[2], base + L.off[4], kk, live, lane, tpe);
+}
+
+template <int D, int NC>
+__global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __grid_constant__ KernelArgs ka) {
   static_assert(NC == D + 2, "Euler");
   extern __shared__ double smem[];
   const DevOps &op = ka.op;
@@ -686,24 +694,15 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
   double *ff = base + L.off[0], *rq = base + L.off[1];
   long long *diff = reinterpret_cast<long long *>(base + L.off[2]);
   long long *rqi = reinterpret_cast<long long *>(rq);
-  Fx *Lam = reinterpret_cast<Fx *>(base + L.off[3]), *hnq = reinterpret_cast<Fx *>(base + L.off[4]),
-     *hnf = reinterpret_cast<Fx *>(base + L.off[5]), *node = reinterpret_cast<Fx *>(base + L.off[6]);
-  double *noded = base + L.off[6];
-  FxPair *pair = reinterpret_cast<FxPair *>(base + L.off[7]);
-  unsigned *key = reinterpret_cast<unsigned *>(base + L.off[8]);
-  signed char *ns = reinterpret_cast<signed char *>(base + L.off[9]);
+  Fx *node = reinterpret_cast<Fx *>(base + L.off[3]);
+  double *noded = base + L.off[3];
+  FxPair *pair = reinterpret_cast<FxPair *>(base + L.off[4]);
+  unsigned *key = reinterpret_cast<unsigned *>(base + L.off[5]);
+  signed char *ns = reinterpret_cast<signed char *>(base + L.off[6]);
+  // metric terms, read through L1
+  const Fx *Lam = fx.Lam + (size_t)kk * nq * D * D, *hnq = fx.hnq + (size_t)kk * D * nfac * nq,
+           *hnf = fx.hnf + (size_t)kk * D * nf;
 
-  // metric terms, landing while the node values are formed
-  {
-    const Fx *g = fx.Lam + (size_t)kk * nq * D * D;
-    for (int t = lane; t < nq * D * D; t += tpe) fx_copy_async(Lam + t, g + t);
-    if (op.nfp > 0) {
-      g = fx.hnq + (size_t)kk * D * nfac * nq;
-      for (int t = lane; t < D * nfac * nq; t += tpe) fx_copy_async(hnq + t, g + t);
-      g = fx.hnf + (size_t)kk * D * nf;
-      for (int t = lane; t < D * nf; t += tpe) fx_copy_async(hnf + t, g + t);
-    }
-  }
   for (int t = lane; t < nq + nf; t += tpe) ns[t] = fx.n[(size_t)kk * (nq + nf) + t];
   if (lane < 5) key[lane] = 0u;
   // FP64 node values [rho, p, h, V] of the volume nodes, the facet nodes and
@@ -787,15 +786,12 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
     atomicMax(key + 3, k3);
     atomicMax(key + 4, k4);
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const int eG = fx.eG[kk];
   const FxScale sc(key, eG);
   // a block with an element out of range runs in FP64 as a whole
   if (!__syncthreads_and(sc.ok)) {
-    double *b64 = smem + (size_t)team * ka.layB.team_doubles;
-    fd_fluxes<D, NC>(ka, b64, kk, lane, tpe);
-    fd_tail<D, NC>(ka, b64 + ka.layB.off[3], b64 + ka.layB.off[2], b64 + ka.layB.off[4], kk, live, lane, tpe);
+    fd_fp64<D, NC>(ka, smem + (size_t)team * ka.layB.team_doubles, kk, live, lane, tpe);
     return;
   }
   const int kappa = sc.eH - 2 * sc.eV, eP = sc.eR + sc.eH - 2;
@@ -825,17 +821,8 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
   // volume flux differencing: pass 1 one flux per pair, pass 2 each node's sum
   // over its pairs (as fd_fluxes, in integers)
   const int CH = ka.fx_chunk;
-  int cur[kMaxNodeSlots];
-#pragma unroll
-  for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
-    const int i = lane + sl * tpe;
-    cur[sl] = i < nq ? fx.vp_inc_ptr[i] : 0;
-    if (i < nq)
-#pragma unroll
-      for (int e = 0; e < NC; ++e) rqi[e * nq + i] = 0;
-  }
-  for (int c0 = 0; c0 < op.nvp; c0 += CH) {
-    const int c1 = min(op.nvp, c0 + CH);
+  for (int c = 0; c < fx.vp_chunks; ++c) {
+    const int c0 = c * CH, c1 = min(op.nvp, c0 + CH);
     for (int p = c0 + lane; p < c1; p += tpe) {
       const int ij = fx.vp_ij[p];
       const int i = ij & 0xffff, j = ij >> 16;
@@ -864,26 +851,20 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
       for (int e = 0; e < NC; ++e) dp[e] = out[e];
     }
     __syncthreads();
-#pragma unroll
-    for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
-      const int i = lane + sl * tpe;
-      if (i >= nq) continue;
+    for (int i = lane; i < nq; i += tpe) {
+      const int n = ns[i], qe = fx.vp_ptr[(c + 1) * nq + i];
       long long acc[NC];
 #pragma unroll
-      for (int e = 0; e < NC; ++e) acc[e] = rqi[e * nq + i];
-      int q = cur[sl];
-      const int qe = fx.vp_inc_ptr[i + 1];
-      for (; q < qe; ++q) {
+      for (int e = 0; e < NC; ++e) acc[e] = c == 0 ? 0 : rqi[e * nq + i];
+      // r_q[i] += -diff if i is the pair's first node, +diff otherwise
+#pragma unroll 4
+      for (int q = fx.vp_ptr[c * nq + i]; q < qe; ++q) {
         const int inc = fx.vp_inc[q];
-        const int p = inc >> 8;
-        if (p >= c1) break;
-        const FxShift down((inc >> 1 & 127) - ns[i]);
-        const long long *dp = diff + (size_t)(p - c0) * NC;
-        // r_q[i] += -diff if i is the pair's first node, +diff otherwise
+        const FxShift down((inc >> 1 & 127) - n);
+        const long long *dp = diff + (size_t)((inc >> 8) - c0) * NC;
 #pragma unroll
         for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
       }
-      cur[sl] = q;
 #pragma unroll
       for (int e = 0; e < NC; ++e) rqi[e * nq + i] = acc[e];
     }
@@ -899,15 +880,10 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
   // facet correction and interface flux, chunked the same way; the sums are
   // subtracted from r_q (integers) and f_f (converted, FP64)
   const float rnpf = qrcp(npf > 0 ? npf : 1);
-#pragma unroll
-  for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
-    const int t = lane + sl * tpe;
-    cur[sl] = op.nfp == 0 ? 0 : (t < nq ? op.fp_q_ptr[t] : (t < nq + nf ? op.fp_f_ptr[t - nq] : 0));
-  }
   // the pairs nfp .. nfp + nf - 1 are the facet nodes with their facing nodes
   const int nall = op.nfp + nf;
-  for (int c0 = 0; c0 < nall; c0 += CH) {
-    const int c1 = min(nall, c0 + CH);
+  for (int c = 0; c < fx.fp_chunks; ++c) {
+    const int c0 = c * CH, c1 = min(nall, c0 + CH);
     for (int p = c0 + lane; p < c1; p += tpe) {
       Fx G[D];
       int i, j;
@@ -934,34 +910,24 @@ __global__ void __launch_bounds__(256) fd_time_derivative_fx_kernel(KernelArgs k
       for (int e = 0; e < NC; ++e) dp[e] = out[e];
     }
     __syncthreads();
-#pragma unroll
-    for (int sl = 0; sl < kMaxNodeSlots; ++sl) {
-      const int t = lane + sl * tpe;
-      if (t >= nq + nf) continue;
+    for (int t = lane; t < nq + nf; t += tpe) {
+      const int n = ns[t], qe = fx.fp_ptr[(c + 1) * (nq + nf) + t];
       long long acc[NC];
 #pragma unroll
       for (int e = 0; e < NC; ++e) acc[e] = 0;
-      const bool vol = t < nq;
-      const int r = vol ? t : t - nq;
-      if (op.nfp > 0) {
-        const int *lst = vol ? fx.fp_q : fx.fp_f;
-        const int qe = vol ? op.fp_q_ptr[r + 1] : op.fp_f_ptr[r + 1];
-        int q = cur[sl];
-        for (; q < qe; ++q) {
-          const int p = lst[q] >> 8;
-          if (p >= c1) break;
-          const FxShift down((lst[q] >> 1 & 127) - ns[t]);
-          const long long *dp = diff + (size_t)(p - c0) * NC;
+#pragma unroll 4
+      for (int q = fx.fp_ptr[c * (nq + nf) + t]; q < qe; ++q) {
+        const int inc = fx.fp_inc[q];
+        const FxShift down((inc >> 1 & 127) - n);
+        const long long *dp = diff + (size_t)((inc >> 8) - c0) * NC;
 #pragma unroll
-          for (int e = 0; e < NC; ++e) acc[e] -= down(dp[e]);
-        }
-        cur[sl] = q;
+        for (int e = 0; e < NC; ++e) acc[e] -= down(dp[e]);
       }
-      if (vol) {
+      if (t < nq) {
 #pragma unroll
-        for (int e = 0; e < NC; ++e) rqi[e * nq + r] += acc[e];
+        for (int e = 0; e < NC; ++e) rqi[e * nq + t] += acc[e];
       } else {
-        const int p = op.nfp + r;
+        const int r = t - nq, p = op.nfp + r;
         if (p >= c0 && p < c1) {
           const long long *dp = diff + (size_t)(p - c0) * NC;
 #pragma unroll
@@ -1024,7 +990,7 @@ __global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLa
     double s = 0.0;
     *kmin = kFxMaxK;
     if (t < nq) {
-      for (int q = fx.vp_inc_ptr[t]; q < fx.vp_inc_ptr[t + 1]; ++q) {
+      for (int q = fx.vp_ptr[t]; q < fx.vp_ptr[fx.vp_chunks * nq + t]; ++q) {
         s += volume_norm(fx.vp_inc[q]);
         *kmin = min(*kmin, fx.vp_inc[q] >> 1 & 127);
       }
@@ -1034,12 +1000,9 @@ __global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLa
       larger(b);
       s += b;
     }
-    if (op.nfp > 0) {
-      const int *ptr = t < nq ? op.fp_q_ptr + t : op.fp_f_ptr + (t - nq), *lst = t < nq ? fx.fp_q : fx.fp_f;
-      for (int q = ptr[0]; q < ptr[1]; ++q) {
-        s += facet_norm(lst[q]);
-        *kmin = min(*kmin, lst[q] >> 1 & 127);
-      }
+    for (int q = fx.fp_ptr[t]; q < fx.fp_ptr[fx.fp_chunks * (nq + nf) + t]; ++q) {
+      s += facet_norm(fx.fp_inc[q]);
+      *kmin = min(*kmin, fx.fp_inc[q] >> 1 & 127);
     }
     return s;
   };
@@ -2209,9 +2172,12 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
   // the fixed-point passes wherever their tables exist (the EC flux with
   // gamma <= 1.7); their blocks choose FP64 for themselves
   if (ka.fx.on) {
-    sm = (size_t)ka.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
-    if (ka.op.d == 2) fd_time_derivative_fx_kernel<2, 4><<<grid, ka.tpb, sm, st>>>(ka);
-    else fd_time_derivative_fx_kernel<3, 5><<<grid, ka.tpb, sm, st>>>(ka);
+    KernelArgs kx = ka;
+    kx.epb = ka.epb_bx;
+    const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
+    sm = (size_t)kx.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
+    if (ka.op.d == 2) fd_time_derivative_fx_kernel<2, 4><<<gridx, ka.tpb_bx, sm, st>>>(kx);
+    else fd_time_derivative_fx_kernel<3, 5><<<gridx, ka.tpb_bx, sm, st>>>(kx);
   } else if (ka.fd) {
     SSE_DISPATCH(D, NC, (fd_time_derivative_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka)));
   } else {

@@ -35,10 +35,16 @@ struct FxTables {
   int on;             // 0: no fixed-point tables, phase B runs in FP64
   const int *vp_ij;   // i | j << 16
   const Fx *vp_S;     // nvp x d: S / 2 in units 2^(eS - k)
-  // incident pairs per node: pair << 8 | k << 1 | sign (volume pairs: node is i)
-  const int *vp_inc_ptr, *vp_inc;
+  // incident pairs per volume node: pair << 8 | k << 1 | (node is i), ascending;
+  // those in chunk c (ka.fx_chunk pairs) of node i: vp_ptr[c nq + i] to
+  // vp_ptr[(c + 1) nq + i]
+  int vp_chunks;
+  const int *vp_ptr, *vp_inc;
+  // facet-correction pairs followed by the nf interface pairs; incident
+  // facet-correction pairs of the volume, then the facet nodes
+  int fp_chunks;
   const Fx *fp_C;     // C / 2 in units 2^(eC - k)
-  const int *fp_q, *fp_f;  // pair << 8 | k << 1, at DevOps::fp_q_ptr, fp_f_ptr
+  const int *fp_ptr, *fp_inc;
   int eS, eC;
   const int *eG;      // per element: metric vectors in units 2^eG (kFxNone: none)
   const Fx *Lam;      // Lambda_q in units 2^(eG - eS), the layout of Lambda_q
@@ -57,8 +63,7 @@ struct KernelArgs {
   Physics ph;
   Layout layA, layB;
   Layout layBx;      // fixed-point phase B: 0 facet fluxes, 1 r_q, 2 pair buffer and tail scratch,
-                     // 3 Lambda_q, 4 halfnJq, 5 halfnJf, 6 node values, 7 float pairs, 8 extremes,
-                     // 9 node shifts
+                     // 3 node values, 4 float pairs, 5 extremes, 6 node shifts
   Layout layBm;      // mixed-form phase B layout, offsets and team size in floats:
                      // 0 volume states (then r_q), 1 facet states, 2 facet fluxes,
                      // 3 mass operator, 4 pair buffer, 5 Lambda_q, 6 halfnJq,
@@ -100,6 +105,7 @@ struct KernelArgs {
   int fd_chunk;      // pairs per chunk in the FP64 flux-differencing passes
   int fx_chunk;      // pairs per chunk in the fixed-point passes
   int vp_split;      // volume pairs per interface lane in the one-chunk pass (0: even split)
+  int epb_bx, tpb_bx;  // elements and threads per block of the fixed-point phase B
   int epb_bm;        // elements per block of the FP32 phase-B kernel (blocks of tpb threads)
   int epb_am;        // elements per block of the mixed phase-A kernel (blocks of tpb threads)
   int epb_a;         // elements per block of the FP64 phase-A kernel (blocks of tpb threads)
