@@ -22,6 +22,7 @@
 
 #include "../../include/sse_gb300.h"
 #include "sse_kernels.cuh"
+#include "sse_fixed_ops.cuh"
 
 using namespace sse;
 
@@ -320,6 +321,100 @@ int setup_fx_lists(sse_solver *s, const FxLists &lists) {
   if ((e = flatten(lists.vol, s->ka.op.nvp, &fx.vp_chunks, &fx.vp_ptr, &fx.vp_inc)) ||
       (e = flatten(lists.fac, s->ka.op.nfp + s->ka.op.nf, &fx.fp_chunks, &fx.fp_ptr, &fx.fp_inc)))
     return cuda_fail(s, e, "fixed-point incidence lists");
+  return SSE_OK;
+}
+
+// Fixed-point operators of phase A (ka.fx.A, B, C, T, K, R, eR) for a
+// tensor-product V of at most 8 nodes and modes a direction (the sums of cross
+// products then stay below 2^63).
+int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
+  KernelArgs &ka = s->ka;
+  FxTables &fx = ka.fx;
+  const sse_config &c = s->cfg;
+  const DevOps &op = ka.op;
+  if (!op.has_vdm || op.dense_v || op.p1 > 8 || op.M1 > 8 || op.M2 > 8 || (c.d == 3 && op.M3 > 8)) return SSE_OK;
+  const int p1 = op.p1, M3 = c.d == 3 ? op.M3 : 1;
+  // one factor, `vectors` mode vectors of M nodes: node a times 2^k[a] <= 1 (the
+  // node's largest entry brought down to the smallest such over the nodes),
+  // then vector t times 2^-ex[t] to at most 1/4; false when not finite
+  auto scale = [](const double *v, int M, size_t vectors, std::vector<Fx> *out, std::vector<int> *k,
+                  std::vector<int> *ex) {
+    out->assign((size_t)M * vectors, Fx{0, 0});
+    k->assign(M, 0);
+    ex->assign(vectors, 0);
+    std::vector<double> g(M, 0.0);
+    for (size_t t = 0; t < vectors * M; ++t) {
+      if (!std::isfinite(v[t]) || std::fabs(v[t]) > 1e30) return false;
+      g[t % M] = std::max(g[t % M], std::fabs(v[t]));
+    }
+    const double least = *std::min_element(g.begin(), g.end());
+    if (!(least > 1e-30)) return false;
+    for (int a = 0; a < M; ++a) (*k)[a] = std::max(-20, std::ilogb(least) - std::ilogb(g[a]));
+    for (size_t t = 0; t < vectors; ++t) {
+      double m = 0.0;
+      for (int a = 0; a < M; ++a) m = std::max(m, std::ldexp(std::fabs(v[t * M + a]), (*k)[a]));
+      if (!(m > 1e-30)) continue;
+      (*ex)[t] = std::ilogb(m) + 1;
+      for (int a = 0; a < M; ++a)
+        (*out)[t * M + a] = fo_from_double(std::ldexp(v[t * M + a], (*k)[a]), (*ex)[t] + kFoUp);
+    }
+    return true;
+  };
+  std::vector<Fx> A, B, C, R;
+  std::vector<int> kA, kB, kC(1, 0), eA, eB, eC;
+  if (!scale(ops->vdm_A, op.M1, p1, &A, &kA, &eA) || !scale(ops->vdm_B, op.M2, (size_t)p1 * p1, &B, &kB, &eB) ||
+      (c.d == 3 && !scale(ops->vdm_C, M3, (size_t)p1 * p1 * p1, &C, &kC, &eC)))
+    return SSE_OK;
+  std::vector<signed char> T(c.n_p), K(c.n_q), eR(c.n_f, 0);
+  for (size_t t = 0; t < (size_t)p1 * p1 * (c.d == 3 ? p1 : 1); ++t) {
+    const int64_t l = ops->vdm_sigma_in[t];
+    if (l == 0) continue;
+    const int b1 = (int)(t % p1), b2 = (int)((t / p1) % p1);
+    const int e = eA[b1] + eB[b1 + p1 * b2] + (c.d == 3 ? eC[t] : 0);
+    if (std::abs(e) > 25) return SSE_OK;
+    T[l - 1] = (signed char)e;
+  }
+  for (int i = 0; i < c.n_q; ++i)
+    K[i] = (signed char)(kA[i / (op.M2 * M3)] + kB[(i / M3) % op.M2] + kC[i % M3]);
+  const CsrHost r = csc_to_csr(ops->R, false);
+  R.assign(std::max<size_t>(1, r.val.size()), Fx{0, 0});
+  for (int j = 0; j < c.n_f; ++j) {
+    double row = 0.0;
+    for (int q = r.ptr[j]; q < r.ptr[j + 1]; ++q) row += std::ldexp(std::fabs(r.val[q]), -K[r.idx[q]]);
+    if (!(row < 1e30)) return SSE_OK;
+    if (!(row > 1e-30)) continue;
+    eR[j] = (signed char)(std::ilogb(row) + 1);
+    for (int q = r.ptr[j]; q < r.ptr[j + 1]; ++q) R[q] = fo_from_double(std::ldexp(r.val[q], -K[r.idx[q]]), eR[j]);
+  }
+  cudaError_t e;
+  if ((e = upload(s, A.data(), A.size(), &fx.A)) || (e = upload(s, B.data(), B.size(), &fx.B)) ||
+      (c.d == 3 && (e = upload(s, C.data(), C.size(), &fx.C))) || (e = upload(s, R.data(), R.size(), &fx.R)) ||
+      (e = upload(s, eR.data(), eR.size(), &fx.eR)) || (e = upload(s, K.data(), K.size(), &fx.K)) ||
+      (e = upload(s, T.data(), T.size(), &fx.T)))
+    return cuda_fail(s, e, "fixed-point operators");
+  return SSE_OK;
+}
+
+// Fixed-point mass operators, by the same rule on memory as the metric terms
+int setup_fx_mass(sse_solver *s) {
+  KernelArgs &ka = s->ka;
+  const sse_config &c = s->cfg;
+  const size_t ne = c.n_e, n = ne * c.n_p * c.n_p;
+  size_t freeb = 0, totalb = 0;
+  cudaError_t e;
+  if (!ka.Ak) return SSE_OK;
+  if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
+  if (n * sizeof(Fx) > freeb / 4) return SSE_OK;
+  void *A, *eA, *eW;
+  if ((e = alloc(s, n * sizeof(Fx), &A)) || (e = alloc(s, ne * sizeof(int), &eA)) ||
+      (e = alloc(s, ne * sizeof(int), &eW)) ||
+      (e = launch_fx_mass_operators(ka, (Fx *)A, (int *)eA, (int *)eW, s->stream)) ||
+      (e = cudaStreamSynchronize(s->stream)))
+    return cuda_fail(s, e, "fixed-point mass operators");
+  ka.fx.A_k = (const Fx *)A;
+  ka.fx.eA = (const int *)eA;
+  ka.fx.eW = (const int *)eW;
+  ka.fx.on_a = 1;
   return SSE_OK;
 }
 
@@ -739,7 +834,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     // fx_ec_flux (gamma <= 1.7)
     ka.fx = FxTables{};
     if (c.law == SSE_EULER && c.two_point_flux == SSE_EC_FLUX && c.gamma > 1.0 && c.gamma <= 1.7 &&
-        (rc = setup_fx_pairs(s, vp_ij, vp_S, fp_C, fp_inc, &fx_lists)))
+        ((rc = setup_fx_pairs(s, vp_ij, vp_S, fp_C, fp_inc, &fx_lists)) || (rc = setup_fx_operators(s, ops))))
       return rc;
   }
 
@@ -952,6 +1047,17 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   // of 128 (p = 4 tets: 3.14 -> 3.09 ms per stage, fewer barrier stalls)
   ka.epb_a = (tpe >= 256 && nq + nf <= 256) ? epb * (tpe / 128) : epb;
   if ((size_t)ka.epb_a * ka.layA.team_doubles * 8 > 220 * 1024) ka.epb_a = epb;
+  if (ka.fx.T) {
+    // two volume or facet nodes a thread, and blocks of at least 128 threads
+    // (p = 3 tets: 64 threads 0.388 ms, 128 0.436; p = 5: 128 threads 0.823, 256
+    // 0.849; p = 4 triangles: 16 threads 0.106, 32 0.123)
+    int tpe_x = 16;
+    while (tpe_x < 256 && (nq + nf) / 2 > 1.414 * tpe_x) tpe_x *= 2;
+    ka.epb_ax = tpe_x < 128 ? 128 / tpe_x : 1;
+    ka.tpb_ax = ka.epb_ax * tpe_x;
+    finish(ka.layAx, {nc * std::max(np, nq), nc * std::max(np, nq), zsz, wsz, (3 * nc + 1) / 2});
+    if ((size_t)ka.epb_ax * ka.layAx.team_doubles * 8 > 220 * 1024) ka.fx.T = nullptr;
+  }
   // opt in to large dynamic shared memory for every kernel instantiation used
   size_t smA = (size_t)std::max(epb, ka.epb_a) * ka.layA.team_doubles * 8,
          smB = (size_t)epb * ka.layB.team_doubles * 8;
@@ -976,6 +1082,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     }
   }
   if (ka.fx.vp_ij && ((rc = setup_fx_lists(s, fx_lists)) || (rc = setup_fx_geometry(s)))) return rc;
+  if (ka.fx.T && (rc = setup_fx_mass(s))) return rc;
   if (ka.fx.on) {
     ka.layB = fx_layB;
     ka.fd_chunk = fx_fd_chunk;

@@ -62,7 +62,7 @@ SSE_HD long long fx_dot(const Fx *a, const Fx *b) {
   return h;
 }
 
-// x 2^(60 - e) for |x| < 2^(e + 2), truncated toward zero in magnitude (exact
+// x 2^(60 - e) for |x| < 2^(e + 3), truncated toward zero in magnitude (exact
 // when x's last bit is at least 2^(e - 60)); integer operations only
 SSE_HD long long fx_from_double(double x, int e) {
   const long long b = sse_bits(x);

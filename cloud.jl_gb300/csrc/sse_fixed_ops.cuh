@@ -1,0 +1,262 @@
+// sse_fixed_ops.cuh -- team-parallel operator applications in block fixed
+// point (sse_fixed.cuh), the counterparts of sse_ops.cuh for the FP64 form.
+//
+// A product with an operator entry is three integer multiply-adds, a tenth of
+// one FP64 FMA's issue time, so the contractions of an element leave the FP64
+// pipe altogether.
+//
+// Values here have 62 fraction bits, hi 2^31 + lo with lo in [-2^30, 2^30).
+// The entries of V's factors are scaled to at most 1/4 per mode vector (the
+// headroom that the sums of up to 8 cross products need; products are moved up
+// by 2 bits again) and per node: row i of V is taken times 2^K_i, K_i <= 0, about
+// the square root of the node's quadrature weight, because the orthonormal
+// basis grows like its inverse toward the collapsed vertex; without it the
+// modes' scales 2^T_l would cost the leading modes 5 to 8 bits.  With modal
+// values in a unit that bounds sum_l 2^T_l |x_l| no partial sum of the sum
+// factorisation exceeds the unit, and the unit is that tight for the values at
+// hand.
+#pragma once
+
+#include "sse_kernels.cuh"
+
+namespace sse {
+
+// v 2^-s to the nearest integer, 0 <= s < 63
+struct FxShift {
+  int s;
+  long long half;
+  __device__ __forceinline__ explicit FxShift(int s_) : s(s_), half((1LL << s_) >> 1) {}
+  __device__ __forceinline__ long long operator()(long long v) const { return (v + half) >> s; }
+};
+
+// FP64 value of a fixed-point sum v 2^e with two FMAs: the words of v as the
+// low bits of two doubles, their offsets taken out by exact FMAs
+struct FxUnit {
+  double lo, hi, off;  // 2^e, 2^(e + 32), their offsets
+  __device__ __forceinline__ explicit FxUnit(int e) {
+    lo = fx_pow2(e);
+    hi = fx_pow2(e + 32);
+    off = sse_from_bits(sse_bits(-(0x1p84 + 0x1p63 + 0x1p52)) + ((long long)e << 52));
+  }
+  __device__ __forceinline__ double operator()(long long v) const {
+    const double h = __hiloint2double(0x43300000, (int)(v >> 32) ^ 0x80000000);
+    const double l = __hiloint2double(0x43300000, (int)v);
+    return fma(l, lo, fma(h, hi, off));
+  }
+};
+
+constexpr int kFoLow = 31;       // bits of the low part
+constexpr int kFoUp = 2;         // operator entries are at most 2^-2
+__host__ __device__ __forceinline__ Fx fo_split(long long v) {
+  return Fx{(int)((unsigned)v << 1) >> 1, (int)((v + (1LL << (kFoLow - 1))) >> kFoLow)};
+}
+__device__ __forceinline__ long long fo_join(Fx a) { return ((long long)a.hi << kFoLow) + a.lo; }
+// x 2^(62 - e)
+__host__ __device__ __forceinline__ Fx fo_from_double(double x, int e) { return fo_split(fx_from_double(x, e - 2)); }
+
+// NC sums of products with one operator entry each
+template <int NC>
+struct FxSums {
+  long long h[NC], x[NC];
+  __device__ __forceinline__ FxSums() {
+#pragma unroll
+    for (int e = 0; e < NC; ++e) { h[e] = 0; x[e] = 0; }
+  }
+  // += a v[e stride]
+  __device__ __forceinline__ void add(Fx a, const Fx *v, int stride) {
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      const Fx b = v[e * stride];
+      x[e] = fx_wide(a.hi, b.lo, fx_wide(a.lo, b.hi, x[e]));
+      h[e] = fx_wide(a.hi, b.hi, h[e]);
+    }
+  }
+  // the sum, up by UP bits
+  template <int UP>
+  __device__ __forceinline__ long long value(int e) const {
+    return (long long)((unsigned long long)h[e] << UP) + (x[e] >> (kFoLow - UP));
+  }
+  template <int UP>
+  __device__ __forceinline__ void store(Fx *v, int stride) const {
+#pragma unroll
+    for (int e = 0; e < NC; ++e) v[e * stride] = fo_split(value<UP>(e));
+  }
+};
+
+// y (NC x nq, times 2^K_i) = V x (NC x np, times 2^T_l)
+template <int D, int NC>
+__device__ void fx_vdm_mul(const DevOps &op, const FxTables &fx, const Fx *x, Fx *y, Fx *Z, Fx *W, int lane, int tpe) {
+  const int np = op.np, nq = op.nq, p1 = op.p1, M1 = op.M1, M2 = op.M2;
+  const float rM2 = qrcp(M2), rM3 = qrcp(op.M3 > 0 ? op.M3 : 1);
+  if constexpr (D == 2) {
+    for (int s = lane; s < p1 * M2; s += tpe) {
+      const int b1 = qdiv(s, rM2), a2 = s - b1 * M2;
+      FxSums<NC> acc;
+      for (int b2 = 0; b2 < p1 - b1; ++b2) acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], x + modes_index2(op, b1, b2), np);
+      acc.template store<kFoUp>(Z + b1 * M2 + a2, p1 * M2);
+    }
+    __syncthreads();
+    for (int s = lane; s < M1 * M2; s += tpe) {
+      const int a1 = qdiv(s, rM2), a2 = s - a1 * M2;
+      FxSums<NC> acc;
+      for (int b1 = 0; b1 < p1; ++b1) acc.add(fx.A[a1 + M1 * b1], Z + b1 * M2 + a2, p1 * M2);
+      acc.template store<kFoUp>(y + M2 * a1 + a2, nq);
+    }
+    __syncthreads();
+  } else {
+    const int M3 = op.M3, nb12 = op.nb12;
+    for (int s = lane; s < nb12 * M3; s += tpe) {
+      const int q = qdiv(s, rM3), a3 = s - q * M3;
+      const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
+      FxSums<NC> acc;
+      for (int b3 = 0; b3 < p1 - b1 - b2; ++b3)
+        acc.add(fx.C[a3 + M3 * (b1 + p1 * (b2 + p1 * b3))], x + modes_index3(op, b1, b2, b3), np);
+      acc.template store<kFoUp>(Z + q * M3 + a3, nb12 * M3);
+    }
+    __syncthreads();
+    for (int s = lane; s < p1 * M2 * M3; s += tpe) {
+      const int r = qdiv(s, rM3), a3 = s - r * M3, b1 = qdiv(r, rM2), a2 = r - b1 * M2;
+      FxSums<NC> acc;
+      for (int b2 = 0; b2 < p1 - b1; ++b2)
+        acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], Z + op.b12_index[b1 + p1 * b2] * M3 + a3, nb12 * M3);
+      acc.template store<kFoUp>(W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+    }
+    __syncthreads();
+    for (int s = lane; s < M1 * M2 * M3; s += tpe) {
+      const int r = qdiv(s, rM3), a3 = s - r * M3, a1 = qdiv(r, rM2), a2 = r - a1 * M2;
+      FxSums<NC> acc;
+      for (int b1 = 0; b1 < p1; ++b1) acc.add(fx.A[a1 + M1 * b1], W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+      acc.template store<kFoUp>(y + (M2 * a1 + a2) * M3 + a3, nq);
+    }
+    __syncthreads();
+  }
+}
+
+// x (NC x np, without the factors 2^T_l) = V^T y (NC x nq, times 2^-K_i)
+template <int D, int NC>
+__device__ void fx_vdm_tmul(const DevOps &op, const FxTables &fx, const Fx *y, Fx *x, Fx *Z, Fx *W, int lane, int tpe) {
+  const int np = op.np, nq = op.nq, p1 = op.p1, M1 = op.M1, M2 = op.M2;
+  const float rM2 = qrcp(M2), rM3 = qrcp(op.M3 > 0 ? op.M3 : 1);
+  if constexpr (D == 2) {
+    for (int s = lane; s < p1 * M2; s += tpe) {
+      const int b1 = qdiv(s, rM2), a2 = s - b1 * M2;
+      FxSums<NC> acc;
+      for (int a1 = 0; a1 < M1; ++a1) acc.add(fx.A[a1 + M1 * b1], y + M2 * a1 + a2, nq);
+      acc.template store<kFoUp>(Z + b1 * M2 + a2, p1 * M2);
+    }
+    __syncthreads();
+    for (int l = lane; l < np; l += tpe) {
+      const int b1 = op.modes[l] & 0xff, b2 = (op.modes[l] >> 8) & 0xff;
+      FxSums<NC> acc;
+      for (int a2 = 0; a2 < M2; ++a2) acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], Z + b1 * M2 + a2, p1 * M2);
+      acc.template store<kFoUp>(x + l, np);
+    }
+    __syncthreads();
+  } else {
+    const int M3 = op.M3, nb12 = op.nb12;
+    for (int s = lane; s < p1 * M2 * M3; s += tpe) {
+      const int r = qdiv(s, rM3), a3 = s - r * M3, b1 = qdiv(r, rM2), a2 = r - b1 * M2;
+      FxSums<NC> acc;
+      for (int a1 = 0; a1 < M1; ++a1) acc.add(fx.A[a1 + M1 * b1], y + (M2 * a1 + a2) * M3 + a3, nq);
+      acc.template store<kFoUp>(W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+    }
+    __syncthreads();
+    for (int s = lane; s < nb12 * M3; s += tpe) {
+      const int q = qdiv(s, rM3), a3 = s - q * M3;
+      const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
+      FxSums<NC> acc;
+      for (int a2 = 0; a2 < M2; ++a2)
+        acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+      acc.template store<kFoUp>(Z + q * M3 + a3, nb12 * M3);
+    }
+    __syncthreads();
+    for (int l = lane; l < np; l += tpe) {
+      const int b1 = op.modes[l] & 0xff, b2 = (op.modes[l] >> 8) & 0xff, b3 = (op.modes[l] >> 16) & 0xff;
+      const int q = op.b12_index[b1 + p1 * b2];
+      FxSums<NC> acc;
+      for (int a3 = 0; a3 < M3; ++a3) acc.add(fx.C[a3 + M3 * (b1 + p1 * (b2 + p1 * b3))], Z + q * M3 + a3, nb12 * M3);
+      acc.template store<kFoUp>(x + l, np);
+    }
+    __syncthreads();
+  }
+}
+
+// y (NC x np) = A x (NC x np) for the element's mass operator A (column-major,
+// the absolute sums of its rows at most 1)
+template <int NC>
+__device__ void fx_mass(const Fx *A, const Fx *x, Fx *y, int np, int lane, int tpe) {
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = t / np, a = t - e * np;
+    FxSums<1> acc;
+    const Fx *xe = x + e * np;
+#pragma unroll 4
+    for (int b = 0; b < np; ++b) acc.add(A[b * np + a], xe + b, 0);
+    acc.template store<0>(y + t, 0);
+  }
+  __syncthreads();
+}
+
+// Unit exponents of the NC vectors of modal values: unit[e] with
+// sum_l 2^T_l |x_l| < 2^unit[e]; each group of `width` lanes takes whole
+// components.  kFxBad: not finite (or beyond 2^900).
+constexpr int kFxBad = 100000;
+
+// x in FP64
+template <int NC>
+__device__ __forceinline__ void fx_modal_units(const double *x, const signed char *T, int np, int *unit, int lane,
+                                               int tpe) {
+  const int width = tpe < 32 ? tpe : 32, groups = tpe / width, g = lane / width, w = lane - g * width;
+  for (int e0 = 0; e0 < NC; e0 += groups) {
+    const int e = e0 + g;
+    int m = -2000;
+    if (e < NC)
+      for (int l = w; l < np; l += width) {
+        const int ex = (__double2hiint(x[e * np + l]) >> 20) & 0x7ff;
+        if (ex > 0) m = max(m, ex == 0x7ff ? kFxBad : ex - 1023 + T[l]);
+      }
+    for (int o = width >> 1; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float s = 0.f;
+    if (e < NC)
+      for (int l = w; l < np; l += width) {
+        const double v = x[e * np + l];
+        const int ex = (__double2hiint(v) >> 20) & 0x7ff, d = m - (ex - 1023 + T[l]);
+        // the mantissa, rounded up, times 2^-d
+        const float f = __int_as_float(0x3f800000 + ((__double2hiint(v) & 0xfffff) << 3) + 8);
+        if (ex > 0 && d < 100) s += f * __int_as_float((127 - d) << 23);
+      }
+    for (int o = width >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (e < NC && w == 0)
+      unit[e] = m > 900 ? kFxBad : max(-800, m + (__float_as_int(s * 1.0001f) >> 23) - 126);
+  }
+}
+
+// x in fixed point, unit 2^0, times 2^T_l where scaled
+template <int NC>
+__device__ __forceinline__ void fx_modal_units(const Fx *x, const signed char *T, int np, int *unit, int lane, int tpe) {
+  const int width = tpe < 32 ? tpe : 32, groups = tpe / width, g = lane / width, w = lane - g * width;
+  for (int e0 = 0; e0 < NC; e0 += groups) {
+    const int e = e0 + g;
+    float s = 0.f;
+    if (e < NC)
+      for (int l = w; l < np; l += width)
+        s += ((float)abs((float)x[e * np + l].hi) + 1.f) * __int_as_float((127 - kFoLow + T[l]) << 23);
+    for (int o = width >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (e < NC && w == 0) unit[e] = (__float_as_int(s * 1.0001f) >> 23) - 126;
+  }
+}
+
+// FP64 value of v in unit 2^(unit + more); NaN for kFxBad
+__device__ __forceinline__ double fx_value(long long v, int unit, int more = 0) {
+  const int e = unit + more - 2 * kFoLow;
+  if (e > 900) return __longlong_as_double(0x7ff8000000000000LL);
+  return e < -900 ? 0.0 : FxUnit(e)(v);
+}
+__device__ __forceinline__ double fx_value(Fx v, int unit, int more = 0) { return fx_value(fo_join(v), unit, more); }
+
+// x 2^s, |s| < 60, the result at most 1
+__device__ __forceinline__ Fx fx_scale(Fx a, int s) {
+  const long long v = fo_join(a);
+  return fo_split(s >= 0 ? (long long)((unsigned long long)v << s) : FxShift(-s)(v));
+}
+
+}  // namespace sse

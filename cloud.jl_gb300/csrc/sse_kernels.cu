@@ -19,6 +19,7 @@
 #include "sse_kernels.cuh"
 #include "sse_tma.cuh"
 #include "sse_ops.cuh"
+#include "sse_fixed_ops.cuh"
 
 namespace sse {
 
@@ -112,6 +113,160 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
   __syncthreads();
   for (int t = lane; t < NC * nf; t += tpe)
     if (live) uf_out[t] = F[t];
+}
+
+// ---------------------------------------------------------------------------
+// Phase A of flux differencing on a modal tensor-product basis (Euler), the
+// operators in block fixed point (sse_fixed_ops.cuh)
+//
+// nodal_values_kernel's FP64 pipe was 87 % busy; V, V^T, the mass solve and R
+// were 29 K of its 47 K FP64 instructions per p = 4 tet.  Here they are integer
+// multiply-adds and FP64 is left to the entropy-variable maps, about 19 K.  64
+// registers keep 32 warps on an SM (24 warps 1.63 ms, 40 with spills 1.53).
+// 24,576 p = 4 tets 2.69 -> 1.47 ms, 7,986 p = 5 tets 1.55 -> 0.82 ms, 13,182
+// p = 2 tets 0.383 -> 0.210 ms, 8,192 p = 4 triangles 0.149 -> 0.106 ms.  The
+// residual's error against extended precision falls to 0.4 to 0.8 of that
+// with the FP64 operators (40 modal configurations, p = 2 to 6).
+// ---------------------------------------------------------------------------
+template <int D, int NC>
+__global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_constant__ KernelArgs ka) {
+  static_assert(NC == D + 2, "Euler");
+  extern __shared__ double smem[];
+  const DevOps &op = ka.op;
+  const Physics &ph = ka.ph;
+  const FxTables &fx = ka.fx;
+  const Layout &L = ka.layAx;
+  const int tpe = blockDim.x / ka.epb;
+  const int team = threadIdx.x / tpe, lane = threadIdx.x % tpe;
+  const int k = blockIdx.x * ka.epb + team;
+  const bool live = k < ka.ne;
+  const int kk = live ? k : 0;
+  const int np = op.np, nq = op.nq, nf = op.nf;
+  double *base = smem + (size_t)team * L.team_doubles;
+  Fx *X = reinterpret_cast<Fx *>(base + L.off[0]), *Y = reinterpret_cast<Fx *>(base + L.off[1]),
+     *Z = reinterpret_cast<Fx *>(base + L.off[2]), *W = reinterpret_cast<Fx *>(base + L.off[3]);
+  double *Xd = base + L.off[0], *Yd = base + L.off[1];
+  int *unit = reinterpret_cast<int *>(base + L.off[4]), *unit2 = unit + NC;
+  unsigned *key = reinterpret_cast<unsigned *>(unit + 2 * NC);
+
+  // u_q = V u
+  const double *uk = ka.u + (size_t)kk * NC * np;
+  for (int t = lane; t < NC * np; t += tpe) Yd[t] = uk[t];
+  if (lane < NC) key[lane] = 0u;
+  __syncthreads();
+  fx_modal_units<NC>(Yd, fx.T, np, unit, lane, tpe);
+  __syncthreads();
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = t / np;
+    X[t] = fo_from_double(Yd[t], unit[e] - fx.T[t - e * np]);
+  }
+  __syncthreads();
+  fx_vdm_mul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  // w_q = WJ c2e(u_q)
+  const double *WJ = ka.geo.WJ + (size_t)kk * nq;
+  unsigned kmax[NC];
+#pragma unroll
+  for (int e = 0; e < NC; ++e) kmax[e] = 0u;
+  for (int i = lane; i < nq; i += tpe) {
+    double ui[NC], wi[NC];
+#pragma unroll
+    for (int e = 0; e < NC; ++e) ui[e] = fx_value(Y[e * nq + i], unit[e], -fx.K[i]);
+    if (!(ui[0] > 0.0)) ka.flag_nonphysical();
+    cons_to_entropy_fast<D>(ph.gamma, ph.gm1, ph.igm1, ui, wi, op.math_tab);
+    const double s = WJ[i];
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      kmax[e] = max(kmax[e], (unsigned)__double2hiint(wi[e]) & 0x7fffffffu);
+      Xd[e * nq + i] = wi[e] * s;
+    }
+  }
+  const int width = tpe < 32 ? tpe : 32;
+#pragma unroll
+  for (int e = 0; e < NC; ++e) {
+    for (int o = width >> 1; o > 0; o >>= 1) kmax[e] = max(kmax[e], __shfl_xor_sync(0xffffffffu, kmax[e], o));
+    if ((lane & (width - 1)) == 0) atomicMax(key + e, kmax[e]);
+  }
+  __syncthreads();
+  // sum_i |WJ_i w_i| 2^-K_i < 2^eW max |w|
+  if (lane < NC) unit[lane] = key[lane] >= (1023u + 900u) << 20 ? kFxBad : max(-800, fx_exponent(key[lane])) + fx.eW[kk];
+  __syncthreads();
+  for (int i = lane; i < nq; i += tpe)
+#pragma unroll
+    for (int e = 0; e < NC; ++e) X[e * nq + i] = fo_from_double(Xd[e * nq + i], unit[e] + fx.K[i]);
+  __syncthreads();
+  // V^T, then the mass solve in the unit of its own input, then V in the unit
+  // of its own; the last unit[e] is that of w_q
+  fx_vdm_tmul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  fx_modal_units<NC>(Y, fx.T, np, unit2, lane, tpe);
+  __syncthreads();
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = t / np;
+    Y[t] = fx_scale(Y[t], fx.T[t - e * np] - unit2[e]);
+  }
+  __syncthreads();
+  if (lane < NC && unit[lane] != kFxBad) unit[lane] += unit2[lane] + fx.eA[kk];
+  fx_mass<NC>(fx.A_k + (size_t)kk * np * np, Y, X, np, lane, tpe);
+  fx_modal_units<NC>(X, fx.T, np, unit2, lane, tpe);
+  __syncthreads();
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = t / np;
+    X[t] = fx_scale(X[t], fx.T[t - e * np] - unit2[e]);
+  }
+  if (lane < NC && unit[lane] != kFxBad) unit[lane] += unit2[lane];
+  __syncthreads();
+  fx_vdm_mul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  // u_q = e2c(w_q), u_f = e2c(R w_q)
+  for (int t = lane; t < nq + nf; t += tpe) {
+    const bool vol = t < nq;
+    const int r = vol ? t : t - nq, n = vol ? nq : nf;
+    double wi[NC], ui[NC];
+    if (vol) {
+#pragma unroll
+      for (int e = 0; e < NC; ++e) wi[e] = fx_value(Y[e * nq + r], unit[e], -fx.K[r]);
+    } else {
+      FxSums<NC> acc;
+      for (int q = op.R_ptr[r]; q < op.R_ptr[r + 1]; ++q) acc.add(fx.R[q], Y + op.R_idx[q], nq);
+#pragma unroll
+      for (int e = 0; e < NC; ++e) wi[e] = fx_value(acc.template value<0>(e), unit[e], fx.eR[r]);
+    }
+    entropy_to_cons_fast<D>(ph.gamma, ph.gm1, ph.igm1, ph.log_gm1, wi, ui, op.math_tab);
+    double *dst = (vol ? ka.u_q : ka.u_f) + (size_t)kk * NC * n + r;
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      if (live) dst[(size_t)e * n] = ui[e];
+      if (!(ui[0] > 0.0) || !isfinite(ui[e])) ka.flag_nonphysical();
+    }
+  }
+}
+
+// Fixed-point mass operators of phase A: A_k scaled by 2^-eA so that the
+// absolute sums of its rows are at most 1, and eW with sum_i W J 2^-K_i < 2^eW
+__global__ void __launch_bounds__(128) fx_mass_operator_kernel(const double *__restrict__ Ak, const double *__restrict__ WJ,
+                                                               const signed char *__restrict__ K, int np, int nq,
+                                                               Fx *oA, int *oeA, int *oeW) {
+  __shared__ unsigned row;
+  __shared__ double part[128];
+  const size_t k = blockIdx.x;
+  const double *A = Ak + k * np * np;
+  if (threadIdx.x == 0) row = 0u;
+  double w = 0.0;
+  for (int i = threadIdx.x; i < nq; i += blockDim.x) w += fabs(WJ[k * nq + i]) * fx_pow2(-K[i]);
+  part[threadIdx.x] = w;
+  __syncthreads();
+  for (int a = threadIdx.x; a < np; a += blockDim.x) {
+    double s = 0.0;
+    for (int b = 0; b < np; ++b) s += fabs(A[b * np + a]);
+    atomicMax(&row, (unsigned)__double2hiint(s * (1.0 + 1e-6)));
+  }
+  __syncthreads();
+  const int e = min(400, max(-400, fx_exponent(row)));
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int t = 0; t < (int)blockDim.x; ++t) s += part[t];
+    oeA[k] = e;
+    oeW[k] = min(400, max(-400, fx_exponent((unsigned)__double2hiint(s * (1.0 + 1e-6)))));
+  }
+  for (int t = threadIdx.x; t < np * np; t += blockDim.x) oA[k * np * np + t] = fo_from_double(A[t], e);
 }
 
 // ---------------------------------------------------------------------------
@@ -622,30 +777,6 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // configurations (modal and nodal, p = 2 to 6, both metrics and interface
 // fluxes).
 // ---------------------------------------------------------------------------
-
-// FP64 value of a fixed-point sum v 2^e with two FMAs: the words of v as the
-// low bits of two doubles, their offsets taken out by exact FMAs
-struct FxUnit {
-  double lo, hi, off;  // 2^e, 2^(e + 32), their offsets
-  __device__ __forceinline__ explicit FxUnit(int e) {
-    lo = fx_pow2(e);
-    hi = fx_pow2(e + 32);
-    off = -(0x1p84 + 0x1p63 + 0x1p52) * lo;
-  }
-  __device__ __forceinline__ double operator()(long long v) const {
-    const double h = __hiloint2double(0x43300000, (int)(v >> 32) ^ 0x80000000);
-    const double l = __hiloint2double(0x43300000, (int)v);
-    return fma(l, lo, fma(h, hi, off));
-  }
-};
-
-// v 2^-s to the nearest integer, 0 <= s < 63
-struct FxShift {
-  int s;
-  long long half;
-  __device__ __forceinline__ explicit FxShift(int s_) : s(s_), half((1LL << s_) >> 1) {}
-  __device__ __forceinline__ long long operator()(long long v) const { return (v + half) >> s; }
-};
 
 // Exponents of an element's units from the extremes of its node values (upper
 // words of the largest density, enthalpy and |velocity component| and
@@ -2062,6 +2193,9 @@ cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
     if (ka.fd) set((const void *)fd_time_derivative_kernel<D, NC>, smB);
     if (!ka.fd) set((const void *)std_time_derivative_kernel<D, NC>, smB);
   });
+  if (ka.fx.T)
+    set(ka.op.d == 2 ? (const void *)nodal_values_fx_kernel<2, 4> : (const void *)nodal_values_fx_kernel<3, 5>,
+        (size_t)ka.epb_ax * ka.layAx.team_doubles * sizeof(double));
   if (ka.fx.vp_ij)
     set(ka.op.d == 2 ? (const void *)fd_time_derivative_fx_kernel<2, 4>
                      : (const void *)fd_time_derivative_fx_kernel<3, 5>, smB);
@@ -2080,6 +2214,17 @@ cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st) {
     if (ka.op.d == 2 && ka.op.nc == 4) nodal_values_mixed_kernel<2, 4><<<grida, ka.tpb, sm, st>>>(km);
     else if (ka.op.d == 3 && ka.op.nc == 5) nodal_values_mixed_kernel<3, 5><<<grida, ka.tpb, sm, st>>>(km);
     else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+  }
+  // the fixed-point operators wherever their tables exist (EC flux, modal
+  // tensor-product basis)
+  if (ka.fx.on_a) {
+    KernelArgs kx = ka;
+    kx.epb = ka.epb_ax;
+    const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
+    const size_t smx = (size_t)kx.epb * ka.layAx.team_doubles * sizeof(double);
+    if (ka.op.d == 2) nodal_values_fx_kernel<2, 4><<<gridx, ka.tpb_ax, smx, st>>>(kx);
+    else nodal_values_fx_kernel<3, 5><<<gridx, ka.tpb_ax, smx, st>>>(kx);
     return cudaGetLastError();
   }
   // the FP64 phase A has its own team geometry (epb_a elements per block of
@@ -2190,6 +2335,11 @@ cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, 
                                cudaStream_t st) {
   if (ka.op.d == 2) fx_geometry_kernel<2><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
   else fx_geometry_kernel<3><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_mass_operators(const KernelArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st) {
+  fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.op.np, ka.op.nq, A, eA, eW);
   return cudaGetLastError();
 }
 

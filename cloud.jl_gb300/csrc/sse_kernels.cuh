@@ -52,6 +52,14 @@ struct FxTables {
   const Fx *hnf;      // halfnJf in units 2^(eG - eC)
   const Fx *bn;       // BJf n_f / 2 in units 2^(eG - n), d x nf x ne
   const signed char *n;  // node shifts n_i, (nq + nf) x ne
+  // phase A (on_a), see sse_fixed_ops.cuh: the factors of a tensor-product V,
+  // scaled per node (2^K_i) and mode (2^T_l); R times 2^-K_q, row j in units
+  // 2^eR_j (absolute row sums at most 1; CSR values); the mass operators in
+  // units 2^eA (absolute row sums at most 1) and 2^eW > sum of W J 2^-K
+  int on_a;
+  const Fx *A, *B, *C, *R, *A_k;
+  const signed char *T, *K, *eR;
+  const int *eA, *eW;
 };
 constexpr int kFxMaxK = 30;  // largest k_p
 constexpr int kFxNone = -100000;
@@ -62,6 +70,7 @@ struct KernelArgs {
   DevGeo geo;
   Physics ph;
   Layout layA, layB;
+  Layout layAx;      // fixed-point phase A: 0 X, 1 Y, 2 Z, 3 W, 4 units and extremes
   Layout layBx;      // fixed-point phase B: 0 facet fluxes, 1 r_q, 2 pair buffer and tail scratch,
                      // 3 node values, 4 float pairs, 5 extremes, 6 node shifts
   Layout layBm;      // mixed-form phase B layout, offsets and team size in floats:
@@ -105,6 +114,7 @@ struct KernelArgs {
   int fd_chunk;      // pairs per chunk in the FP64 flux-differencing passes
   int fx_chunk;      // pairs per chunk in the fixed-point passes
   int vp_split;      // volume pairs per interface lane in the one-chunk pass (0: even split)
+  int epb_ax, tpb_ax;  // elements and threads per block of the fixed-point phase A
   int epb_bx, tpb_bx;  // elements and threads per block of the fixed-point phase B
   int epb_bm;        // elements per block of the FP32 phase-B kernel (blocks of tpb threads)
   int epb_am;        // elements per block of the mixed phase-A kernel (blocks of tpb threads)
@@ -200,6 +210,8 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st);
 // the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG)
 cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st);
+// the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW)
+cudaError_t launch_fx_mass_operators(const KernelArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st);
 cudaError_t launch_mass_operator(const KernelArgs &ka, double *Ak, cudaStream_t st);
 cudaError_t launch_energy(const KernelArgs &ka, const double *u, const double *dudt, double *partial,
                           cudaStream_t st);

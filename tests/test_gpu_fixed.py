@@ -81,3 +81,39 @@ def test_fluid_at_rest_stays_at_rest(gpu_lib):
     u = S.initialize(_Flow(3, 1.4, 0.0, 0.2), host.sd)
     r = cases.PKG.GB300Solver(host).residual(u)
     assert np.all(r[:, 0] == 0.0) and np.all(r[:, 4] == 0.0)
+
+
+@pytest.mark.parametrize("shape,p,cells", [("Tri", 1, 3), ("Tri", 7, 2), ("Tri", 8, 2), ("Tet", 1, 1), ("Tet", 3, 1),
+                                           ("Tet", 6, 1)])
+@pytest.mark.parametrize("a,b", [(1.0, 1.0), (3.0e-9, 2.0e5), (7.0e12, 1.0e-6)])
+def test_operators_of_the_projection(gpu_lib, shape, p, cells, a, b):
+    """Fixed-point operators of the entropy projection at the smallest and
+    largest degrees they take (and p = 8, which keeps FP64), in other units of
+    density (a) and velocity (b), with a vanishing momentum component: to the
+    parity tolerance of nodal values, 1e-12 of each variable."""
+    host = _host(shape, p, cells, "ModalTensor")
+    u = S.initialize(_Flow(host.cfg.d, 1.4, 0.4, 0.1), host.sd)
+    u[:, 2] = 0.0
+    u[:, 0] *= a
+    u[:, 1:-1] *= a * b
+    u[:, -1] *= a * b * b
+    got_q, got_f = cases.PKG.GB300Solver(host).nodal_values(u)
+    want_q, want_f = Oracle(host).nodal_values(u)
+    speed = np.abs(want_q[:, 1]).max()
+    for e in range(host.N_c):
+        scale = speed if 0 < e < host.N_c - 1 else np.abs(want_q[:, e]).max()
+        assert np.abs(got_q[:, e] - want_q[:, e]).max() <= 1.0e-12 * scale
+        assert np.abs(got_f[e] - want_f[e]).max() <= 1.0e-12 * scale
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -1.0])
+@pytest.mark.parametrize("variable", [0, 1, -1])
+def test_non_physical_states_are_reported(gpu_lib, value, variable):
+    if value == -1.0 and variable == 1:
+        pytest.skip("a negative momentum is physical")
+    host = _host("Tet", 2, 1, "ModalTensor")
+    u = S.initialize(_Flow(3, 1.4, 0.4, 0.1), host.sd)
+    u[host.N_e - 1, variable] = value
+    with pytest.raises(cases.PKG.SSEError) as err:
+        cases.PKG.GB300Solver(host).residual(u)
+    assert err.value.code == 4
