@@ -295,32 +295,77 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
   return SSE_OK;
 }
 
-// The incidence lists of the fixed-point passes, with each node's range in
-// every chunk of ka.fx_chunk pairs.
-int setup_fx_lists(sse_solver *s, const FxLists &lists) {
-  FxTables &fx = s->ka.fx;
-  const int CH = s->ka.fx_chunk;
-  auto flatten = [&](const std::vector<std::vector<int>> &inc, int pairs, int *chunks, const int **ptr_d,
-                     const int **inc_d) {
-    *chunks = (pairs + CH - 1) / CH;
-    const size_t n = inc.size();
-    std::vector<int> flat, ptr((*chunks + 1) * n);
-    for (size_t t = 0; t < n; ++t) {
+// The node sums of the fixed-point passes (FxTables::Sums): in every chunk of
+// ka.fx_chunk pairs each node's list in parts of at most `most` entries, the
+// `most` for which the team takes the fewest steps; a node's 1, 2 or 4 parts are
+// adjacent tasks.
+int setup_fx_sums(sse_solver *s, const FxLists &lists) {
+  KernelArgs &ka = s->ka;
+  const int CH = ka.fx_chunk, tpe = ka.tpb_bx / ka.epb_bx;
+  auto build = [&](const std::vector<std::vector<int>> &inc, int pairs, FxTables::Sums *S) {
+    const int chunks = (pairs + CH - 1) / CH, n = (int)inc.size();
+    std::vector<int> flat, first(n + 1, 0);
+    std::vector<std::vector<int>> begin(chunks + 1, std::vector<int>(n));  // of each node's entries of a chunk
+    for (int t = 0; t < n; ++t) {
       size_t q = 0;
-      for (int c = 0; c <= *chunks; ++c) {
+      for (int c = 0; c <= chunks; ++c) {
         while (q < inc[t].size() && (inc[t][q] >> 8) / CH < c) ++q;
-        ptr[c * n + t] = (int)(flat.size() + q);
+        begin[c][t] = first[t] + (int)q;
       }
       flat.insert(flat.end(), inc[t].begin(), inc[t].end());
+      first[t + 1] = (int)flat.size();
+    }
+    std::vector<std::vector<int2>> task(chunks);
+    int tasks = 0;
+    for (int c = 0; c < chunks; ++c) {
+      auto len = [&](int t) { return begin[c + 1][t] - begin[c][t]; };
+      auto parts = [&](int t, int most) { return len(t) <= most ? 0 : (len(t) <= 2 * most ? 1 : 2); };
+      int longest = 1, best = 0;
+      for (int t = 0; t < n; ++t) longest = std::max(longest, len(t));
+      long cost = 0;
+      for (int most = (longest + 3) / 4; most <= longest; ++most) {
+        long count = 0;
+        for (int t = 0; t < n; ++t) count += 1 << parts(t, most);
+        // a task costs about eight steps beside its own (p = 2 tets: 0.297 ms,
+        // with three 0.306)
+        const long steps = (count + tpe - 1) / tpe * (most + 8);
+        if (best == 0 || steps < cost) { best = most; cost = steps; }
+      }
+      // nodes of many parts first: groups stay aligned
+      for (int g = 2; g >= 0; --g)
+        for (int t = 0; t < n; ++t) {
+          if (parts(t, best) != g) continue;
+          for (int k = 0; k < 1 << g; ++k) {
+            const int a = len(t) * k >> g, b = len(t) * (k + 1) >> g;
+            task[c].push_back(make_int2(begin[c][t] + a, t | (b - a) << 16 | g << 28));
+          }
+        }
+      tasks = std::max(tasks, (int)task[c].size());
+    }
+    tasks = (tasks + tpe - 1) / tpe * tpe;
+    std::vector<int2> all;
+    for (auto &v : task) {
+      v.resize(tasks, make_int2(0, (int)(0xfu << 28)));
+      all.insert(all.end(), v.begin(), v.end());
     }
     if (flat.empty()) flat.push_back(0);
-    cudaError_t e = upload(s, ptr.data(), ptr.size(), ptr_d);
-    return e ? e : upload(s, flat.data(), flat.size(), inc_d);
+    S->chunks = chunks;
+    S->tasks = tasks;
+    cudaError_t e = upload(s, flat.data(), flat.size(), &S->inc);
+    if (e == cudaSuccess) e = upload(s, first.data(), first.size(), &S->first);
+    return e ? e : upload(s, all.data(), all.size(), &S->task);
   };
+  // nodes take 16 bits of a task, entries of one node 12
+  size_t most = 0;
+  for (const auto *l : {&lists.vol, &lists.fac})
+    for (const auto &v : *l) most = std::max(most, v.size());
+  if (most >= 1 << 12) {
+    ka.fx = FxTables{};
+    return SSE_OK;
+  }
   cudaError_t e;
-  if ((e = flatten(lists.vol, s->ka.op.nvp, &fx.vp_chunks, &fx.vp_ptr, &fx.vp_inc)) ||
-      (e = flatten(lists.fac, s->ka.op.nfp + s->ka.op.nf, &fx.fp_chunks, &fx.fp_ptr, &fx.fp_inc)))
-    return cuda_fail(s, e, "fixed-point incidence lists");
+  if ((e = build(lists.vol, ka.op.nvp, &ka.fx.vol)) || (e = build(lists.fac, ka.op.nfp + ka.op.nf, &ka.fx.fac)))
+    return cuda_fail(s, e, "fixed-point node sums");
   return SSE_OK;
 }
 
@@ -1081,7 +1126,8 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       ka.Ak = (const double *)p;
     }
   }
-  if (ka.fx.vp_ij && ((rc = setup_fx_lists(s, fx_lists)) || (rc = setup_fx_geometry(s)))) return rc;
+  if (ka.fx.vp_ij && (rc = setup_fx_sums(s, fx_lists))) return rc;
+  if (ka.fx.vp_ij && (rc = setup_fx_geometry(s))) return rc;
   if (ka.fx.T && (rc = setup_fx_mass(s))) return rc;
   if (ka.fx.on) {
     ka.layB = fx_layB;

@@ -29,21 +29,16 @@ struct FxShift {
   __device__ __forceinline__ long long operator()(long long v) const { return (v + half) >> s; }
 };
 
-// FP64 value of a fixed-point sum v 2^e with two FMAs: the words of v as the
-// low bits of two doubles, their offsets taken out by exact FMAs
-struct FxUnit {
-  double lo, hi, off;  // 2^e, 2^(e + 32), their offsets
-  __device__ __forceinline__ explicit FxUnit(int e) {
-    lo = fx_pow2(e);
-    hi = fx_pow2(e + 32);
-    off = sse_from_bits(sse_bits(-(0x1p84 + 0x1p63 + 0x1p52)) + ((long long)e << 52));
-  }
-  __device__ __forceinline__ double operator()(long long v) const {
-    const double h = __hiloint2double(0x43300000, (int)(v >> 32) ^ 0x80000000);
-    const double l = __hiloint2double(0x43300000, (int)v);
-    return fma(l, lo, fma(h, hi, off));
-  }
-};
+// v 2^e to the nearest double, |e| <= 900, by integer operations (two FP64 FMAs
+// would take the place of a hundred of them)
+__device__ __forceinline__ double fx_to_double(long long v, int e) {
+  const long long s = v >> 63;
+  const unsigned long long a = (unsigned long long)((v ^ s) - s);
+  const int z = __clzll((long long)a);
+  const unsigned long long m = a << z;  // [2^63, 2^64), and v 2^e = m 2^(e - z)
+  const unsigned long long b = ((unsigned long long)(1085 + e - z) << 52) + (m >> 11) + ((m >> 10) & 1);
+  return a == 0 ? 0.0 : __longlong_as_double((long long)(b | ((unsigned long long)s & 0x8000000000000000ULL)));
+}
 
 constexpr int kFoLow = 31;       // bits of the low part
 constexpr int kFoUp = 2;         // operator entries are at most 2^-2
@@ -249,7 +244,7 @@ __device__ __forceinline__ void fx_modal_units(const Fx *x, const signed char *T
 __device__ __forceinline__ double fx_value(long long v, int unit, int more = 0) {
   const int e = unit + more - 2 * kFoLow;
   if (e > 900) return __longlong_as_double(0x7ff8000000000000LL);
-  return e < -900 ? 0.0 : FxUnit(e)(v);
+  return e < -900 ? 0.0 : fx_to_double(v, e);
 }
 __device__ __forceinline__ double fx_value(Fx v, int unit, int more = 0) { return fx_value(fo_join(v), unit, more); }
 

@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
 // were 29 K of its 47 K FP64 instructions per p = 4 tet.  Here they are integer
 // multiply-adds and FP64 is left to the entropy-variable maps, about 19 K.  64
 // registers keep 32 warps on an SM (24 warps 1.63 ms, 40 with spills 1.53).
-// 24,576 p = 4 tets 2.69 -> 1.47 ms, 7,986 p = 5 tets 1.55 -> 0.82 ms, 13,182
-// p = 2 tets 0.383 -> 0.210 ms, 8,192 p = 4 triangles 0.149 -> 0.106 ms.  The
+// 24,576 p = 4 tets 2.69 -> 1.38 ms, 7,986 p = 5 tets 1.55 -> 0.76 ms, 13,182
+// p = 2 tets 0.383 -> 0.185 ms, 8,192 p = 4 triangles 0.149 -> 0.093 ms.  The
 // residual's error against extended precision falls to 0.4 to 0.8 of that
 // with the FP64 operators (40 modal configurations, p = 2 to 6).
 // ---------------------------------------------------------------------------
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
 #pragma unroll
       for (int e = 0; e < NC; ++e) wi[e] = fx_value(acc.template value<0>(e), unit[e], fx.eR[r]);
     }
-    entropy_to_cons_fast<D>(ph.gamma, ph.gm1, ph.igm1, ph.log_gm1, wi, ui, op.math_tab);
+    entropy_to_cons_pressure<D>(ph.gamma, ph.igm1, wi, ui, op.math_tab);
     double *dst = (vol ? ka.u_q : ka.u_f) + (size_t)kk * NC * n + r;
 #pragma unroll
     for (int e = 0; e < NC; ++e) {
@@ -770,13 +770,52 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // tail.  Metric terms are read through L1, which leaves shared memory for
 // three blocks of 256 threads on an SM (80 registers): while one block is in its
 // FP64 part the others keep the integer pipes busy (staged in shared memory,
-// two blocks: 3.58 ms against 2.48).  24,576 p = 4 tets: 8.86 -> 2.48 ms; 7,986
-// p = 5 tets 6.5 -> 2.02 ms; 13,182 p = 2 tets 0.96 -> 0.316 ms; 8,192 p = 4
-// triangles 0.365 -> 0.145 ms.  The error against the
+// two blocks: 3.58 ms against 2.48).  24,576 p = 4 tets: 8.86 -> 2.42 ms; 7,986
+// p = 5 tets 6.5 -> 1.92 ms; 13,182 p = 2 tets 0.96 -> 0.297 ms; 8,192 p = 4
+// triangles 0.365 -> 0.134 ms.  The tail in fixed point too measured 2.54 ms at
+// p = 4 (more barriers, and no FP64 part left to overlap) and, its inputs being
+// sums of all nodes, less exact; it stays in FP64.  The error against the
 // extended-precision residual is 0.81 to 1.00 of the FP64 passes' own on 60
 // configurations (modal and nodal, p = 2 to 6, both metrics and interface
 // fluxes).
 // ---------------------------------------------------------------------------
+
+// Each node's sum of its pairs' contributions (at diff + NC pair), shifted to
+// the node's unit, handed to sink(node, sums).  A list longer than the others is
+// summed by two or four adjacent lanes (a p = 4 tet's facet lists have 5 entries
+// but 25 on the collapsed face: 13 steps instead of 25; 24,576 tets 2.52 ->
+// 2.42 ms, 7,986 p = 5 tets 2.05 -> 1.92 ms).
+template <int NC, typename Sink>
+__device__ __forceinline__ void fx_node_sums(const FxTables::Sums &S, int c, const long long *diff, const signed char *ns,
+                                             int lane, int tpe, Sink sink) {
+  for (int t = lane; t < S.tasks; t += tpe) {
+    const int2 task = S.task[(size_t)c * S.tasks + t];
+    const int node = task.y & 0xffff, len = (task.y >> 16) & 0xfff, g = task.y >> 28;
+    const int n = ns[node];
+    long long acc[NC];
+#pragma unroll
+    for (int e = 0; e < NC; ++e) acc[e] = 0;
+#pragma unroll 2
+    for (int q = task.x; q < task.x + len; ++q) {
+      const int inc = S.inc[q];
+      const FxShift down((inc >> 1 & 127) - n);
+      const long long *dp = diff + (size_t)(inc >> 8) * NC;
+#pragma unroll
+      for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
+    }
+    if (__any_sync(0xffffffffu, g > 0)) {
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1)
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+          const long long other = __shfl_xor_sync(0xffffffffu, acc[e], o);
+          if (g > o >> 1) acc[e] += other;
+        }
+    }
+    // tasks without a node of their own have g < 0
+    if (g >= 0 && (t & ((1 << g) - 1)) == 0) sink(node, acc);
+  }
+}
 
 // Exponents of an element's units from the extremes of its node values (upper
 // words of the largest density, enthalpy and |velocity component| and
@@ -952,7 +991,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
   // volume flux differencing: pass 1 one flux per pair, pass 2 each node's sum
   // over its pairs (as fd_fluxes, in integers)
   const int CH = ka.fx_chunk;
-  for (int c = 0; c < fx.vp_chunks; ++c) {
+  for (int c = 0; c < fx.vol.chunks; ++c) {
     const int c0 = c * CH, c1 = min(op.nvp, c0 + CH);
     for (int p = c0 + lane; p < c1; p += tpe) {
       const int ij = fx.vp_ij[p];
@@ -982,38 +1021,25 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
       for (int e = 0; e < NC; ++e) dp[e] = out[e];
     }
     __syncthreads();
-    for (int i = lane; i < nq; i += tpe) {
-      const int n = ns[i], qe = fx.vp_ptr[(c + 1) * nq + i];
-      long long acc[NC];
+    // r_q[i] += -diff if i is the pair's first node, +diff otherwise
+    fx_node_sums<NC>(fx.vol, c, diff - (size_t)c0 * NC, ns, lane, tpe, [&](int i, const long long *acc) {
 #pragma unroll
-      for (int e = 0; e < NC; ++e) acc[e] = c == 0 ? 0 : rqi[e * nq + i];
-      // r_q[i] += -diff if i is the pair's first node, +diff otherwise
-#pragma unroll 4
-      for (int q = fx.vp_ptr[c * nq + i]; q < qe; ++q) {
-        const int inc = fx.vp_inc[q];
-        const FxShift down((inc >> 1 & 127) - n);
-        const long long *dp = diff + (size_t)((inc >> 8) - c0) * NC;
-#pragma unroll
-        for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
-      }
-#pragma unroll
-      for (int e = 0; e < NC; ++e) rqi[e * nq + i] = acc[e];
-    }
+      for (int e = 0; e < NC; ++e) rqi[e * nq + i] = c == 0 ? acc[e] : rqi[e * nq + i] + acc[e];
+    });
     __syncthreads();
   }
 
-  const FxUnit um(sc.eR + eG + sc.eV - 63), up(eP + eG - 61), ue(eP + eG + sc.eV - 61);
   // a sum of node t (its unit 2^-n_t smaller) in FP64
   auto value = [&](int t, int e, long long v) {
-    const double x = e == 0 ? um(v) : (e == D + 1 ? ue(v) : up(v));
-    return v == 0 ? 0.0 : sse_from_bits(sse_bits(x) - ((long long)ns[t] << 52));
+    const int unit = e == 0 ? sc.eR + eG + sc.eV - 63 : eP + eG - 61 + (e == D + 1 ? sc.eV : 0);
+    return fx_to_double(v, unit - ns[t]);
   };
   // facet correction and interface flux, chunked the same way; the sums are
   // subtracted from r_q (integers) and f_f (converted, FP64)
   const float rnpf = qrcp(npf > 0 ? npf : 1);
   // the pairs nfp .. nfp + nf - 1 are the facet nodes with their facing nodes
   const int nall = op.nfp + nf;
-  for (int c = 0; c < fx.fp_chunks; ++c) {
+  for (int c = 0; c < fx.fac.chunks; ++c) {
     const int c0 = c * CH, c1 = min(nall, c0 + CH);
     for (int p = c0 + lane; p < c1; p += tpe) {
       Fx G[D];
@@ -1041,33 +1067,18 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
       for (int e = 0; e < NC; ++e) dp[e] = out[e];
     }
     __syncthreads();
-    for (int t = lane; t < nq + nf; t += tpe) {
-      const int n = ns[t], qe = fx.fp_ptr[(c + 1) * (nq + nf) + t];
-      long long acc[NC];
-#pragma unroll
-      for (int e = 0; e < NC; ++e) acc[e] = 0;
-#pragma unroll 4
-      for (int q = fx.fp_ptr[c * (nq + nf) + t]; q < qe; ++q) {
-        const int inc = fx.fp_inc[q];
-        const FxShift down((inc >> 1 & 127) - n);
-        const long long *dp = diff + (size_t)((inc >> 8) - c0) * NC;
-#pragma unroll
-        for (int e = 0; e < NC; ++e) acc[e] -= down(dp[e]);
-      }
+    fx_node_sums<NC>(fx.fac, c, diff - (size_t)c0 * NC, ns, lane, tpe, [&](int t, const long long *acc) {
       if (t < nq) {
 #pragma unroll
-        for (int e = 0; e < NC; ++e) rqi[e * nq + t] += acc[e];
+        for (int e = 0; e < NC; ++e) rqi[e * nq + t] -= acc[e];
       } else {
         const int r = t - nq, p = op.nfp + r;
-        if (p >= c0 && p < c1) {
-          const long long *dp = diff + (size_t)(p - c0) * NC;
+        const bool own = p >= c0 && p < c1;
+        const long long *dp = diff + (size_t)(own ? p - c0 : 0) * NC;
 #pragma unroll
-          for (int e = 0; e < NC; ++e) acc[e] += dp[e];
-        }
-#pragma unroll
-        for (int e = 0; e < NC; ++e) ff[e * nf + r] += value(t, e, acc[e]);
+        for (int e = 0; e < NC; ++e) ff[e * nf + r] += value(t, e, (own ? dp[e] : 0) - acc[e]);
       }
-    }
+    });
     __syncthreads();
   }
   for (int i = lane; i < nq; i += tpe)
@@ -1121,9 +1132,9 @@ __global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLa
     double s = 0.0;
     *kmin = kFxMaxK;
     if (t < nq) {
-      for (int q = fx.vp_ptr[t]; q < fx.vp_ptr[fx.vp_chunks * nq + t]; ++q) {
-        s += volume_norm(fx.vp_inc[q]);
-        *kmin = min(*kmin, fx.vp_inc[q] >> 1 & 127);
+      for (int q = fx.vol.first[t]; q < fx.vol.first[t + 1]; ++q) {
+        s += volume_norm(fx.vol.inc[q]);
+        *kmin = min(*kmin, fx.vol.inc[q] >> 1 & 127);
       }
     } else {
       double b = 0.0;
@@ -1131,9 +1142,9 @@ __global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLa
       larger(b);
       s += b;
     }
-    for (int q = fx.fp_ptr[t]; q < fx.fp_ptr[fx.fp_chunks * (nq + nf) + t]; ++q) {
-      s += facet_norm(fx.fp_inc[q]);
-      *kmin = min(*kmin, fx.fp_inc[q] >> 1 & 127);
+    for (int q = fx.fac.first[t]; q < fx.fac.first[t + 1]; ++q) {
+      s += facet_norm(fx.fac.inc[q]);
+      *kmin = min(*kmin, fx.fac.inc[q] >> 1 & 127);
     }
     return s;
   };

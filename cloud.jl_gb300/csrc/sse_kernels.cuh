@@ -35,16 +35,19 @@ struct FxTables {
   int on;             // 0: no fixed-point tables, phase B runs in FP64
   const int *vp_ij;   // i | j << 16
   const Fx *vp_S;     // nvp x d: S / 2 in units 2^(eS - k)
-  // incident pairs per volume node: pair << 8 | k << 1 | (node is i), ascending;
-  // those in chunk c (ka.fx_chunk pairs) of node i: vp_ptr[c nq + i] to
-  // vp_ptr[(c + 1) nq + i]
-  int vp_chunks;
-  const int *vp_ptr, *vp_inc;
-  // facet-correction pairs followed by the nf interface pairs; incident
-  // facet-correction pairs of the volume, then the facet nodes
-  int fp_chunks;
   const Fx *fp_C;     // C / 2 in units 2^(eC - k)
-  const int *fp_ptr, *fp_inc;
+  // Node sums of the volume pairs, and of the facet-correction pairs (followed
+  // by the nf interface pairs) at the volume, then the facet nodes.  inc: the
+  // incident pairs (pair << 8 | k << 1 | (volume pairs: node is i)) of each
+  // node, ascending.  A chunk of ka.fx_chunk pairs has `tasks` tasks, a
+  // multiple of the team's width; task t of chunk c sums inc[x] to inc[x + n] of
+  // node y, task[c tasks + t] = (x, y | n << 16 | g << 28), and 2^g adjacent tasks
+  // (g <= 2) share a node.  first[t], first[t + 1]: the node's whole list.
+  struct Sums {
+    int chunks, tasks;
+    const int *inc, *first;
+    const int2 *task;
+  } vol, fac;
   int eS, eC;
   const int *eG;      // per element: metric vectors in units 2^eG (kFxNone: none)
   const Fx *Lam;      // Lambda_q in units 2^(eG - eS), the layout of Lambda_q
