@@ -291,6 +291,13 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
   if ((e = upload(s, ij.data(), ij.size(), &fx.vp_ij)) || (e = upload(s, S.data(), S.size(), &fx.vp_S)) ||
       (!C.empty() && (e = upload(s, Cx.data(), Cx.size(), &fx.fp_C))))
     return cuda_fail(s, e, "fixed-point pair tables");
+  // P1 nodes a direction, P1^(d-1) a face, one face more than directions
+  for (int P1 = 3; P1 <= 6; ++P1) {
+    const int face = d == 2 ? P1 : P1 * P1;
+    if (nq == face * P1 && s->cfg.nodes_per_face == face && s->cfg.num_faces == d + 1 && s->cfg.n_f == (d + 1) * face &&
+        (!ka.op.has_vdm || ka.op.dense_v || (ka.op.p1 == P1 && ka.op.M1 == P1 && ka.op.M2 == P1 && (d == 2 || ka.op.M3 == P1))))
+      fx.p1_b = P1;
+  }
   ka.fx = fx;
   return SSE_OK;
 }
@@ -410,15 +417,24 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
   if (!scale(ops->vdm_A, op.M1, p1, &A, &kA, &eA) || !scale(ops->vdm_B, op.M2, (size_t)p1 * p1, &B, &kB, &eB) ||
       (c.d == 3 && !scale(ops->vdm_C, M3, (size_t)p1 * p1 * p1, &C, &kC, &eC)))
     return SSE_OK;
-  std::vector<signed char> T(c.n_p), K(c.n_q), eR(c.n_f, 0);
-  for (size_t t = 0; t < (size_t)p1 * p1 * (c.d == 3 ? p1 : 1); ++t) {
-    const int64_t l = ops->vdm_sigma_in[t];
-    if (l == 0) continue;
-    const int b1 = (int)(t % p1), b2 = (int)((t / p1) % p1);
-    const int e = eA[b1] + eB[b1 + p1 * b2] + (c.d == 3 ? eC[t] : 0);
-    if (std::abs(e) > 25) return SSE_OK;
-    T[l - 1] = (signed char)e;
+  std::vector<signed char> T, K(c.n_q), eR(c.n_f, 0);
+  std::vector<int> order, modes, base;
+  for (int b1 = 0; b1 < p1; ++b1) {
+    if (c.d == 2) base.push_back((int)order.size());
+    for (int b2 = 0; b1 + b2 < p1; ++b2) {
+      if (c.d == 3) base.push_back((int)order.size());
+      for (int b3 = 0; b3 < (c.d == 3 ? p1 - b1 - b2 : 1); ++b3) {
+        const size_t t = b1 + (size_t)p1 * (b2 + (size_t)p1 * b3);
+        const int64_t l = ops->vdm_sigma_in[t];
+        const int e = eA[b1] + eB[b1 + p1 * b2] + (c.d == 3 ? eC[t] : 0);
+        if (l == 0 || std::abs(e) > 25) return SSE_OK;
+        order.push_back((int)(l - 1));
+        modes.push_back(b1 | b2 << 8 | b3 << 16);
+        T.push_back((signed char)e);
+      }
+    }
   }
+  if ((int)order.size() != c.n_p) return SSE_OK;
   for (int i = 0; i < c.n_q; ++i)
     K[i] = (signed char)(kA[i / (op.M2 * M3)] + kB[(i / M3) % op.M2] + kC[i % M3]);
   const CsrHost r = csc_to_csr(ops->R, false);
@@ -435,8 +451,10 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
   if ((e = upload(s, A.data(), A.size(), &fx.A)) || (e = upload(s, B.data(), B.size(), &fx.B)) ||
       (c.d == 3 && (e = upload(s, C.data(), C.size(), &fx.C))) || (e = upload(s, R.data(), R.size(), &fx.R)) ||
       (e = upload(s, eR.data(), eR.size(), &fx.eR)) || (e = upload(s, K.data(), K.size(), &fx.K)) ||
-      (e = upload(s, T.data(), T.size(), &fx.T)))
+      (e = upload(s, order.data(), order.size(), &fx.order)) || (e = upload(s, modes.data(), modes.size(), &fx.modes)) ||
+      (e = upload(s, base.data(), base.size(), &fx.base)) || (e = upload(s, T.data(), T.size(), &fx.T)))
     return cuda_fail(s, e, "fixed-point operators");
+  if (fx.p1_b == p1 && op.M1 == p1 && op.M2 == p1 && M3 == (c.d == 3 ? p1 : 1)) fx.p1_a = p1;
   return SSE_OK;
 }
 

@@ -78,117 +78,136 @@ struct FxSums {
   }
 };
 
-// y (NC x nq, times 2^K_i) = V x (NC x np, times 2^T_l)
-template <int D, int NC>
+// Sizes of an element with P1 nodes a direction (and, with a modal tensor-
+// product V, P1 modes): constants of the compiled kernel, so that loops unroll
+// and addresses are offsets; P1 = 0 takes them from the operators.
+template <int D, int P1>
+struct FxSize {
+  static __device__ __forceinline__ int nq(const DevOps &op) { return P1 ? (D == 2 ? P1 * P1 : P1 * P1 * P1) : op.nq; }
+  static __device__ __forceinline__ int npf(const DevOps &op) { return P1 ? (D == 2 ? P1 : P1 * P1) : op.npf; }
+  static __device__ __forceinline__ int nfac(const DevOps &op) { return P1 ? D + 1 : op.nfac; }
+  static __device__ __forceinline__ int nf(const DevOps &op) { return P1 ? nfac(op) * npf(op) : op.nf; }
+  static __device__ __forceinline__ int p1(const DevOps &op) { return P1 ? P1 : op.p1; }
+  static __device__ __forceinline__ int M1(const DevOps &op) { return P1 ? P1 : op.M1; }
+  static __device__ __forceinline__ int M2(const DevOps &op) { return P1 ? P1 : op.M2; }
+  static __device__ __forceinline__ int M3(const DevOps &op) { return P1 ? P1 : op.M3; }
+  static __device__ __forceinline__ int nb12(const DevOps &op) { return P1 ? P1 * (P1 + 1) / 2 : op.nb12; }
+  // s / n for 0 <= s < 2^21
+  static __device__ __forceinline__ int div(int s, int n) { return P1 ? s / n : qdiv(s, qrcp(n)); }
+  static __device__ __forceinline__ int np(const DevOps &op) {
+    return P1 ? (D == 2 ? P1 * (P1 + 1) / 2 : P1 * (P1 + 1) * (P1 + 2) / 6) : op.np;
+  }
+};
+
+// sum over k < n of entry(k) times the vectors at v + k step: P1 steps unrolled
+// where it is given (n <= P1), so that their loads are in flight together
+template <int NC, int P1, typename Entry>
+__device__ __forceinline__ FxSums<NC> fx_line(int n, Entry entry, const Fx *v, int step, int stride) {
+  FxSums<NC> acc;
+  if constexpr (P1 > 0) {
+#pragma unroll
+    for (int k = 0; k < P1; ++k)
+      if (k < n) acc.add(entry(k), v + k * step, stride);
+  } else {
+    for (int k = 0; k < n; ++k) acc.add(entry(k), v + k * step, stride);
+  }
+  return acc;
+}
+
+// y (NC x nq, times 2^K_i) = V x (NC x np, times 2^T_l).  Modal vectors are in
+// the order of the sum factorisation (FxTables::order), the modes of one (b1)
+// or (b1, b2) contiguous from FxTables::base.
+template <int D, int NC, int P1>
 __device__ void fx_vdm_mul(const DevOps &op, const FxTables &fx, const Fx *x, Fx *y, Fx *Z, Fx *W, int lane, int tpe) {
-  const int np = op.np, nq = op.nq, p1 = op.p1, M1 = op.M1, M2 = op.M2;
-  const float rM2 = qrcp(M2), rM3 = qrcp(op.M3 > 0 ? op.M3 : 1);
+  using N = FxSize<D, P1>;
+  const int np = N::np(op), nq = N::nq(op), p1 = N::p1(op), M1 = N::M1(op), M2 = N::M2(op);
   if constexpr (D == 2) {
     for (int s = lane; s < p1 * M2; s += tpe) {
-      const int b1 = qdiv(s, rM2), a2 = s - b1 * M2;
-      FxSums<NC> acc;
-      for (int b2 = 0; b2 < p1 - b1; ++b2) acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], x + modes_index2(op, b1, b2), np);
-      acc.template store<kFoUp>(Z + b1 * M2 + a2, p1 * M2);
+      const int b1 = N::div(s, M2), a2 = s - b1 * M2;
+      fx_line<NC, P1>(p1 - b1, [&](int k) { return fx.B[a2 + M2 * (b1 + p1 * k)]; }, x + fx.base[b1], 1, np)
+          .template store<kFoUp>(Z + s, p1 * M2);
     }
     __syncthreads();
     for (int s = lane; s < M1 * M2; s += tpe) {
-      const int a1 = qdiv(s, rM2), a2 = s - a1 * M2;
-      FxSums<NC> acc;
-      for (int b1 = 0; b1 < p1; ++b1) acc.add(fx.A[a1 + M1 * b1], Z + b1 * M2 + a2, p1 * M2);
-      acc.template store<kFoUp>(y + M2 * a1 + a2, nq);
+      const int a1 = N::div(s, M2), a2 = s - a1 * M2;
+      fx_line<NC, P1>(p1, [&](int k) { return fx.A[a1 + M1 * k]; }, Z + a2, M2, p1 * M2).template store<kFoUp>(y + s, nq);
     }
     __syncthreads();
   } else {
-    const int M3 = op.M3, nb12 = op.nb12;
+    const int M3 = N::M3(op), nb12 = N::nb12(op);
     for (int s = lane; s < nb12 * M3; s += tpe) {
-      const int q = qdiv(s, rM3), a3 = s - q * M3;
+      const int q = N::div(s, M3), a3 = s - q * M3;
       const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
-      FxSums<NC> acc;
-      for (int b3 = 0; b3 < p1 - b1 - b2; ++b3)
-        acc.add(fx.C[a3 + M3 * (b1 + p1 * (b2 + p1 * b3))], x + modes_index3(op, b1, b2, b3), np);
-      acc.template store<kFoUp>(Z + q * M3 + a3, nb12 * M3);
+      fx_line<NC, P1>(p1 - b1 - b2, [&](int k) { return fx.C[a3 + M3 * (b1 + p1 * (b2 + p1 * k))]; }, x + fx.base[q], 1, np)
+          .template store<kFoUp>(Z + s, nb12 * M3);
     }
     __syncthreads();
     for (int s = lane; s < p1 * M2 * M3; s += tpe) {
-      const int r = qdiv(s, rM3), a3 = s - r * M3, b1 = qdiv(r, rM2), a2 = r - b1 * M2;
-      FxSums<NC> acc;
-      for (int b2 = 0; b2 < p1 - b1; ++b2)
-        acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], Z + op.b12_index[b1 + p1 * b2] * M3 + a3, nb12 * M3);
-      acc.template store<kFoUp>(W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+      const int r = N::div(s, M3), a3 = s - r * M3, b1 = N::div(r, M2), a2 = r - b1 * M2;
+      // the (b1, b2) are listed by b1
+      fx_line<NC, P1>(p1 - b1, [&](int k) { return fx.B[a2 + M2 * (b1 + p1 * k)]; }, Z + op.b12_index[b1] * M3 + a3, M3,
+                      nb12 * M3)
+          .template store<kFoUp>(W + s, p1 * M2 * M3);
     }
     __syncthreads();
     for (int s = lane; s < M1 * M2 * M3; s += tpe) {
-      const int r = qdiv(s, rM3), a3 = s - r * M3, a1 = qdiv(r, rM2), a2 = r - a1 * M2;
-      FxSums<NC> acc;
-      for (int b1 = 0; b1 < p1; ++b1) acc.add(fx.A[a1 + M1 * b1], W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
-      acc.template store<kFoUp>(y + (M2 * a1 + a2) * M3 + a3, nq);
+      const int r = N::div(s, M3), a3 = s - r * M3, a1 = N::div(r, M2), a2 = r - a1 * M2;
+      fx_line<NC, P1>(p1, [&](int k) { return fx.A[a1 + M1 * k]; }, W + a2 * M3 + a3, M2 * M3, p1 * M2 * M3)
+          .template store<kFoUp>(y + s, nq);
     }
     __syncthreads();
   }
 }
 
 // x (NC x np, without the factors 2^T_l) = V^T y (NC x nq, times 2^-K_i)
-template <int D, int NC>
+template <int D, int NC, int P1>
 __device__ void fx_vdm_tmul(const DevOps &op, const FxTables &fx, const Fx *y, Fx *x, Fx *Z, Fx *W, int lane, int tpe) {
-  const int np = op.np, nq = op.nq, p1 = op.p1, M1 = op.M1, M2 = op.M2;
-  const float rM2 = qrcp(M2), rM3 = qrcp(op.M3 > 0 ? op.M3 : 1);
+  using N = FxSize<D, P1>;
+  const int np = N::np(op), nq = N::nq(op), p1 = N::p1(op), M1 = N::M1(op), M2 = N::M2(op);
   if constexpr (D == 2) {
     for (int s = lane; s < p1 * M2; s += tpe) {
-      const int b1 = qdiv(s, rM2), a2 = s - b1 * M2;
-      FxSums<NC> acc;
-      for (int a1 = 0; a1 < M1; ++a1) acc.add(fx.A[a1 + M1 * b1], y + M2 * a1 + a2, nq);
-      acc.template store<kFoUp>(Z + b1 * M2 + a2, p1 * M2);
+      const int b1 = N::div(s, M2), a2 = s - b1 * M2;
+      fx_line<NC, P1>(M1, [&](int k) { return fx.A[k + M1 * b1]; }, y + a2, M2, nq).template store<kFoUp>(Z + s, p1 * M2);
     }
     __syncthreads();
     for (int l = lane; l < np; l += tpe) {
-      const int b1 = op.modes[l] & 0xff, b2 = (op.modes[l] >> 8) & 0xff;
-      FxSums<NC> acc;
-      for (int a2 = 0; a2 < M2; ++a2) acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], Z + b1 * M2 + a2, p1 * M2);
-      acc.template store<kFoUp>(x + l, np);
+      const int m = fx.modes[l], b1 = m & 0xff, b2 = (m >> 8) & 0xff;
+      fx_line<NC, P1>(M2, [&](int k) { return fx.B[k + M2 * (b1 + p1 * b2)]; }, Z + b1 * M2, 1, p1 * M2)
+          .template store<kFoUp>(x + l, np);
     }
     __syncthreads();
   } else {
-    const int M3 = op.M3, nb12 = op.nb12;
+    const int M3 = N::M3(op), nb12 = N::nb12(op);
     for (int s = lane; s < p1 * M2 * M3; s += tpe) {
-      const int r = qdiv(s, rM3), a3 = s - r * M3, b1 = qdiv(r, rM2), a2 = r - b1 * M2;
-      FxSums<NC> acc;
-      for (int a1 = 0; a1 < M1; ++a1) acc.add(fx.A[a1 + M1 * b1], y + (M2 * a1 + a2) * M3 + a3, nq);
-      acc.template store<kFoUp>(W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
+      const int r = N::div(s, M3), a3 = s - r * M3, b1 = N::div(r, M2), a2 = r - b1 * M2;
+      fx_line<NC, P1>(M1, [&](int k) { return fx.A[k + M1 * b1]; }, y + a2 * M3 + a3, M2 * M3, nq)
+          .template store<kFoUp>(W + s, p1 * M2 * M3);
     }
     __syncthreads();
     for (int s = lane; s < nb12 * M3; s += tpe) {
-      const int q = qdiv(s, rM3), a3 = s - q * M3;
+      const int q = N::div(s, M3), a3 = s - q * M3;
       const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
-      FxSums<NC> acc;
-      for (int a2 = 0; a2 < M2; ++a2)
-        acc.add(fx.B[a2 + M2 * (b1 + p1 * b2)], W + (b1 * M2 + a2) * M3 + a3, p1 * M2 * M3);
-      acc.template store<kFoUp>(Z + q * M3 + a3, nb12 * M3);
+      fx_line<NC, P1>(M2, [&](int k) { return fx.B[k + M2 * (b1 + p1 * b2)]; }, W + b1 * M2 * M3 + a3, M3, p1 * M2 * M3)
+          .template store<kFoUp>(Z + s, nb12 * M3);
     }
     __syncthreads();
     for (int l = lane; l < np; l += tpe) {
-      const int b1 = op.modes[l] & 0xff, b2 = (op.modes[l] >> 8) & 0xff, b3 = (op.modes[l] >> 16) & 0xff;
-      const int q = op.b12_index[b1 + p1 * b2];
-      FxSums<NC> acc;
-      for (int a3 = 0; a3 < M3; ++a3) acc.add(fx.C[a3 + M3 * (b1 + p1 * (b2 + p1 * b3))], Z + q * M3 + a3, nb12 * M3);
-      acc.template store<kFoUp>(x + l, np);
+      const int m = fx.modes[l], b1 = m & 0xff, b2 = (m >> 8) & 0xff, b3 = (m >> 16) & 0xff;
+      fx_line<NC, P1>(M3, [&](int k) { return fx.C[k + M3 * (b1 + p1 * (b2 + p1 * b3))]; }, Z + op.b12_index[b1 + p1 * b2] * M3,
+                      1, nb12 * M3)
+          .template store<kFoUp>(x + l, np);
     }
     __syncthreads();
   }
 }
 
-// y (NC x np) = A x (NC x np) for the element's mass operator A (column-major,
+// entry (e, a) of A x (NC x np) for the element's mass operator A (column-major,
 // the absolute sums of its rows at most 1)
-template <int NC>
-__device__ void fx_mass(const Fx *A, const Fx *x, Fx *y, int np, int lane, int tpe) {
-  for (int t = lane; t < NC * np; t += tpe) {
-    const int e = t / np, a = t - e * np;
-    FxSums<1> acc;
-    const Fx *xe = x + e * np;
-#pragma unroll 4
-    for (int b = 0; b < np; ++b) acc.add(A[b * np + a], xe + b, 0);
-    acc.template store<0>(y + t, 0);
-  }
-  __syncthreads();
+__device__ __forceinline__ long long fx_mass_row(const Fx *A, const Fx *xe, int np, int a) {
+  FxSums<1> acc;
+#pragma unroll 5
+  for (int b = 0; b < np; ++b) acc.add(A[b * np + a], xe + b, 0);
+  return acc.template value<0>(0);
 }
 
 // Unit exponents of the NC vectors of modal values: unit[e] with
@@ -196,9 +215,10 @@ __device__ void fx_mass(const Fx *A, const Fx *x, Fx *y, int np, int lane, int t
 // components.  kFxBad: not finite (or beyond 2^900).
 constexpr int kFxBad = 100000;
 
-// x in FP64
+// x in FP64; place l is taken from order[l] (null: l), without factors where T is
+// null
 template <int NC>
-__device__ __forceinline__ void fx_modal_units(const double *x, const signed char *T, int np, int *unit, int lane,
+__device__ __forceinline__ void fx_modal_units(const double *x, const signed char *T, const int *order, int np, int *unit, int lane,
                                                int tpe) {
   const int width = tpe < 32 ? tpe : 32, groups = tpe / width, g = lane / width, w = lane - g * width;
   for (int e0 = 0; e0 < NC; e0 += groups) {
@@ -206,15 +226,15 @@ __device__ __forceinline__ void fx_modal_units(const double *x, const signed cha
     int m = -2000;
     if (e < NC)
       for (int l = w; l < np; l += width) {
-        const int ex = (__double2hiint(x[e * np + l]) >> 20) & 0x7ff;
-        if (ex > 0) m = max(m, ex == 0x7ff ? kFxBad : ex - 1023 + T[l]);
+        const int ex = (__double2hiint(x[e * np + (order ? order[l] : l)]) >> 20) & 0x7ff;
+        if (ex > 0) m = max(m, ex == 0x7ff ? kFxBad : ex - 1023 + (T ? T[l] : 0));
       }
     for (int o = width >> 1; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     float s = 0.f;
     if (e < NC)
       for (int l = w; l < np; l += width) {
-        const double v = x[e * np + l];
-        const int ex = (__double2hiint(v) >> 20) & 0x7ff, d = m - (ex - 1023 + T[l]);
+        const double v = x[e * np + (order ? order[l] : l)];
+        const int ex = (__double2hiint(v) >> 20) & 0x7ff, d = m - (ex - 1023 + (T ? T[l] : 0));
         // the mantissa, rounded up, times 2^-d
         const float f = __int_as_float(0x3f800000 + ((__double2hiint(v) & 0xfffff) << 3) + 8);
         if (ex > 0 && d < 100) s += f * __int_as_float((127 - d) << 23);

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
 // residual's error against extended precision falls to 0.4 to 0.8 of that
 // with the FP64 operators (40 modal configurations, p = 2 to 6).
 // ---------------------------------------------------------------------------
-template <int D, int NC>
+template <int D, int NC, int P1>
 __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_constant__ KernelArgs ka) {
   static_assert(NC == D + 2, "Euler");
   extern __shared__ double smem[];
@@ -141,7 +141,8 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
   const int k = blockIdx.x * ka.epb + team;
   const bool live = k < ka.ne;
   const int kk = live ? k : 0;
-  const int np = op.np, nq = op.nq, nf = op.nf;
+  using N = FxSize<D, P1>;
+  const int np = N::np(op), nq = N::nq(op), nf = N::nf(op);
   double *base = smem + (size_t)team * L.team_doubles;
   Fx *X = reinterpret_cast<Fx *>(base + L.off[0]), *Y = reinterpret_cast<Fx *>(base + L.off[1]),
      *Z = reinterpret_cast<Fx *>(base + L.off[2]), *W = reinterpret_cast<Fx *>(base + L.off[3]);
@@ -154,14 +155,14 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
   for (int t = lane; t < NC * np; t += tpe) Yd[t] = uk[t];
   if (lane < NC) key[lane] = 0u;
   __syncthreads();
-  fx_modal_units<NC>(Yd, fx.T, np, unit, lane, tpe);
+  fx_modal_units<NC>(Yd, fx.T, fx.order, np, unit, lane, tpe);
   __syncthreads();
   for (int t = lane; t < NC * np; t += tpe) {
-    const int e = t / np;
-    X[t] = fo_from_double(Yd[t], unit[e] - fx.T[t - e * np]);
+    const int e = N::div(t, np), l = t - e * np;
+    X[t] = fo_from_double(Yd[e * np + fx.order[l]], unit[e] - fx.T[l]);
   }
   __syncthreads();
-  fx_vdm_mul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  fx_vdm_mul<D, NC, P1>(op, fx, X, Y, Z, W, lane, tpe);
   // w_q = WJ c2e(u_q)
   const double *WJ = ka.geo.WJ + (size_t)kk * nq;
   unsigned kmax[NC];
@@ -196,25 +197,29 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
   __syncthreads();
   // V^T, then the mass solve in the unit of its own input, then V in the unit
   // of its own; the last unit[e] is that of w_q
-  fx_vdm_tmul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  fx_vdm_tmul<D, NC, P1>(op, fx, X, Y, Z, W, lane, tpe);
   fx_modal_units<NC>(Y, fx.T, np, unit2, lane, tpe);
   __syncthreads();
   for (int t = lane; t < NC * np; t += tpe) {
-    const int e = t / np;
+    const int e = N::div(t, np);
     Y[t] = fx_scale(Y[t], fx.T[t - e * np] - unit2[e]);
   }
   __syncthreads();
   if (lane < NC && unit[lane] != kFxBad) unit[lane] += unit2[lane] + fx.eA[kk];
-  fx_mass<NC>(fx.A_k + (size_t)kk * np * np, Y, X, np, lane, tpe);
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = N::div(t, np);
+    X[t] = fo_split(fx_mass_row(fx.A_k + (size_t)kk * np * np, Y + e * np, np, t - e * np));
+  }
+  __syncthreads();
   fx_modal_units<NC>(X, fx.T, np, unit2, lane, tpe);
   __syncthreads();
   for (int t = lane; t < NC * np; t += tpe) {
-    const int e = t / np;
+    const int e = N::div(t, np);
     X[t] = fx_scale(X[t], fx.T[t - e * np] - unit2[e]);
   }
   if (lane < NC && unit[lane] != kFxBad) unit[lane] += unit2[lane];
   __syncthreads();
-  fx_vdm_mul<D, NC>(op, fx, X, Y, Z, W, lane, tpe);
+  fx_vdm_mul<D, NC, P1>(op, fx, X, Y, Z, W, lane, tpe);
   // u_q = e2c(w_q), u_f = e2c(R w_q)
   for (int t = lane; t < nq + nf; t += tpe) {
     const bool vol = t < nq;
@@ -242,8 +247,9 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
 // Fixed-point mass operators of phase A: A_k scaled by 2^-eA so that the
 // absolute sums of its rows are at most 1, and eW with sum_i W J 2^-K_i < 2^eW
 __global__ void __launch_bounds__(128) fx_mass_operator_kernel(const double *__restrict__ Ak, const double *__restrict__ WJ,
-                                                               const signed char *__restrict__ K, int np, int nq,
-                                                               Fx *oA, int *oeA, int *oeW) {
+                                                               const signed char *__restrict__ K,
+                                                               const int *__restrict__ order, int np, int nq, Fx *oA,
+                                                               int *oeA, int *oeW) {
   __shared__ unsigned row;
   __shared__ double part[128];
   const size_t k = blockIdx.x;
@@ -266,7 +272,10 @@ __global__ void __launch_bounds__(128) fx_mass_operator_kernel(const double *__r
     oeA[k] = e;
     oeW[k] = min(400, max(-400, fx_exponent((unsigned)__double2hiint(s * (1.0 + 1e-6)))));
   }
-  for (int t = threadIdx.x; t < np * np; t += blockDim.x) oA[k * np * np + t] = fo_from_double(A[t], e);
+  for (int t = threadIdx.x; t < np * np; t += blockDim.x) {
+    const int b = t / np;
+    oA[k * np * np + t] = fo_from_double(A[order[b] * np + order[t - b * np]], e);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -836,6 +845,77 @@ struct FxScale {
   }
 };
 
+// fd_tail for a modal tensor-product V: R^T and V^T in FP64, one (node or mode,
+// variable) a thread where a thread for all variables would leave the FP64
+// units of most of the SM's quarters idle, and the mass solve in fixed point
+// (its FP64 form held two quarters for 70 dependent instructions)
+template <int D, int NC, int P1>
+__device__ __forceinline__ void fx_tail(const KernelArgs &ka, double *rq, const double *ff, double *scratch, int *unit,
+                                        int kk, bool live, int lane, int tpe) {
+  using N = FxSize<D, P1>;
+  const DevOps &op = ka.op;
+  const FxTables &fx = ka.fx;
+  const int np = N::np(op), nq = N::nq(op), p1 = N::p1(op), M1 = N::M1(op), M2 = N::M2(op);
+  rt_apply<double, NC>(op, op.Rt_val, ff, lane, tpe, [&](int t, double v) { rq[t] -= v; });
+  __syncthreads();
+  double *X = scratch, *Z = X + (size_t)NC * np, *W = Z + (size_t)NC * (D == 2 ? p1 * M2 : N::nb12(op) * N::M3(op));
+  Fx *Xf = reinterpret_cast<Fx *>(rq);  // after V^T
+  auto line = [](int n, auto entry, const double *v, int step) {
+    double acc = 0.0;
+    if constexpr (P1 > 0) {
+#pragma unroll
+      for (int k = 0; k < P1; ++k) acc = fma(entry(k), v[k * step], acc);
+    } else {
+      for (int k = 0; k < n; ++k) acc = fma(entry(k), v[k * step], acc);
+    }
+    return acc;
+  };
+  if constexpr (D == 2) {
+    for (int t = lane; t < NC * p1 * M2; t += tpe) {
+      const int e = N::div(t, p1 * M2), s = t - e * p1 * M2, b1 = N::div(s, M2), a2 = s - b1 * M2;
+      Z[t] = line(M1, [&](int k) { return op.A[k + M1 * b1]; }, rq + e * nq + a2, M2);
+    }
+    __syncthreads();
+    for (int t = lane; t < NC * np; t += tpe) {
+      const int e = N::div(t, np), m = fx.modes[t - e * np], b1 = m & 0xff, b2 = (m >> 8) & 0xff;
+      X[t] = line(M2, [&](int k) { return op.B[k + M2 * (b1 + p1 * b2)]; }, Z + (e * p1 + b1) * M2, 1);
+    }
+  } else {
+    const int M3 = N::M3(op), nb12 = N::nb12(op);
+    for (int t = lane; t < NC * p1 * M2 * M3; t += tpe) {
+      const int e = N::div(t, p1 * M2 * M3), s = t - e * p1 * M2 * M3, b1 = N::div(s, M2 * M3), a = s - b1 * M2 * M3;
+      W[t] = line(M1, [&](int k) { return op.A[k + M1 * b1]; }, rq + e * nq + a, M2 * M3);
+    }
+    __syncthreads();
+    for (int t = lane; t < NC * nb12 * M3; t += tpe) {
+      const int e = N::div(t, nb12 * M3), s = t - e * nb12 * M3, q = N::div(s, M3), a3 = s - q * M3;
+      const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
+      Z[t] = line(M2, [&](int k) { return op.B[k + M2 * (b1 + p1 * b2)]; }, W + (e * p1 + b1) * M2 * M3 + a3, M3);
+    }
+    __syncthreads();
+    for (int t = lane; t < NC * np; t += tpe) {
+      const int e = N::div(t, np), m = fx.modes[t - e * np], b1 = m & 0xff, b2 = (m >> 8) & 0xff, b3 = (m >> 16) & 0xff;
+      X[t] = line(M3, [&](int k) { return op.C[k + M3 * (b1 + p1 * (b2 + p1 * b3))]; },
+                  Z + (e * nb12 + op.b12_index[b1 + p1 * b2]) * M3, 1);
+    }
+  }
+  __syncthreads();
+  fx_modal_units<NC>(X, nullptr, nullptr, np, unit, lane, tpe);
+  __syncthreads();
+  for (int t = lane; t < NC * np; t += tpe) Xf[t] = fo_from_double(X[t], unit[N::div(t, np)]);
+  __syncthreads();
+  double *out = ka.dudt + (size_t)kk * NC * np;
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = N::div(t, np), a = t - e * np;
+    const long long v = fx_mass_row(fx.A_k + (size_t)kk * np * np, Xf + e * np, np, a);
+    const double x = fx_value(v, unit[e] == kFxBad ? kFxBad : unit[e] + fx.eA[kk]);
+    if (live) {
+      out[e * np + fx.order[a]] = x;
+      if (!isfinite(x)) ka.flag_nonphysical();
+    }
+  }
+}
+
 // the FP64 passes for a block that leaves the fixed-point ones: out of line, so
 // that their registers are not the kernel's
 template <int D, int NC>
@@ -845,7 +925,7 @@ __device__ __noinline__ void fd_fp64(const KernelArgs &ka, double *base, int kk,
   fd_tail<D, NC>(ka, base + L.off[3], base + L.off[2], base + L.off[4], kk, live, lane, tpe);
 }
 
-template <int D, int NC>
+template <int D, int NC, int P1>
 __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __grid_constant__ KernelArgs ka) {
   static_assert(NC == D + 2, "Euler");
   extern __shared__ double smem[];
@@ -858,7 +938,8 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
   const int k = blockIdx.x * ka.epb + team;
   const bool live = k < ka.ne;
   const int kk = live ? k : 0;
-  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf;
+  using N = FxSize<D, P1>;
+  const int nq = N::nq(op), nf = N::nf(op), nfac = N::nfac(op), npf = N::npf(op);
   constexpr int PS = kFxStride<D>;
   double *base = smem + (size_t)team * L.team_doubles;
   double *ff = base + L.off[0], *rq = base + L.off[1];
@@ -908,8 +989,9 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
       for (int e = 0; e < NC; ++e) u[e] = uqg[e * nq + i];
       store_node(i, u, sse_rcp(u[0]));
     }
+    // (from the other end of the team: the volume nodes leave its last warps idle)
     const double *ufg = ka.u_f + (size_t)kk * NC * nf;
-    for (int j = lane; j < nf; j += tpe) {
+    for (int j = tpe - 1 - lane; j < nf; j += tpe) {
       const int P = ka.geo.mapP[(size_t)kk * nf + j];
       const int jn = P % nf, kn = P / nf;
       double ui[NC], uo[NC];
@@ -982,7 +1064,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
     for (int m = 0; m < kFxNode<D>; ++m) node[(size_t)i * PS + m] = v[m];
   };
   for (int i = lane; i < nq; i += tpe) convert(i);
-  for (int j = lane; j < nf; j += tpe) {
+  for (int j = tpe - 1 - lane; j < nf; j += tpe) {
     convert(nq + j);
     convert(nq + nf + j);
   }
@@ -1085,7 +1167,8 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
 #pragma unroll
     for (int e = 0; e < NC; ++e) rq[e * nq + i] = value(i, e, rqi[e * nq + i]);
   __syncthreads();
-  fd_tail<D, NC>(ka, rq, ff, base + L.off[2], kk, live, lane, tpe);
+  if (fx.on_a) fx_tail<D, NC, P1>(ka, rq, ff, base + L.off[2], reinterpret_cast<int *>(key), kk, live, lane, tpe);
+  else fd_tail<D, NC>(ka, rq, ff, base + L.off[2], kk, live, lane, tpe);
 }
 
 // Fixed-point metric terms of one element per block.  2^eG bounds every
@@ -2193,6 +2276,26 @@ __global__ void __launch_bounds__(256) energy_kernel(KernelArgs ka, const double
   else if (ka.op.d == 3 && ka.op.nc == 5) { constexpr int D = 3, NC = 5; CALL; } \
   else return cudaErrorInvalidValue;
 
+// the fixed-point kernels of this configuration: compiled for 3 to 6 nodes a
+// direction, and for any number
+template <int P1>
+static const void *fx_kernel(const KernelArgs &ka, bool a) {
+  if (ka.op.d == 2)
+    return a ? (const void *)nodal_values_fx_kernel<2, 4, P1> : (const void *)fd_time_derivative_fx_kernel<2, 4, P1>;
+  return a ? (const void *)nodal_values_fx_kernel<3, 5, P1> : (const void *)fd_time_derivative_fx_kernel<3, 5, P1>;
+}
+static const void *fx_kernel(const KernelArgs &ka, bool a, int p1) {
+  switch (p1) {
+    case 3: return fx_kernel<3>(ka, a);
+    case 4: return fx_kernel<4>(ka, a);
+    case 5: return fx_kernel<5>(ka, a);
+    case 6: return fx_kernel<6>(ka, a);
+    default: return fx_kernel<0>(ka, a);
+  }
+}
+static const void *fx_kernel_a(const KernelArgs &ka) { return fx_kernel(ka, true, ka.fx.p1_a); }
+static const void *fx_kernel_b(const KernelArgs &ka) { return fx_kernel(ka, false, ka.fx.p1_b); }
+
 cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
   cudaError_t e = cudaSuccess;
   auto set = [&](const void *f, size_t bytes) {
@@ -2204,12 +2307,8 @@ cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
     if (ka.fd) set((const void *)fd_time_derivative_kernel<D, NC>, smB);
     if (!ka.fd) set((const void *)std_time_derivative_kernel<D, NC>, smB);
   });
-  if (ka.fx.T)
-    set(ka.op.d == 2 ? (const void *)nodal_values_fx_kernel<2, 4> : (const void *)nodal_values_fx_kernel<3, 5>,
-        (size_t)ka.epb_ax * ka.layAx.team_doubles * sizeof(double));
-  if (ka.fx.vp_ij)
-    set(ka.op.d == 2 ? (const void *)fd_time_derivative_fx_kernel<2, 4>
-                     : (const void *)fd_time_derivative_fx_kernel<3, 5>, smB);
+  if (ka.fx.T) set(fx_kernel_a(ka), (size_t)ka.epb_ax * ka.layAx.team_doubles * sizeof(double));
+  if (ka.fx.vp_ij) set(fx_kernel_b(ka), smB);
   return e;
 }
 
@@ -2234,9 +2333,8 @@ cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st) {
     kx.epb = ka.epb_ax;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
     const size_t smx = (size_t)kx.epb * ka.layAx.team_doubles * sizeof(double);
-    if (ka.op.d == 2) nodal_values_fx_kernel<2, 4><<<gridx, ka.tpb_ax, smx, st>>>(kx);
-    else nodal_values_fx_kernel<3, 5><<<gridx, ka.tpb_ax, smx, st>>>(kx);
-    return cudaGetLastError();
+    void *args[] = {&kx};
+    return cudaLaunchKernel(fx_kernel_a(ka), dim3(gridx), dim3(ka.tpb_ax), args, smx, st);
   }
   // the FP64 phase A has its own team geometry (epb_a elements per block of
   // the same tpb threads)
@@ -2332,8 +2430,8 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
     kx.epb = ka.epb_bx;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
     sm = (size_t)kx.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
-    if (ka.op.d == 2) fd_time_derivative_fx_kernel<2, 4><<<gridx, ka.tpb_bx, sm, st>>>(kx);
-    else fd_time_derivative_fx_kernel<3, 5><<<gridx, ka.tpb_bx, sm, st>>>(kx);
+    void *args[] = {&kx};
+    return cudaLaunchKernel(fx_kernel_b(ka), dim3(gridx), dim3(ka.tpb_bx), args, sm, st);
   } else if (ka.fd) {
     SSE_DISPATCH(D, NC, (fd_time_derivative_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka)));
   } else {
@@ -2350,7 +2448,7 @@ cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, 
 }
 
 cudaError_t launch_fx_mass_operators(const KernelArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st) {
-  fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.op.np, ka.op.nq, A, eA, eW);
+  fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.fx.order, ka.op.np, ka.op.nq, A, eA, eW);
   return cudaGetLastError();
 }
 

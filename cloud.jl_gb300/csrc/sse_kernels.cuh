@@ -63,6 +63,13 @@ struct FxTables {
   const Fx *A, *B, *C, *R, *A_k;
   const signed char *T, *K, *eR;
   const int *eA, *eW;
+  // modal vectors (T, A_k) are in the order of the sum factorisation: place l
+  // holds mode order[l] = packed b1 | b2 << 8 | b3 << 16 modes[l]; those of one b1
+  // (2-D) or (b1, b2) (3-D) start at base
+  const int *order, *modes, *base;
+  // nodes a direction where the element's sizes are those of FxSize (and, for
+  // phase A, V's too), else 0
+  int p1_a, p1_b;
 };
 constexpr int kFxMaxK = 30;  // largest k_p
 constexpr int kFxNone = -100000;
