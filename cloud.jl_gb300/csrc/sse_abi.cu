@@ -447,8 +447,21 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
     eR[j] = (signed char)(std::ilogb(row) + 1);
     for (int q = r.ptr[j]; q < r.ptr[j + 1]; ++q) R[q] = fo_from_double(std::ldexp(r.val[q], -K[r.idx[q]]), eR[j]);
   }
+  const CsrHost rt = csc_to_csr(ops->R, true);
+  std::vector<Fx> Rt(std::max<size_t>(1, rt.val.size()), Fx{0, 0});
+  double rows = 0.0;
+  for (int i = 0; i < c.n_q; ++i) {
+    double row = 0.0;
+    for (int q = rt.ptr[i]; q < rt.ptr[i + 1]; ++q) row += std::ldexp(std::fabs(rt.val[q]), -K[i]);
+    rows = std::max(rows, row);
+  }
+  fx.eRt = rows > 1e-30 ? std::ilogb(rows) + 1 : 0;
+  fx.eRmin = *std::min_element(eR.begin(), eR.end());
+  if (std::abs(fx.eRt - fx.eRmin) > 25) return SSE_OK;
+  for (int i = 0; i < c.n_q; ++i)
+    for (int q = rt.ptr[i]; q < rt.ptr[i + 1]; ++q) Rt[q] = fo_from_double(std::ldexp(rt.val[q], -K[i]), fx.eRt);
   cudaError_t e;
-  if ((e = upload(s, A.data(), A.size(), &fx.A)) || (e = upload(s, B.data(), B.size(), &fx.B)) ||
+  if ((e = upload(s, A.data(), A.size(), &fx.A)) || (e = upload(s, Rt.data(), Rt.size(), &fx.Rt)) || (e = upload(s, B.data(), B.size(), &fx.B)) ||
       (c.d == 3 && (e = upload(s, C.data(), C.size(), &fx.C))) || (e = upload(s, R.data(), R.size(), &fx.R)) ||
       (e = upload(s, eR.data(), eR.size(), &fx.eR)) || (e = upload(s, K.data(), K.size(), &fx.K)) ||
       (e = upload(s, order.data(), order.size(), &fx.order)) || (e = upload(s, modes.data(), modes.size(), &fx.modes)) ||
@@ -1029,13 +1042,13 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       const int budget = 110 * 1024 / 8 / epb_x;
       const int nodes = nq + 2 * nf, pairs = std::max(op.nvp, op.nfp + nf), stride = d == 2 ? kFxStride<2> : kFxStride<3>;
       auto layout_x = [&](int n) {
-        finish(ka.layBx, {nc * nf, nc * nq, std::max(n * nc, final_scratch), nodes * stride, 2 * nodes, 4,
+        finish(ka.layBx, {nc * nf, nc * nq, std::max(n * nc, std::max(final_scratch, nc * (np + nq + nf))), nodes * stride, 2 * nodes, 6,
                           (nq + nf + 7) / 8});
         return ka.layBx.team_doubles;
       };
       int n = pairs;
       if (layout_x(n) > budget) {
-        const int fixed = layout_x(0) - ((std::max(0, final_scratch) + 1) & ~1);
+        const int fixed = layout_x(0) - ((std::max(final_scratch, nc * (np + nq + nf)) + 1) & ~1);
         const int cap1 = (int)((size_t)220 * 1024 / 8 / epb_x);
         int room = budget - fixed;
         if (room / nc < std::max(std::min(tpe_x, pairs), pairs / 3)) room = cap1 - fixed;

@@ -66,6 +66,14 @@ struct FxSums {
       h[e] = fx_wide(a.hi, b.hi, h[e]);
     }
   }
+  // what the cross products have above 2^-62, moved to the others
+  __device__ __forceinline__ void fold() {
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      h[e] += x[e] >> kFoLow;
+      x[e] &= (1LL << kFoLow) - 1;
+    }
+  }
   // the sum, up by UP bits
   template <int UP>
   __device__ __forceinline__ long long value(int e) const {
@@ -203,11 +211,30 @@ __device__ void fx_vdm_tmul(const DevOps &op, const FxTables &fx, const Fx *y, F
 
 // entry (e, a) of A x (NC x np) for the element's mass operator A (column-major,
 // the absolute sums of its rows at most 1)
+template <int MAXU>
 __device__ __forceinline__ long long fx_mass_row(const Fx *A, const Fx *xe, int np, int a) {
   FxSums<1> acc;
-#pragma unroll 5
+#pragma unroll MAXU
   for (int b = 0; b < np; ++b) acc.add(A[b * np + a], xe + b, 0);
   return acc.template value<0>(0);
+}
+
+// *m = max(*m, v) over the team (m in shared memory)
+__device__ __forceinline__ void fx_team_max(unsigned *m, unsigned v, int lane, int tpe) {
+  if (tpe >= 32) {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((lane & 31) == 0) atomicMax(m, v);
+  } else {
+    for (int o = tpe >> 1; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) atomicMax(m, v);
+  }
+}
+
+// fetch the lines of `bytes` bytes at p into L2
+__device__ __forceinline__ void fx_prefetch(const void *p, size_t bytes, int lane, int tpe) {
+  const char *c = static_cast<const char *>(p);
+  for (size_t o = (size_t)lane * 128; o < bytes; o += (size_t)tpe * 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(c + o));
 }
 
 // Unit exponents of the NC vectors of modal values: unit[e] with

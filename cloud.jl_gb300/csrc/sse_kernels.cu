@@ -181,12 +181,8 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
       Xd[e * nq + i] = wi[e] * s;
     }
   }
-  const int width = tpe < 32 ? tpe : 32;
 #pragma unroll
-  for (int e = 0; e < NC; ++e) {
-    for (int o = width >> 1; o > 0; o >>= 1) kmax[e] = max(kmax[e], __shfl_xor_sync(0xffffffffu, kmax[e], o));
-    if ((lane & (width - 1)) == 0) atomicMax(key + e, kmax[e]);
-  }
+  for (int e = 0; e < NC; ++e) fx_team_max(key + e, kmax[e], lane, tpe);
   __syncthreads();
   // sum_i |WJ_i w_i| 2^-K_i < 2^eW max |w|
   if (lane < NC) unit[lane] = key[lane] >= (1023u + 900u) << 20 ? kFxBad : max(-800, fx_exponent(key[lane])) + fx.eW[kk];
@@ -208,7 +204,7 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
   if (lane < NC && unit[lane] != kFxBad) unit[lane] += unit2[lane] + fx.eA[kk];
   for (int t = lane; t < NC * np; t += tpe) {
     const int e = N::div(t, np);
-    X[t] = fo_split(fx_mass_row(fx.A_k + (size_t)kk * np * np, Y + e * np, np, t - e * np));
+    X[t] = fo_split(fx_mass_row<5>(fx.A_k + (size_t)kk * np * np, Y + e * np, np, t - e * np));
   }
   __syncthreads();
   fx_modal_units<NC>(X, fx.T, np, unit2, lane, tpe);
@@ -229,10 +225,22 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
 #pragma unroll
       for (int e = 0; e < NC; ++e) wi[e] = fx_value(Y[e * nq + r], unit[e], -fx.K[r]);
     } else {
-      FxSums<NC> acc;
-      for (int q = op.R_ptr[r]; q < op.R_ptr[r + 1]; ++q) acc.add(fx.R[q], Y + op.R_idx[q], nq);
+      // two entries at a time: nodal values are up to 1 each, and the low part
+      // of an entry times their high part up to 2^61
+      long long w[NC];
 #pragma unroll
-      for (int e = 0; e < NC; ++e) wi[e] = fx_value(acc.template value<0>(e), unit[e], fx.eR[r]);
+      for (int e = 0; e < NC; ++e) w[e] = 0;
+      const int qe = op.R_ptr[r + 1];
+#pragma unroll 3
+      for (int q = op.R_ptr[r]; q < qe; q += 2) {
+        FxSums<NC> acc;
+        acc.add(fx.R[q], Y + op.R_idx[q], nq);
+        if (q + 1 < qe) acc.add(fx.R[q + 1], Y + op.R_idx[q + 1], nq);
+#pragma unroll
+        for (int e = 0; e < NC; ++e) w[e] += acc.template value<0>(e);
+      }
+#pragma unroll
+      for (int e = 0; e < NC; ++e) wi[e] = fx_value(w[e], unit[e], fx.eR[r]);
     }
     entropy_to_cons_pressure<D>(ph.gamma, ph.igm1, wi, ui, op.math_tab);
     double *dst = (vol ? ka.u_q : ka.u_f) + (size_t)kk * NC * n + r;
@@ -845,70 +853,81 @@ struct FxScale {
   }
 };
 
-// fd_tail for a modal tensor-product V: R^T and V^T in FP64, one (node or mode,
-// variable) a thread where a thread for all variables would leave the FP64
-// units of most of the SM's quarters idle, and the mass solve in fixed point
-// (its FP64 form held two quarters for 70 dependent instructions)
-template <int D, int NC, int P1>
-__device__ __forceinline__ void fx_tail(const KernelArgs &ka, double *rq, const double *ff, double *scratch, int *unit,
-                                        int kk, bool live, int lane, int tpe) {
+// fd_tail for a modal tensor-product V in block fixed point.  rqi: r_q as integer
+// sums in units 2^(u(e) - n_i); f_f in FP64; unit, part: scratch of 2 N_c ints and
+// N_c floats a warp.  With c_j the sum of |R_ji| 2^-K_i, at
+// most 2^eR_j, every partial sum of V^T (r_q - R^T f_f) is bounded by
+//   S_e = sum_i |r_q,i| 2^-K_i + sum_j |f_f,j| 2^eR_j,
+// which is formed for the element at hand.
+template <int D, int NC, int P1, typename Unit>
+__device__ __forceinline__ void fx_tail(const KernelArgs &ka, const long long *rqi, const double *ff, double *scratch,
+                                        int *unit, float *part, const signed char *ns, Unit u, int kk, bool live, int lane, int tpe) {
   using N = FxSize<D, P1>;
   const DevOps &op = ka.op;
   const FxTables &fx = ka.fx;
-  const int np = N::np(op), nq = N::nq(op), p1 = N::p1(op), M1 = N::M1(op), M2 = N::M2(op);
-  rt_apply<double, NC>(op, op.Rt_val, ff, lane, tpe, [&](int t, double v) { rq[t] -= v; });
-  __syncthreads();
-  double *X = scratch, *Z = X + (size_t)NC * np, *W = Z + (size_t)NC * (D == 2 ? p1 * M2 : N::nb12(op) * N::M3(op));
-  Fx *Xf = reinterpret_cast<Fx *>(rq);  // after V^T
-  auto line = [](int n, auto entry, const double *v, int step) {
-    double acc = 0.0;
-    if constexpr (P1 > 0) {
+  const int np = N::np(op), nq = N::nq(op), nf = N::nf(op);
+  Fx *X = reinterpret_cast<Fx *>(scratch), *Y = X + NC * np, *Z = Y + NC * nq,
+     *W = Z + NC * (D == 2 ? N::p1(op) * N::M2(op) : N::nb12(op) * N::M3(op)), *F = Z;
+  // S_e in FP32, relative to 2^u(e): the upper words of the sums rounded up, and
+  // the powers of two above f_f (below 2^90, the Mach number's scale being at
+  // least 2^-20)
+  float sum[NC];
 #pragma unroll
-      for (int k = 0; k < P1; ++k) acc = fma(entry(k), v[k * step], acc);
-    } else {
-      for (int k = 0; k < n; ++k) acc = fma(entry(k), v[k * step], acc);
+  for (int e = 0; e < NC; ++e) sum[e] = 0.f;
+  for (int t = lane; t < nq + nf; t += tpe)
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      if (t < nq) {
+        const int hi = (int)(rqi[e * nq + t] >> 32);
+        sum[e] += ((float)(hi < 0 ? ~hi : hi) + 1.f) * __int_as_float((127 + 32 - ns[t] - fx.K[t]) << 23);
+      } else {
+        const int ex = ((__double2hiint(ff[e * nf + t - nq]) >> 20) & 0x7ff) - 1022 - u(e) + fx.eR[t - nq];
+        sum[e] += __int_as_float(min(254, max(0, 127 + ex)) << 23);
+      }
     }
-    return acc;
-  };
-  if constexpr (D == 2) {
-    for (int t = lane; t < NC * p1 * M2; t += tpe) {
-      const int e = N::div(t, p1 * M2), s = t - e * p1 * M2, b1 = N::div(s, M2), a2 = s - b1 * M2;
-      Z[t] = line(M1, [&](int k) { return op.A[k + M1 * b1]; }, rq + e * nq + a2, M2);
-    }
-    __syncthreads();
-    for (int t = lane; t < NC * np; t += tpe) {
-      const int e = N::div(t, np), m = fx.modes[t - e * np], b1 = m & 0xff, b2 = (m >> 8) & 0xff;
-      X[t] = line(M2, [&](int k) { return op.B[k + M2 * (b1 + p1 * b2)]; }, Z + (e * p1 + b1) * M2, 1);
-    }
-  } else {
-    const int M3 = N::M3(op), nb12 = N::nb12(op);
-    for (int t = lane; t < NC * p1 * M2 * M3; t += tpe) {
-      const int e = N::div(t, p1 * M2 * M3), s = t - e * p1 * M2 * M3, b1 = N::div(s, M2 * M3), a = s - b1 * M2 * M3;
-      W[t] = line(M1, [&](int k) { return op.A[k + M1 * b1]; }, rq + e * nq + a, M2 * M3);
-    }
-    __syncthreads();
-    for (int t = lane; t < NC * nb12 * M3; t += tpe) {
-      const int e = N::div(t, nb12 * M3), s = t - e * nb12 * M3, q = N::div(s, M3), a3 = s - q * M3;
-      const int b1 = op.b12[q] & 0xff, b2 = op.b12[q] >> 8;
-      Z[t] = line(M2, [&](int k) { return op.B[k + M2 * (b1 + p1 * b2)]; }, W + (e * p1 + b1) * M2 * M3 + a3, M3);
-    }
-    __syncthreads();
-    for (int t = lane; t < NC * np; t += tpe) {
-      const int e = N::div(t, np), m = fx.modes[t - e * np], b1 = m & 0xff, b2 = (m >> 8) & 0xff, b3 = (m >> 16) & 0xff;
-      X[t] = line(M3, [&](int k) { return op.C[k + M3 * (b1 + p1 * (b2 + p1 * b3))]; },
-                  Z + (e * nb12 + op.b12_index[b1 + p1 * b2]) * M3, 1);
+  const int width = tpe < 32 ? tpe : 32, groups = tpe / width;
+#pragma unroll
+  for (int e = 0; e < NC; ++e) {
+    for (int o = width >> 1; o > 0; o >>= 1) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
+    if ((lane & (width - 1)) == 0) part[lane / width * NC + e] = sum[e];
+  }
+  __syncthreads();
+  if (lane < NC) {
+    float s = 0.f;
+    for (int g = 0; g < groups; ++g) s += part[g * NC + lane];
+    unit[lane] = max(-800, u(lane) + (__float_as_int(s * 1.0001f) >> 23) - 126);
+  }
+  __syncthreads();
+  for (int t = lane; t < NC * nf; t += tpe) F[t] = fo_from_double(ff[t], unit[N::div(t, nf)] - fx.eRmin);
+  __syncthreads();
+  for (int i = lane; i < nq; i += tpe) {
+    FxSums<NC> acc;
+#pragma unroll 4
+    for (int q = op.Rt_ptr[i]; q < op.Rt_ptr[i + 1]; ++q) acc.add(fx.Rt[q], F + op.Rt_idx[q], nf);
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      // both in units 2^-62 of 2^unit
+      const int sh = u(e) - ns[i] - fx.K[i] - unit[e] + 2 * kFoLow, d = fx.eRt - fx.eRmin;
+      const long long r = rqi[e * nq + i], f = acc.template value<0>(e);
+      Y[e * nq + i] = fo_split((sh >= 0 ? (long long)((unsigned long long)r << min(sh, 62)) : FxShift(min(-sh, 62))(r)) -
+                               (d >= 0 ? (long long)((unsigned long long)f << d) : FxShift(-d)(f)));
     }
   }
   __syncthreads();
-  fx_modal_units<NC>(X, nullptr, nullptr, np, unit, lane, tpe);
+  fx_vdm_tmul<D, NC, P1>(op, fx, Y, X, Z, W, lane, tpe);
+  int *unit2 = unit + NC;
+  fx_modal_units<NC>(X, fx.T, np, unit2, lane, tpe);
   __syncthreads();
-  for (int t = lane; t < NC * np; t += tpe) Xf[t] = fo_from_double(X[t], unit[N::div(t, np)]);
+  for (int t = lane; t < NC * np; t += tpe) {
+    const int e = N::div(t, np);
+    X[t] = fx_scale(X[t], fx.T[t - e * np] - unit2[e]);
+  }
   __syncthreads();
   double *out = ka.dudt + (size_t)kk * NC * np;
   for (int t = lane; t < NC * np; t += tpe) {
     const int e = N::div(t, np), a = t - e * np;
-    const long long v = fx_mass_row(fx.A_k + (size_t)kk * np * np, Xf + e * np, np, a);
-    const double x = fx_value(v, unit[e] == kFxBad ? kFxBad : unit[e] + fx.eA[kk]);
+    const long long v = fx_mass_row<12>(fx.A_k + (size_t)kk * np * np, X + e * np, np, a);
+    const double x = fx_value(v, unit[e] == kFxBad ? kFxBad : unit[e] + unit2[e] + fx.eA[kk]);
     if (live) {
       out[e * np + fx.order[a]] = x;
       if (!isfinite(x)) ka.flag_nonphysical();
@@ -956,6 +975,15 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
 
   for (int t = lane; t < nq + nf; t += tpe) ns[t] = fx.n[(size_t)kk * (nq + nf) + t];
   if (lane < 5) key[lane] = 0u;
+  // the element's slabs into L2 while the node values are formed (p = 4 tets:
+  // 2.35 -> 2.21 ms; triangles' are too small to gain)
+  if constexpr (D == 3) {
+    fx_prefetch(Lam, nq * D * D * sizeof(Fx), lane, tpe);
+    fx_prefetch(hnq, D * nfac * nq * sizeof(Fx), lane, tpe);
+    fx_prefetch(hnf, D * nf * sizeof(Fx), lane, tpe);
+    fx_prefetch(fx.bn + (size_t)kk * D * nf, D * nf * sizeof(Fx), lane, tpe);
+    if (fx.on_a) fx_prefetch(fx.A_k + (size_t)kk * op.np * op.np, op.np * op.np * sizeof(Fx), lane, tpe);
+  }
   // FP64 node values [rho, p, h, V] of the volume nodes, the facet nodes and
   // the facing nodes of the neighbours; the Lax-Friedrichs term of a facet
   // node from its two states
@@ -1022,22 +1050,12 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
       }
     }
   }
-  const int width = tpe < 32 ? tpe : 32;
-  for (int o = width >> 1; o > 0; o >>= 1) {
-    k0 = max(k0, __shfl_xor_sync(0xffffffffu, k0, o));
-    k1 = max(k1, __shfl_xor_sync(0xffffffffu, k1, o));
-    k2 = max(k2, __shfl_xor_sync(0xffffffffu, k2, o));
-    k3 = max(k3, __shfl_xor_sync(0xffffffffu, k3, o));
-    k4 = max(k4, __shfl_xor_sync(0xffffffffu, k4, o));
-  }
   __syncthreads();  // key cleared
-  if ((lane & (width - 1)) == 0) {
-    atomicMax(key + 0, k0);
-    atomicMax(key + 1, k1);
-    atomicMax(key + 2, k2);
-    atomicMax(key + 3, k3);
-    atomicMax(key + 4, k4);
-  }
+  fx_team_max(key + 0, k0, lane, tpe);
+  fx_team_max(key + 1, k1, lane, tpe);
+  fx_team_max(key + 2, k2, lane, tpe);
+  fx_team_max(key + 3, k3, lane, tpe);
+  fx_team_max(key + 4, k4, lane, tpe);
   __syncthreads();
   const int eG = fx.eG[kk];
   const FxScale sc(key, eG);
@@ -1111,11 +1129,8 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
     __syncthreads();
   }
 
-  // a sum of node t (its unit 2^-n_t smaller) in FP64
-  auto value = [&](int t, int e, long long v) {
-    const int unit = e == 0 ? sc.eR + eG + sc.eV - 63 : eP + eG - 61 + (e == D + 1 ? sc.eV : 0);
-    return fx_to_double(v, unit - ns[t]);
-  };
+  // a sum of node t counts units 2^(unit_of(e) - n_t)
+  auto unit_of = [&](int e) { return e == 0 ? sc.eR + eG + sc.eV - 63 : eP + eG - 61 + (e == D + 1 ? sc.eV : 0); };
   // facet correction and interface flux, chunked the same way; the sums are
   // subtracted from r_q (integers) and f_f (converted, FP64)
   const float rnpf = qrcp(npf > 0 ? npf : 1);
@@ -1158,17 +1173,21 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
         const bool own = p >= c0 && p < c1;
         const long long *dp = diff + (size_t)(own ? p - c0 : 0) * NC;
 #pragma unroll
-        for (int e = 0; e < NC; ++e) ff[e * nf + r] += value(t, e, (own ? dp[e] : 0) - acc[e]);
+        for (int e = 0; e < NC; ++e) ff[e * nf + r] += fx_to_double((own ? dp[e] : 0) - acc[e], unit_of(e) - ns[t]);
       }
     });
     __syncthreads();
   }
+  if (fx.on_a) {
+    fx_tail<D, NC, P1>(ka, rqi, ff, base + L.off[2], reinterpret_cast<int *>(key),
+                       reinterpret_cast<float *>(pair), ns, unit_of, kk, live, lane, tpe);
+    return;
+  }
   for (int i = lane; i < nq; i += tpe)
 #pragma unroll
-    for (int e = 0; e < NC; ++e) rq[e * nq + i] = value(i, e, rqi[e * nq + i]);
+    for (int e = 0; e < NC; ++e) rq[e * nq + i] = fx_to_double(rqi[e * nq + i], unit_of(e) - ns[i]);
   __syncthreads();
-  if (fx.on_a) fx_tail<D, NC, P1>(ka, rq, ff, base + L.off[2], reinterpret_cast<int *>(key), kk, live, lane, tpe);
-  else fd_tail<D, NC>(ka, rq, ff, base + L.off[2], kk, live, lane, tpe);
+  fd_tail<D, NC>(ka, rq, ff, base + L.off[2], kk, live, lane, tpe);
 }
 
 // Fixed-point metric terms of one element per block.  2^eG bounds every

@@ -63,6 +63,10 @@ struct FxTables {
   const Fx *A, *B, *C, *R, *A_k;
   const signed char *T, *K, *eR;
   const int *eA, *eW;
+  // R^T rows times 2^-K_i in units 2^eRt (absolute row sums at most 1; CSR values)
+  // and the smallest eR_j, for the tail of phase B
+  const Fx *Rt;
+  int eRt, eRmin;
   // modal vectors (T, A_k) are in the order of the sum factorisation: place l
   // holds mode order[l] = packed b1 | b2 << 8 | b3 << 16 modes[l]; those of one b1
   // (2-D) or (b1, b2) (3-D) start at base
