@@ -12,7 +12,15 @@
 // element's coordinates, derivatives and metric terms stay in shared memory
 // and only the GeometricFactors fields are written to HBM.  The reference
 // matrices (a few hundred KB at most) are read through L1/L2 by every CTA;
-// each load feeds 3 to 18 FMAs (the vectors sharing that matrix).
+// each load feeds 3 to 18 products (the vectors sharing that matrix).
+//
+// The matrix products of tetrahedra, nearly all of their work, run in block
+// fixed point (sse_fixed_ops.cuh): in FP64 the curl kernel kept the FP64 pipe
+// 99 % busy.  A matrix is scaled so that its absolute row sums are at most 1, a
+// vector to at most 1/4, and the cross products are carried over every four
+// terms, so that no sum overflows.  Products and metrics at the nodes stay in
+// FP64.  10,368 p = 4 tets, curl form, the whole call: 4.80 -> 1.99 ms.
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <utility>
@@ -22,6 +30,7 @@
 
 #include "../../include/sse_gb300.h"
 #include "sse_kernels.cuh"
+#include "sse_fixed_ops.cuh"
 
 namespace sse {
 namespace {
@@ -32,7 +41,75 @@ struct MetricArgs {
   const double *N1, *D1[3], *Vq1, *Vf1, *P;
   const double *xyz[3];
   double *J_q, *Lambda_q, *J_f, *nJf, *nJq;
+  // fixed-point copies (tetrahedra): Drst, Vq, Vf, Drst_Nplus1, Vq_Nplus1,
+  // Vf_Nplus1, project, each times 2^-exponent
+  const Fx *fDr[3], *fVq, *fVf, *fD1[3], *fVq1, *fVf1, *fP;
+  const int *ex;  // exponents in the order of kEx*
 };
+enum { kExDr = 0, kExVq, kExVf, kExD1, kExVq1, kExVf1, kExP, kExCount };
+
+// Fixed-point copies of one group of matrices (m x n, column-major) a block
+struct FixGroup {
+  const double *in[3];
+  Fx *out[3];
+  int count, m, n;
+};
+struct FixGroups {
+  FixGroup g[kExCount];
+};
+
+__global__ void __launch_bounds__(256) fix_matrices_kernel(FixGroups groups, int *ex) {
+  __shared__ unsigned row;
+  const FixGroup &f = groups.g[blockIdx.x];
+  if (threadIdx.x == 0) row = 0u;
+  __syncthreads();
+  for (int t = threadIdx.x; t < f.count * f.m; t += blockDim.x) {
+    const double *a = f.in[t / f.m] + t % f.m;
+    double s = 0.0;
+    for (int j = 0; j < f.n; ++j) s += fabs(a[(size_t)j * f.m]);
+    atomicMax(&row, (unsigned)__double2hiint(s * (1.0 + 1e-6)));
+  }
+  __syncthreads();
+  const int e = min(400, max(-400, fx_exponent(row)));
+  if (threadIdx.x == 0) ex[blockIdx.x] = row >= 0x7ff00000u ? kFxBad : e;
+  for (int c = 0; c < f.count; ++c)
+    for (int t = threadIdx.x; t < f.m * f.n; t += blockDim.x) f.out[c][t] = fo_from_double(f.in[c][t], e);
+}
+
+// The unit of values up to the one with upper word `key`: they are at most 1/4
+__device__ __forceinline__ int vector_unit(unsigned key) {
+  return key >= (1023u + 900u) << 20 ? kFxBad : max(-800, fx_exponent(key) + 2);
+}
+
+// x scaled in place to one unit, which is returned; *key: scratch in shared
+// memory, zero on entry.  Synchronises the block.
+__device__ __forceinline__ int fix_vectors(double *x, int count, unsigned *key) {
+  unsigned m = 0u;
+  for (int t = threadIdx.x; t < count; t += blockDim.x) m = max(m, (unsigned)__double2hiint(x[t]) & 0x7fffffffu);
+  fx_team_max(key, m, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int unit = vector_unit(*key);
+  Fx *f = reinterpret_cast<Fx *>(x);
+  for (int t = threadIdx.x; t < count; t += blockDim.x) f[t] = fo_from_double(x[t], unit);
+  __syncthreads();
+  return unit;
+}
+
+// Row i of A applied to NV vectors; acc in FP64
+template <int NV>
+__device__ __forceinline__ void fix_row(const Fx *__restrict__ A, int m, int n, int i, const Fx *x, int xs, int unit,
+                                        double *acc) {
+  FxSums<NV> s;
+  int j = 0;
+  for (; j + 4 <= n; j += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s.add(A[i + (size_t)(j + q) * m], x + j + q, xs);
+    s.fold();
+  }
+  for (; j < n; ++j) s.add(A[i + (size_t)j * m], x + j, xs);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) acc[v] = fx_value(s.template value<0>(v), unit);
+}
 
 template <int NA>
 struct Mats {
@@ -160,20 +237,35 @@ __device__ __forceinline__ void load_xyz(const MetricArgs &g, int64_t k, int D, 
 template <int D>
 __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   extern __shared__ double sm[];
+  __shared__ unsigned key[3];
   const int64_t k = blockIdx.x;
   double *X = sm;
   double *G = X + D * g.n_map;          // G[(a * D + c)] = D_a x_c
   double *Jq = G + D * D * g.n_map;
   load_xyz(g, k, D, X);
-  Mats<D> Dm;
+  if (threadIdx.x < 3) key[threadIdx.x] = 0u;
+  __syncthreads();
+  int uG = 0;
+  if constexpr (D == 2) {
+    matvecs<D, D>(Mats<D>{{g.Dr[0], g.Dr[1]}}, g.n_map, g.n_map, X, g.n_map, G, g.n_map);
+    __syncthreads();
+  } else {
+    const int uX = fix_vectors(X, D * g.n_map, key);
+    for (int t = threadIdx.x; t < D * g.n_map; t += blockDim.x) {
+      const int a = t / g.n_map, i = t - a * g.n_map;
+      double acc[D];
+      fix_row<D>(g.fDr[a], g.n_map, g.n_map, i, reinterpret_cast<const Fx *>(X), g.n_map, uX + g.ex[kExDr], acc);
 #pragma unroll
-  for (int a = 0; a < D; ++a) Dm.p[a] = g.Dr[a];
-  __syncthreads();
-  matvecs<D, D>(Dm, g.n_map, g.n_map, X, g.n_map, G, g.n_map);
-  __syncthreads();
+      for (int c = 0; c < D; ++c) G[(a * D + c) * g.n_map + i] = acc[c];
+    }
+    __syncthreads();
+    uG = fix_vectors(G, D * D * g.n_map, key + 1);
+  }
+  const Fx *Gf = reinterpret_cast<const Fx *>(G);
   for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
     double acc[D * D];
-    row_apply<D * D>(g.Vq, g.n_q, g.n_map, i, G, g.n_map, acc);
+    if constexpr (D == 2) row_apply<D * D>(g.Vq, g.n_q, g.n_map, i, G, g.n_map, acc);
+    else fix_row<D * D>(g.fVq, g.n_q, g.n_map, i, Gf, g.n_map, uG + g.ex[kExVq], acc);
     double a[D][D], adj[D][D];
 #pragma unroll
     for (int m = 0; m < D; ++m)
@@ -192,7 +284,8 @@ __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   }
   for (int i = threadIdx.x; i < g.n_f; i += blockDim.x) {
     double acc[D * D];
-    row_apply<D * D>(g.Vf, g.n_f, g.n_map, i, G, g.n_map, acc);
+    if constexpr (D == 2) row_apply<D * D>(g.Vf, g.n_f, g.n_map, i, G, g.n_map, acc);
+    else fix_row<D * D>(g.fVf, g.n_f, g.n_map, i, Gf, g.n_map, uG + g.ex[kExVf], acc);
     double a[D][D], adj[D][D];
 #pragma unroll
     for (int m = 0; m < D; ++m)
@@ -208,9 +301,12 @@ __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   }
   if (g.project) {
     __syncthreads();
+    int uJ = 0;
+    if constexpr (D == 3) uJ = fix_vectors(Jq, g.n_q, key + 2);
     for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
       double acc[1];
-      row_apply<1>(g.P, g.n_q, g.n_q, i, Jq, g.n_q, acc);
+      if constexpr (D == 2) row_apply<1>(g.P, g.n_q, g.n_q, i, Jq, g.n_q, acc);
+      else fix_row<1>(g.fP, g.n_q, g.n_q, i, reinterpret_cast<const Fx *>(Jq), 0, uJ + g.ex[kExP], acc);
       g.J_q[(size_t)g.n_q * k + i] = acc[0];
     }
   }
@@ -260,9 +356,13 @@ __global__ void __launch_bounds__(128) curl_metrics_2d_kernel(MetricArgs g) {
 //   (J ∇ξ_a)_n = -ê_n · ∇_ξ × (x_l ∇_ξ x_m),
 // brought back through Vq * Nplus1_to_N.  Shared memory: X[3][n_map],
 // G[9][n_map], Jm[n_map], X1[3][n1], G1[9][n1] (reused for the metric terms),
-// F[9][n1].
+// F[9][n1].  The coordinates' own derivatives stay in FP64: the curl amplifies
+// their rounding, and other (smaller) errors there would move the results by
+// more than the FP64 evaluations differ among themselves.  Two warps an element
+// at p = 4, whose 56 nodes of degree 5 set the length of the large steps.
 __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
   extern __shared__ double sm[];
+  __shared__ unsigned key[3];
   const int64_t k = blockIdx.x;
   const int nm = g.n_map, n1 = g.n1;
   double *X = sm;
@@ -272,6 +372,7 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
   double *G1 = X1 + 3 * n1;   // D1_a x1_c, later the metric terms M[m + 3 n]
   double *F = G1 + 9 * n1;    // F[p * 3 + a]
   load_xyz(g, k, 3, X);
+  if (threadIdx.x < 3) key[threadIdx.x] = 0u;
   __syncthreads();
   matvecs<3, 3>(Mats<3>{{g.Dr[0], g.Dr[1], g.Dr[2]}}, nm, nm, X, nm, G, nm);
   matvecs<1, 3>(Mats<1>{{g.N1}}, n1, nm, X, nm, X1, n1);
@@ -282,13 +383,14 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
     const double xt = G[6 * nm + i], yt = G[7 * nm + i], zt = G[8 * nm + i];
     Jm[i] = xr * (ys * zt - zs * yt) - yr * (xs * zt - zs * xt) + zr * (xs * yt - ys * xt);
   }
+  const int uJ = fix_vectors(Jm, nm, key);
   matvecs<3, 3>(Mats<3>{{g.D1[0], g.D1[1], g.D1[2]}}, n1, n1, X1, n1, G1, n1);
-  __syncthreads();
   for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
     double acc[1];
-    row_apply<1>(g.Vq, g.n_q, nm, i, Jm, nm, acc);
+    fix_row<1>(g.fVq, g.n_q, nm, i, reinterpret_cast<const Fx *>(Jm), 0, uJ + g.ex[kExVq], acc);
     g.J_q[(size_t)g.n_q * k + i] = acc[0];
   }
+  __syncthreads();
   // pairs (differentiated, multiplier): (y, z) -> n = x, (x, z) -> n = y
   // (negated), (y, x) -> n = z (negated)
   for (int i = threadIdx.x; i < n1; i += blockDim.x) {
@@ -299,50 +401,48 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
       for (int a = 0; a < 3; ++a) F[(p * 3 + a) * n1 + i] = G1[(a * 3 + dc[p]) * n1 + i] * X1[mc[p] * n1 + i];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n1; i += blockDim.x) {
-    // per pair: D_t F_s, D_s F_t, D_r F_t, D_t F_r, D_s F_r, D_r F_s
-    double acc[3][6];
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) acc[p][q] = 0.0;
+  const int uF = fix_vectors(F, 9 * n1, key + 1) + g.ex[kExD1];
+  const Fx *Ff = reinterpret_cast<const Fx *>(F);
+  for (int t = threadIdx.x; t < 3 * n1; t += blockDim.x) {
+    // of pair p: D_t F_s - D_s F_t, D_r F_t - D_t F_r, D_s F_r - D_r F_s
+    const int p = t / n1, i = t - p * n1;
+    const Fx *f = Ff + 3 * p * n1;
+    FxSums<1> c[3];
+    auto minus = [](Fx a) { return Fx{-a.lo, -a.hi}; };
+#pragma unroll 2
     for (int j = 0; j < n1; ++j) {
       const size_t o = i + (size_t)j * n1;
-      const double dr = __ldg(g.D1[0] + o), ds = __ldg(g.D1[1] + o), dt = __ldg(g.D1[2] + o);
+      if ((j & 1) == 0)
 #pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        const double fr = F[(p * 3 + 0) * n1 + j], fs = F[(p * 3 + 1) * n1 + j],
-                     ft = F[(p * 3 + 2) * n1 + j];
-        acc[p][0] = fma(dt, fs, acc[p][0]);
-        acc[p][1] = fma(ds, ft, acc[p][1]);
-        acc[p][2] = fma(dr, ft, acc[p][2]);
-        acc[p][3] = fma(dt, fr, acc[p][3]);
-        acc[p][4] = fma(ds, fr, acc[p][4]);
-        acc[p][5] = fma(dr, fs, acc[p][5]);
-      }
+        for (int q = 0; q < 3; ++q) c[q].fold();
+      const Fx dr = g.fD1[0][o], ds = g.fD1[1][o], dt = g.fD1[2][o];
+      const Fx *fr = f + j, *fs = f + n1 + j, *ft = f + 2 * n1 + j;
+      c[0].add(dt, fs, 0);
+      c[0].add(minus(ds), ft, 0);
+      c[1].add(dr, ft, 0);
+      c[1].add(minus(dt), fr, 0);
+      c[2].add(ds, fr, 0);
+      c[2].add(minus(dr), fs, 0);
     }
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      const double c0 = acc[p][0] - acc[p][1];
-      const double c1 = acc[p][2] - acc[p][3];
-      const double c2 = acc[p][4] - acc[p][5];
-      const double sgn = p == 0 ? 1.0 : -1.0;
-      G1[(0 + 3 * p) * n1 + i] = sgn * c0;
-      G1[(1 + 3 * p) * n1 + i] = sgn * c1;
-      G1[(2 + 3 * p) * n1 + i] = sgn * c2;
+    for (int q = 0; q < 3; ++q) {
+      const double v = fx_value(c[q].template value<0>(0), uF);
+      G1[(q + 3 * p) * n1 + i] = p == 0 ? v : -v;
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
+  const int uM = fix_vectors(G1, 9 * n1, key + 2);
+  const Fx *Mf = reinterpret_cast<const Fx *>(G1);
+  for (int t = threadIdx.x; t < g.n_q + g.n_f; t += blockDim.x) {
     double L[9];
-    row_apply<9>(g.Vq1, g.n_q, n1, i, G1, n1, L);
-    store_lambda<3>(g, k, i, L);
-    write_nJq<3>(g, k, i, L);
-  }
-  for (int i = threadIdx.x; i < g.n_f; i += blockDim.x) {
-    double L[9];
-    row_apply<9>(g.Vf1, g.n_f, n1, i, G1, n1, L);
-    write_nJf<3>(g, k, i, L);
+    if (t < g.n_q) {
+      fix_row<9>(g.fVq1, g.n_q, n1, t, Mf, n1, uM + g.ex[kExVq1], L);
+      store_lambda<3>(g, k, t, L);
+      write_nJq<3>(g, k, t, L);
+    } else {
+      fix_row<9>(g.fVf1, g.n_f, n1, t - g.n_q, Mf, n1, uM + g.ex[kExVf1], L);
+      write_nJf<3>(g, k, t - g.n_q, L);
+    }
   }
 }
 
@@ -464,6 +564,36 @@ int geometric_factors_run(const sse_metric_operators *ops, int64_t n_e, const do
   if (g.project) pack.add(ops->project, (size_t)nq * nq, &g.P);
   if ((e = pack.upload(buf)) != cudaSuccess) return cuda(e, "upload reference matrices");
 
+  if (d == 3) {
+    const double *const none[3] = {nullptr, nullptr, nullptr};
+    const double *const Vq[3] = {g.Vq}, *const Vf[3] = {g.Vf}, *const Vq1[3] = {g.Vq1},
+                 *const Vf1[3] = {g.Vf1}, *const P[3] = {g.P};
+    struct Group { const double *const *in; const Fx **out; int count, m, n; };
+    const Group all[kExCount] = {{g.Dr, g.fDr, curl3 ? 0 : 3, nm, nm}, {Vq, &g.fVq, 1, nq, nm}, {Vf, &g.fVf, curl3 ? 0 : 1, nf, nm},
+                                 {curl3 ? g.D1 : none, g.fD1, curl3 ? 3 : 0, n1, n1},
+                                 {Vq1, &g.fVq1, curl3, nq, n1}, {Vf1, &g.fVf1, curl3, nf, n1}, {P, &g.fP, g.project, nq, nq}};
+    size_t total = 0;
+    for (const Group &a : all) total += (size_t)a.count * a.m * a.n;
+    void *p = nullptr;
+    if ((e = buf.alloc(total * sizeof(Fx) + kExCount * sizeof(int), &p)) != cudaSuccess) return cuda(e, "allocate");
+    Fx *next = (Fx *)p;
+    FixGroups groups{};
+    for (int t = 0; t < kExCount; ++t) {
+      groups.g[t].count = all[t].count;
+      groups.g[t].m = all[t].m;
+      groups.g[t].n = all[t].n;
+      for (int c = 0; c < all[t].count; ++c) {
+        groups.g[t].in[c] = all[t].in[c];
+        groups.g[t].out[c] = next;
+        all[t].out[c] = next;
+        next += (size_t)all[t].m * all[t].n;
+      }
+    }
+    g.ex = (const int *)next;
+    fix_matrices_kernel<<<kExCount, 256>>>(groups, (int *)next);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda(e, "fixed-point matrices");
+  }
+
   const size_t ne = (size_t)n_e;
   const size_t len[5] = {(size_t)nq * ne, (size_t)nq * d * d * ne, (size_t)nf * ne,
                          (size_t)d * nf * ne, (size_t)d * ops->num_faces * nq * ne};
@@ -487,7 +617,8 @@ int geometric_factors_run(const sse_metric_operators *ops, int64_t n_e, const do
   g.nJf = dev_out[3];
   g.nJq = dev_out[4];
 
-  const int threads = d == 2 ? 32 : 128;
+  // the curl kernel: whole warps for the n1 nodes of its large steps
+  const int threads = d == 2 ? 32 : (curl3 ? std::min(128, (n1 + 31) / 32 * 32) : 128);
   const dim3 grid((unsigned)n_e);
   if (ops->metrics == SSE_EXACT_METRICS) {
     if (d == 2) {

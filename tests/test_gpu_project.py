@@ -47,3 +47,24 @@ def test_projection_rejects_a_negative_jacobian(gpu_lib, pkg):
     with pytest.raises(pkg.SSEError) as e:
         pkg.gb300.project_function(sd.reference_approximation, J, uq)
     assert e.value.code == pkg.abi.SSE_ERR_NONPHYSICAL
+
+
+@pytest.mark.parametrize("shape,p", [("Tri", 1), ("Tri", 2), ("Tri", 5), ("Tet", 1), ("Tet", 3), ("Tet", 6)])
+@pytest.mark.parametrize("scale", [1.0, 3.0e-40, 7.0e30])
+def test_sizes_and_units(gpu_lib, pkg, shape, p, scale):
+    """Tiles of M that np does not fill, node counts that are no multiple of
+    four, and data far from one: within 1e-12 of each projection's largest
+    coefficient (as test_projection's whole-vector bound), and an element of zero
+    data stays zero."""
+    d = 2 if shape == "Tri" else 3
+    ra = cases.R.reference_approximation("ModalTensor", shape, p, mapping_degree=p)
+    mesh = cases.M.uniform_periodic_mesh(ra, ((0.0, 1.0),) * d, (2,) * d)
+    J = cases.M.spatial_discretization(mesh, ra, metrics="Exact").geometric_factors.J_q
+    uq = scale * (1.0 + np.stack([np.sin(x) for x in mesh.xyzq], axis=1))
+    uq[0] = 0.0
+    got = pkg.gb300.project_function(ra, J, np.ascontiguousarray(uq))
+    V, WJ = ra.V, ra.W[None, :] * J
+    mass = np.einsum("qa,kq,qb->kab", V, WJ, V)
+    want = np.linalg.solve(mass, np.einsum("qa,keq->kae", V, uq * WJ[:, None, :])).transpose(0, 2, 1)
+    assert np.all(got[0] == 0.0)
+    assert np.abs(got - want).max() <= 1.0e-12 * np.abs(want).max()
