@@ -54,7 +54,7 @@ struct CsrHost {
 
 struct sse_solver {
   sse_config cfg{};
-  KernelArgs ka{};
+  FxArgs ka{};
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::vector<void *> allocations;  // device buffers owned by the handle
@@ -247,7 +247,7 @@ struct FxLists {
 // as integers with its own factor 2^k, and the incidence lists with k.
 int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vector<double> &vp_S,
                    const std::vector<double> &C, const std::vector<std::vector<int>> &fp_inc, FxLists *lists) {
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const int d = s->cfg.d, nq = s->cfg.n_q, nvp = (int)vp_ij.size();
   auto largest = [](const double *v, size_t n) {
     double m = 0.0;
@@ -307,7 +307,7 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
 // `most` for which the team takes the fewest steps; a node's 1, 2 or 4 parts are
 // adjacent tasks.
 int setup_fx_sums(sse_solver *s, const FxLists &lists) {
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const int CH = ka.fx_chunk, tpe = ka.tpb_bx / ka.epb_bx;
   auto build = [&](const std::vector<std::vector<int>> &inc, int pairs, FxTables::Sums *S) {
     const int chunks = (pairs + CH - 1) / CH, n = (int)inc.size();
@@ -380,7 +380,7 @@ int setup_fx_sums(sse_solver *s, const FxLists &lists) {
 // tensor-product V of at most 8 nodes and modes a direction (the sums of cross
 // products then stay below 2^63).
 int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   FxTables &fx = ka.fx;
   const sse_config &c = s->cfg;
   const DevOps &op = ka.op;
@@ -473,7 +473,7 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
 
 // Fixed-point mass operators, by the same rule on memory as the metric terms
 int setup_fx_mass(sse_solver *s) {
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const sse_config &c = s->cfg;
   const size_t ne = c.n_e, n = ne * c.n_p * c.n_p;
   size_t freeb = 0, totalb = 0;
@@ -497,7 +497,7 @@ int setup_fx_mass(sse_solver *s) {
 // Fixed-point metric terms, when they take at most a quarter of the free
 // device memory; without them phase B runs in FP64.
 int setup_fx_geometry(sse_solver *s) {
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const sse_config &c = s->cfg;
   const size_t ne = c.n_e, nl = ne * c.n_q * c.d * c.d, nh = ne * c.n_q * c.d * c.num_faces, nf = ne * c.n_f * c.d;
   size_t freeb = 0, totalb = 0;
@@ -529,7 +529,7 @@ int setup_fx_geometry(sse_solver *s) {
 // configuration outside that scope keeps the two-phase kernels.
 int setup_compact(sse_solver *s, const sse_operators *ops, const std::vector<int> &mapP) {
   const sse_config &c = s->cfg;
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const int np = c.n_p, nq = c.n_q, nf = c.n_f, d = c.d, nc = c.n_c;
   const int npf = c.nodes_per_face, nfac = c.num_faces;
   ka.compact = 0;
@@ -772,7 +772,7 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   }
 
   s->cfg = c;
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   DevOps &op = ka.op;
   op.d = c.d; op.nc = c.n_c; op.np = c.n_p; op.nq = c.n_q; op.nf = c.n_f;
   op.nfac = c.num_faces; op.npf = c.nodes_per_face;
@@ -1194,7 +1194,7 @@ int enable_mixed(sse_solver *s) {
   if (s->ka.op.has_vdm && s->mode0 < 0)
     return fail(s, SSE_ERR_UNSUPPORTED, "SSE_MIXED needs a modal basis with a constant basis function");
   if (s->mixed_ready) return SSE_OK;
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   DevOps &op = ka.op;
   DevGeo &g = ka.geo;
   cudaError_t e;
@@ -1501,7 +1501,7 @@ int ensure_reference(sse_solver *s, const double *u_dev) {
   {
     double uref[5] = {ph.rho_ref, 0.0, 0.0, 0.0, 0.0};
     uref[c.n_c - 1] = ph.E_ref;
-    KernelArgs kb = s->ka;
+    FxArgs kb = s->ka;
     kb.mixed = 0;
     kb.dudt = s->d_rref;
     if ((e = launch_fill_constant_state(kb.u_q, c.n_q, c.n_c, c.n_e, uref, s->stream)) ||
@@ -1522,7 +1522,7 @@ int ensure_reference(sse_solver *s, const double *u_dev) {
 cudaError_t residual_device(sse_solver *s, const double *u, double *dudt, double *u_q = nullptr,
                             double *u_f = nullptr, bool two_phase = false) {
   if (s->ka.mixed && !s->ref_ready && ensure_reference(s, u) != SSE_OK) return cudaErrorInvalidValue;
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   // (a residual written over its own input, which the neighbours' traces
   // read, takes the two-phase kernels)
   if (ka.compact && !u_q && !two_phase && dudt != u) {
@@ -1567,7 +1567,7 @@ int enable_adjoint(sse_solver *s) {
   if (!s->mapP_involution)
     return fail(s, SSE_ERR_UNSUPPORTED, "the discrete adjoint needs mapP to pair facet nodes (mapP(mapP(x)) == x)");
   if (s->adj_ready) return SSE_OK;
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const DevOps &op = ka.op;
   const int nc = c.n_c, np = c.n_p, nq = c.n_q, nf = c.n_f, d = c.d, ps = 3 + d;
   int zsz = 0, wsz = 0;
@@ -1652,7 +1652,7 @@ int enable_adjoint(sse_solver *s) {
 int enable_adjoint_mixed(sse_solver *s) {
   if (s->adj_mixed_ready) return SSE_OK;
   const sse_config &c = s->cfg;
-  KernelArgs &ka = s->ka;
+  FxArgs &ka = s->ka;
   const DevOps &op = ka.op;
   if (!op.has_vdm)
     return fail(s, SSE_ERR_UNSUPPORTED, "the mixed-form adjoint covers modal (ModalTensor) bases");
@@ -1701,7 +1701,7 @@ int enable_adjoint_mixed(sse_solver *s) {
 // mu = (dR/du)^T lam for the mixed form at u: its phase A writes the FP32
 // perturbation states, then the FP32 transposes run with lam~.
 cudaError_t vjp_device_mixed(sse_solver *s, const double *u, const double *lam, double *mu) {
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   ka.mixed = 1;
   ka.u = u;
   ka.lam = lam;
@@ -1715,7 +1715,7 @@ cudaError_t vjp_device_mixed(sse_solver *s, const double *u, const double *lam, 
 // u when already computed (a recorded stage), else phase A runs first.
 cudaError_t vjp_device(sse_solver *s, const double *u, const double *lam, double *mu,
                        const double *u_q = nullptr, const double *u_f = nullptr) {
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   ka.mixed = 0;
   ka.u = u;
   ka.lam = lam;
@@ -2042,7 +2042,7 @@ int32_t sse_residual_static_scratch(sse_solver *s, const double *u_dev, double *
   // the mixed form picks its reference state on its first call; that uses
   // buffers the handle allocated when SSE_MIXED was set, and synchronises
   if (mixed && (rc = ensure_reference(s, u_dev)) != SSE_OK) return rc;
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   ka.u = u_dev;
   ka.dudt = dudt_dev;
   // the nodal states are fully written by phase A before phase B reads
@@ -2073,7 +2073,7 @@ int32_t sse_nodal_values(sse_solver *s, const double *u, double *u_q, double *u_
   } else if (memory != SSE_DEVICE) {
     return fail(s, SSE_ERR_INVALID_ARGUMENT, "memory must be SSE_HOST or SSE_DEVICE");
   }
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   ka.mixed = 0;  // FP64 nodal values in the reference's layouts
   ka.u = du;
   if ((e = launch_nodal_values(ka, s->stream))) return cuda_fail(s, e, "nodal values");
@@ -2702,7 +2702,7 @@ int32_t sse_phase_timings(sse_solver *s, const double *u_dev, int32_t n_iter, do
     int rc = ensure_reference(s, u_dev);
     if (rc != SSE_OK) return rc;
   }
-  KernelArgs ka = s->ka;
+  FxArgs ka = s->ka;
   ka.u = u_dev;
   ka.dudt = s->d_dudt;
   size_t n = (size_t)s->cfg.n_p * s->cfg.n_c * s->cfg.n_e;

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
 // with the FP64 operators (40 modal configurations, p = 2 to 6).
 // ---------------------------------------------------------------------------
 template <int D, int NC, int P1>
-__global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_constant__ KernelArgs ka) {
+__global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_constant__ FxArgs ka) {
   static_assert(NC == D + 2, "Euler");
   extern __shared__ double smem[];
   const DevOps &op = ka.op;
@@ -860,7 +860,7 @@ struct FxScale {
 //   S_e = sum_i |r_q,i| 2^-K_i + sum_j |f_f,j| 2^eR_j,
 // which is formed for the element at hand.
 template <int D, int NC, int P1, typename Unit>
-__device__ __forceinline__ void fx_tail(const KernelArgs &ka, const long long *rqi, const double *ff, double *scratch,
+__device__ __forceinline__ void fx_tail(const FxArgs &ka, const long long *rqi, const double *ff, double *scratch,
                                         int *unit, float *part, const signed char *ns, Unit u, int kk, bool live, int lane, int tpe) {
   using N = FxSize<D, P1>;
   const DevOps &op = ka.op;
@@ -945,7 +945,7 @@ __device__ __noinline__ void fd_fp64(const KernelArgs &ka, double *base, int kk,
 }
 
 template <int D, int NC, int P1>
-__global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __grid_constant__ KernelArgs ka) {
+__global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __grid_constant__ FxArgs ka) {
   static_assert(NC == D + 2, "Euler");
   extern __shared__ double smem[];
   const DevOps &op = ka.op;
@@ -1195,7 +1195,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
 // halfnJ at most 1/2; 2^-n_i bounds the sum of |G|_1 over the pairs of node i
 // in that unit (no sum of fluxes overflows).
 template <int D>
-__global__ void __launch_bounds__(128) fx_geometry_kernel(KernelArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
+__global__ void __launch_bounds__(128) fx_geometry_kernel(FxArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
                                                           signed char *on, int *oeG) {
   __shared__ double sh[3][128];
   const DevOps &op = ka.op;
@@ -2298,12 +2298,12 @@ __global__ void __launch_bounds__(256) energy_kernel(KernelArgs ka, const double
 // the fixed-point kernels of this configuration: compiled for 3 to 6 nodes a
 // direction, and for any number
 template <int P1>
-static const void *fx_kernel(const KernelArgs &ka, bool a) {
+static const void *fx_kernel(const FxArgs &ka, bool a) {
   if (ka.op.d == 2)
     return a ? (const void *)nodal_values_fx_kernel<2, 4, P1> : (const void *)fd_time_derivative_fx_kernel<2, 4, P1>;
   return a ? (const void *)nodal_values_fx_kernel<3, 5, P1> : (const void *)fd_time_derivative_fx_kernel<3, 5, P1>;
 }
-static const void *fx_kernel(const KernelArgs &ka, bool a, int p1) {
+static const void *fx_kernel(const FxArgs &ka, bool a, int p1) {
   switch (p1) {
     case 3: return fx_kernel<3>(ka, a);
     case 4: return fx_kernel<4>(ka, a);
@@ -2312,10 +2312,10 @@ static const void *fx_kernel(const KernelArgs &ka, bool a, int p1) {
     default: return fx_kernel<0>(ka, a);
   }
 }
-static const void *fx_kernel_a(const KernelArgs &ka) { return fx_kernel(ka, true, ka.fx.p1_a); }
-static const void *fx_kernel_b(const KernelArgs &ka) { return fx_kernel(ka, false, ka.fx.p1_b); }
+static const void *fx_kernel_a(const FxArgs &ka) { return fx_kernel(ka, true, ka.fx.p1_a); }
+static const void *fx_kernel_b(const FxArgs &ka) { return fx_kernel(ka, false, ka.fx.p1_b); }
 
-cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
+cudaError_t sse_set_smem_limits(const FxArgs &ka, size_t smA, size_t smB) {
   cudaError_t e = cudaSuccess;
   auto set = [&](const void *f, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -2331,7 +2331,7 @@ cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB) {
   return e;
 }
 
-cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st) {
+cudaError_t launch_nodal_values(const FxArgs &ka, cudaStream_t st) {
   int grid = (ka.ne + ka.epb - 1) / ka.epb;
   if (ka.mixed && ka.op.has_vdm && ka.geo.P1) {
     // the mixed phase A has its own team geometry (epb_am elements per block
@@ -2348,7 +2348,7 @@ cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st) {
   // the fixed-point operators wherever their tables exist (EC flux, modal
   // tensor-product basis)
   if (ka.fx.on_a) {
-    KernelArgs kx = ka;
+    FxArgs kx = ka;
     kx.epb = ka.epb_ax;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
     const size_t smx = (size_t)kx.epb * ka.layAx.team_doubles * sizeof(double);
@@ -2420,7 +2420,7 @@ cudaError_t sse_set_smem_limit_mixed(const KernelArgs &ka, size_t smBm) {
   return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smBm);
 }
 
-cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
+cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st) {
   int grid = (ka.ne + ka.epb - 1) / ka.epb;
   size_t sm = (size_t)ka.epb * ka.layB.team_doubles * sizeof(double);
   if (ka.mixed) {
@@ -2445,7 +2445,7 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
   // the fixed-point passes wherever their tables exist (the EC flux with
   // gamma <= 1.7); their blocks choose FP64 for themselves
   if (ka.fx.on) {
-    KernelArgs kx = ka;
+    FxArgs kx = ka;
     kx.epb = ka.epb_bx;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
     sm = (size_t)kx.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
@@ -2459,14 +2459,14 @@ cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
+cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st) {
   if (ka.op.d == 2) fx_geometry_kernel<2><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
   else fx_geometry_kernel<3><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
   return cudaGetLastError();
 }
 
-cudaError_t launch_fx_mass_operators(const KernelArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st) {
+cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st) {
   fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.fx.order, ka.op.np, ka.op.nq, A, eA, eW);
   return cudaGetLastError();
 }

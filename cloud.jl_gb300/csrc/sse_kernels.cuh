@@ -80,13 +80,9 @@ constexpr int kFxNone = -100000;
 
 struct KernelArgs {
   DevOps op;
-  FxTables fx;
   DevGeo geo;
   Physics ph;
   Layout layA, layB;
-  Layout layAx;      // fixed-point phase A: 0 X, 1 Y, 2 Z, 3 W, 4 units and extremes
-  Layout layBx;      // fixed-point phase B: 0 facet fluxes, 1 r_q, 2 pair buffer and tail scratch,
-                     // 3 node values, 4 float pairs, 5 extremes, 6 node shifts
   Layout layBm;      // mixed-form phase B layout, offsets and team size in floats:
                      // 0 volume states (then r_q), 1 facet states, 2 facet fluxes,
                      // 3 mass operator, 4 pair buffer, 5 Lambda_q, 6 halfnJq,
@@ -126,10 +122,7 @@ struct KernelArgs {
   int pair_chunk;    // pairs per shared-memory chunk in the pair-adjoint passes
   int pair_chunk_generic;  // the same for the conservative two-point flux
   int fd_chunk;      // pairs per chunk in the FP64 flux-differencing passes
-  int fx_chunk;      // pairs per chunk in the fixed-point passes
   int vp_split;      // volume pairs per interface lane in the one-chunk pass (0: even split)
-  int epb_ax, tpb_ax;  // elements and threads per block of the fixed-point phase A
-  int epb_bx, tpb_bx;  // elements and threads per block of the fixed-point phase B
   int epb_bm;        // elements per block of the FP32 phase-B kernel (blocks of tpb threads)
   int epb_am;        // elements per block of the mixed phase-A kernel (blocks of tpb threads)
   int epb_a;         // elements per block of the FP64 phase-A kernel (blocks of tpb threads)
@@ -156,6 +149,19 @@ struct KernelArgs {
   __device__ __forceinline__ void flag_nonphysical() const { atomicOr(flag, 1); }
   // a bounded wait on a device copy gave up (reported as SSE_ERR_CUDA)
   __device__ __forceinline__ void flag_timeout() const { atomicOr(flag, 2); }
+};
+
+// The fixed-point kernels' arguments; the others take the base alone (the tables
+// in every kernel's parameters made a time loop of short launches 224 us, 218
+// without).
+struct FxArgs : KernelArgs {
+  FxTables fx;
+  Layout layAx;      // fixed-point phase A: 0 X, 1 Y, 2 Z, 3 W, 4 units and extremes
+  Layout layBx;      // fixed-point phase B: 0 facet fluxes, 1 r_q, 2 pair buffer and tail scratch,
+                     // 3 node values, 4 float pairs, 5 extremes, 6 node shifts
+  int fx_chunk;      // pairs per chunk in the fixed-point passes
+  int epb_ax, tpb_ax;  // elements and threads per block of the fixed-point phase A
+  int epb_bx, tpb_bx;  // elements and threads per block of the fixed-point phase B
 };
 
 // most elements (warps) per block of std_compact_kernel
@@ -185,7 +191,7 @@ struct CompactStage {
   double *out;
 };
 
-cudaError_t sse_set_smem_limits(const KernelArgs &ka, size_t smA, size_t smB);
+cudaError_t sse_set_smem_limits(const FxArgs &ka, size_t smA, size_t smB);
 cudaError_t sse_set_smem_limit_compact(const KernelArgs &ka, size_t bytes);
 cudaError_t launch_std_compact(const KernelArgs &ka, const CompactStage &st, cudaStream_t s);
 // column a of V (np blocks; V applied to the unit vectors), nq x np column-major
@@ -217,15 +223,15 @@ cudaError_t launch_round_transpose(const double *in, float *out, size_t nmat, in
 // M is FP64 scratch of n_p x 4 quads doubles
 cudaError_t launch_tail_operators(const KernelArgs &ka, const double *Vd, double *M, float *E, int quads,
                                   cudaStream_t st);
-cudaError_t launch_nodal_values(const KernelArgs &ka, cudaStream_t st);
+cudaError_t launch_nodal_values(const FxArgs &ka, cudaStream_t st);
 cudaError_t launch_projection_of_one(const KernelArgs &ka, double *P1, double *RP1, cudaStream_t st);
 cudaError_t sse_set_smem_limits_mixed_a(const KernelArgs &ka);
-cudaError_t launch_time_derivative(const KernelArgs &ka, cudaStream_t st);
+cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st);
 // the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG)
-cudaError_t launch_fx_geometry(const KernelArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
+cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st);
 // the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW)
-cudaError_t launch_fx_mass_operators(const KernelArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st);
+cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st);
 cudaError_t launch_mass_operator(const KernelArgs &ka, double *Ak, cudaStream_t st);
 cudaError_t launch_energy(const KernelArgs &ka, const double *u, const double *dudt, double *partial,
                           cudaStream_t st);
