@@ -494,7 +494,8 @@ int setup_fx_mass(sse_solver *s) {
   return SSE_OK;
 }
 
-// Fixed-point metric terms, when they take at most a quarter of the free
+// Fixed-point metric terms, when the kernel that forms them fits in shared
+// memory and they take at most a quarter of the free
 // device memory; without them phase B runs in FP64.
 int setup_fx_geometry(sse_solver *s) {
   FxArgs &ka = s->ka;
@@ -503,7 +504,7 @@ int setup_fx_geometry(sse_solver *s) {
   size_t freeb = 0, totalb = 0;
   cudaError_t e;
   if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
-  if ((nl + nh + 2 * nf) * sizeof(Fx) > freeb / 4) return SSE_OK;
+  if ((nl + nh + 2 * nf) * sizeof(Fx) > freeb / 4 || fx_geometry_smem(ka) > (size_t)220 * 1024) return SSE_OK;
   void *lam, *hnq, *hnf, *bn, *n, *eG;
   if ((e = alloc(s, nl * sizeof(Fx), &lam)) || (e = alloc(s, nh * sizeof(Fx), &hnq)) ||
       (e = alloc(s, nf * sizeof(Fx), &hnf)) || (e = alloc(s, nf * sizeof(Fx), &bn)) ||

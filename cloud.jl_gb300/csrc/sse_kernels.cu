@@ -1194,104 +1194,135 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
 // pair's |G|_1 2^k (no flux overflows) and keeps the scaled Lambda_q and
 // halfnJ at most 1/2; 2^-n_i bounds the sum of |G|_1 over the pairs of node i
 // in that unit (no sum of fluxes overflows).
+//
+// The norms only have to be bounds, so they are formed in FP32 from Lambda_q
+// and halfnJ scaled below 1, with their rounding added: a term is a sum of at
+// most 18 products below 2 with relative errors of a few 2^-24, 2^-16 in all.
+// n_i is at most the smallest k of the row, so the margin can shorten it only
+// where a row's norm is within 2^-10 of a power of two.  One walk over the
+// lists, operands in shared memory: creating the handle of 24,576 tets p = 4
+// takes 25.0 ms; 36.0 ms with FP64 norms from global memory, walked twice, of
+// which this kernel was 13.0 ms.
+constexpr float kFxNormError = 1.0f / 65536.0f;
+
 template <int D>
-__global__ void __launch_bounds__(128) fx_geometry_kernel(FxArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
+__global__ void __launch_bounds__(256) fx_geometry_kernel(FxArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
                                                           signed char *on, int *oeG) {
-  __shared__ double sh[3][128];
+  extern __shared__ double smem[];
+  __shared__ double sh[2][8];
   const DevOps &op = ka.op;
   const FxTables &fx = ka.fx;
-  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf > 0 ? op.npf : 1;
+  const int nq = op.nq, nf = op.nf, nfac = op.nfac, npf = op.npf > 0 ? op.npf : 1, rows = nq + nf;
+  const int nl = nq * D * D, nh = D * nfac * nq, nhf = D * nf;
+  double *row = smem;                             // norm of each row
+  float *fLam = reinterpret_cast<float *>(row + rows), *fhq = fLam + nl, *fhf = fhq + nh;
+  int *kmin = reinterpret_cast<int *>(fhf + nhf);
   const size_t k = blockIdx.x;
-  const double *Lam = ka.geo.Lambda_q + k * nq * D * D, *hnq = ka.geo.halfnJq + k * D * nfac * nq,
-               *hnf = ka.geo.halfnJf + k * D * nf, *BJf = ka.geo.BJf + k * nf, *n_f = ka.geo.n_f + k * D * nf;
-  const int lane = threadIdx.x;
-  double gmax = 0.0, lmax = 0.0, hmax = 0.0;
-  // |G|_1 of a pair; gmax: the largest with the pair's factor 2^k (NaN kept)
-  auto larger = [&](double v) { gmax = v > gmax || !(v >= 0.0) ? v : gmax; };
-  auto volume_norm = [&](int inc) {
-    const int p = inc >> 8, a = fx.vp_ij[p] & 0xffff, b = fx.vp_ij[p] >> 16, kp = inc >> 1 & 127;
-    double s = 0.0;
-    for (int n = 0; n < D; ++n) {
-      double g = 0.0;
-      for (int m = 0; m < D; ++m)
-        g = fma(fx_to_unit_double(fx.vp_S[(size_t)p * D + m]), Lam[a + nq * (m + D * n)] + Lam[b + nq * (m + D * n)], g);
-      s += fabs(g);
+  const double *Lam = ka.geo.Lambda_q + k * nl, *hnq = ka.geo.halfnJq + k * nh, *hnf = ka.geo.halfnJf + k * nhf,
+               *BJf = ka.geo.BJf + k * nf, *n_f = ka.geo.n_f + k * nhf;
+  const int lane = threadIdx.x, warps = blockDim.x / 32;
+  auto larger = [](double a, double v) { return v > a || !(v >= 0.0) ? v : a; };  // NaN kept
+  auto block_max = [&](double &x, double &y) {
+    for (int o = 16; o; o >>= 1) {
+      x = larger(x, __shfl_xor_sync(0xffffffffu, x, o));
+      y = larger(y, __shfl_xor_sync(0xffffffffu, y, o));
     }
-    s *= fx_pow2(fx.eS);
-    larger(s);
-    return s * fx_pow2(-kp);
+    __syncthreads();
+    if (lane % 32 == 0) { sh[0][lane / 32] = x; sh[1][lane / 32] = y; }
+    __syncthreads();
+    for (int w = 0; w < warps; ++w) { x = larger(x, sh[0][w]); y = larger(y, sh[1][w]); }
   };
-  auto facet_norm = [&](int inc) {
-    const int p = inc >> 8, i = op.fp_ij[p] & 0xffff, j = op.fp_ij[p] >> 16, f = j / npf, kp = inc >> 1 & 127;
+  double lmax = 0.0, hmax = 0.0;
+  for (int t = lane; t < nl; t += blockDim.x) lmax = larger(lmax, fabs(Lam[t]));
+  for (int t = lane; t < nh; t += blockDim.x) hmax = larger(hmax, fabs(hnq[t]));
+  for (int t = lane; t < nhf; t += blockDim.x) hmax = larger(hmax, fabs(hnf[t]));
+  block_max(lmax, hmax);
+  bool bad = !(lmax < 1e60) || !(hmax < 1e60);
+  auto ex = [](double x) { return fx_exponent((unsigned)__double2hiint(x)); };
+  const int eL = ex(fmax(lmax, 1e-60)), eH = ex(fmax(hmax, 1e-60));
+  if (bad) {
+    if (lane == 0) oeG[k] = kFxNone;
+    return;
+  }
+  const double sL = fx_pow2(-eL), sH = fx_pow2(-eH);
+  for (int t = lane; t < nl; t += blockDim.x) fLam[t] = (float)(Lam[t] * sL);
+  for (int t = lane; t < nh; t += blockDim.x) fhq[t] = (float)(hnq[t] * sH);
+  for (int t = lane; t < nhf; t += blockDim.x) fhf[t] = (float)(hnf[t] * sH);
+  __syncthreads();
+  const double uL = fx_pow2(eL + fx.eS), uH = fx_pow2(eH + fx.eC);  // units of the norms
+  auto unit_float = [](const Fx &v) { return (float)v.hi * (1.0f / 1073741824.0f); };
+  double gmax = 0.0, gtrue = 0.0;  // the largest |G|_1 2^k, bounded and as formed
+  for (int t = lane; t < rows; t += blockDim.x) {
+    float vol = 0.0f, fac = 0.0f, most = 0.0f, fmost = 0.0f;
     double s = 0.0;
-    for (int m = 0; m < D; ++m) s += fabs(fx_to_unit_double(fx.fp_C[p]) * (hnf[m + D * j] + hnq[m + D * (f + nfac * i)]));
-    s *= fx_pow2(fx.eC);
-    larger(s);
-    return s * fx_pow2(-kp);
-  };
-  // the sum over the pairs of node t; and the smallest k among them
-  auto row_norm = [&](int t, int *kmin) {
-    double s = 0.0;
-    *kmin = kFxMaxK;
+    int least = kFxMaxK;
+    auto up = [](float a, float v) { return v > a || !(v >= 0.0f) ? v : a; };
     if (t < nq) {
       for (int q = fx.vol.first[t]; q < fx.vol.first[t + 1]; ++q) {
-        s += volume_norm(fx.vol.inc[q]);
-        *kmin = min(*kmin, fx.vol.inc[q] >> 1 & 127);
+        const int inc = fx.vol.inc[q], p = inc >> 8, a = fx.vp_ij[p] & 0xffff, b = fx.vp_ij[p] >> 16, kp = inc >> 1 & 127;
+        float S[D], v = 0.0f;
+        for (int m = 0; m < D; ++m) S[m] = unit_float(fx.vp_S[(size_t)p * D + m]);
+        for (int n = 0; n < D; ++n) {
+          float g = 0.0f;
+          for (int m = 0; m < D; ++m) g = fmaf(S[m], fLam[a + nq * (m + D * n)] + fLam[b + nq * (m + D * n)], g);
+          v += fabsf(g);
+        }
+        most = up(most, v);
+        vol = fmaf(v + kFxNormError, __int_as_float((127 - kp) << 23), vol);
+        least = min(least, kp);
       }
     } else {
-      double b = 0.0;
-      for (int m = 0; m < D; ++m) b += fabs(0.5 * BJf[t - nq] * n_f[m + D * (t - nq)]);
-      larger(b);
-      s += b;
+      for (int m = 0; m < D; ++m) s += fabs(0.5 * BJf[t - nq] * n_f[m + D * (t - nq)]);
+      gmax = larger(gmax, s);
+      gtrue = larger(gtrue, s);
     }
     for (int q = fx.fac.first[t]; q < fx.fac.first[t + 1]; ++q) {
-      s += facet_norm(fx.fac.inc[q]);
-      *kmin = min(*kmin, fx.fac.inc[q] >> 1 & 127);
+      const int inc = fx.fac.inc[q], p = inc >> 8, i = op.fp_ij[p] & 0xffff, j = op.fp_ij[p] >> 16, f = j / npf,
+                kp = inc >> 1 & 127;
+      const float C = unit_float(fx.fp_C[p]);
+      float v = 0.0f;
+      for (int m = 0; m < D; ++m) v += fabsf(C * (fhf[m + D * j] + fhq[m + D * (f + nfac * i)]));
+      fmost = up(fmost, v);
+      fac = fmaf(v + kFxNormError, __int_as_float((127 - kp) << 23), fac);
+      least = min(least, kp);
     }
-    return s;
-  };
-  int kmin;
-  for (int t = lane; t < nq + nf; t += blockDim.x) row_norm(t, &kmin);
-  for (int t = lane; t < nq * D * D; t += blockDim.x) lmax = fmax(lmax, fabs(Lam[t]));
-  for (int t = lane; t < D * nfac * nq; t += blockDim.x) hmax = fmax(hmax, fabs(hnq[t]));
-  for (int t = lane; t < D * nf; t += blockDim.x) hmax = fmax(hmax, fabs(hnf[t]));
-  sh[0][lane] = gmax;
-  sh[1][lane] = lmax;
-  sh[2][lane] = hmax;
-  __syncthreads();
-  bool bad = false;
-  for (int t = 0; t < (int)blockDim.x; ++t) {
-    const double r = sh[0][t];
-    bad = bad || !(r >= 0.0 && r < 1e60);
-    gmax = fmax(gmax, r);
-    lmax = fmax(lmax, sh[1][t]);
-    hmax = fmax(hmax, sh[2][t]);
+    gtrue = larger(gtrue, (double)most * uL);
+    gtrue = larger(gtrue, (double)fmost * uH);
+    if (most > 0.0f) gmax = larger(gmax, ((double)most + kFxNormError) * uL);
+    if (fmost > 0.0f) gmax = larger(gmax, ((double)fmost + kFxNormError) * uH);
+    // (at most 2^12 entries: their sum is within 2^-12)
+    row[t] = s + ((double)vol * uL + (double)fac * uH) * (1.0 + 1.0 / 2048);
+    kmin[t] = least;
   }
-  bad = bad || !(gmax > 1e-60) || !(lmax < 1e60) || !(hmax < 1e60);
-  auto ex = [](double x) { return fx_exponent((unsigned)__double2hiint(x)); };
+  block_max(gmax, gtrue);
+  bad = !(gtrue > 1e-60 && gtrue < 1e60);
   int eG = ex(gmax * (1.0 + 1e-10));
-  eG = max(eG, ex(fmax(lmax, 1e-60)) + 1 + fx.eS);
-  if (op.nfp > 0) eG = max(eG, ex(fmax(hmax, 1e-60)) + 1 + fx.eC);
+  eG = max(eG, eL + 1 + fx.eS);
+  if (op.nfp > 0) eG = max(eG, eH + 1 + fx.eC);
   if (lane == 0) oeG[k] = bad ? kFxNone : eG;
   if (bad) return;
-  for (int t = lane; t < nq * D * D; t += blockDim.x)
-    oLam[k * nq * D * D + t] = fx_split_near(fx_from_double(Lam[t], eG - fx.eS));
-  for (int t = lane; t < D * nfac * nq; t += blockDim.x) {
+  for (int t = lane; t < nl; t += blockDim.x) oLam[k * nl + t] = fx_split_near(fx_from_double(Lam[t], eG - fx.eS));
+  for (int t = lane; t < nh; t += blockDim.x) {
     const int i = t % nq, fm = t / nq, f = fm / D, m = fm - f * D;
-    ohnq[k * D * nfac * nq + t] = fx_split_near(fx_from_double(hnq[m + D * (f + nfac * i)], eG - fx.eC));
+    ohnq[k * nh + t] = fx_split_near(fx_from_double(hnq[m + D * (f + nfac * i)], eG - fx.eC));
   }
-  for (int t = lane; t < D * nf; t += blockDim.x)
-    ohnf[k * D * nf + t] = fx_split_near(fx_from_double(hnf[t], eG - fx.eC));
-  for (int t = lane; t < nq + nf; t += blockDim.x) {
-    const double s = row_norm(t, &kmin) * (1.0 + 1e-10);
-    const int n = min(kmin, max(-kFxMaxK, s > 1e-60 ? eG - ex(s) : kFxMaxK));
-    on[k * (nq + nf) + t] = (signed char)n;
+  for (int t = lane; t < nhf; t += blockDim.x) ohnf[k * nhf + t] = fx_split_near(fx_from_double(hnf[t], eG - fx.eC));
+  for (int t = lane; t < rows; t += blockDim.x) {
+    const double s = row[t];
+    const int n = min(kmin[t], max(-kFxMaxK, s > 1e-60 ? eG - ex(s) : kFxMaxK));
+    on[k * rows + t] = (signed char)n;
     if (t >= nq)
       for (int m = 0; m < D; ++m) {
         const int o = m + D * (t - nq);
-        obn[k * D * nf + o] = fx_split_near(fx_from_double(0.5 * BJf[t - nq] * n_f[o], eG - n));
+        obn[k * nhf + o] = fx_split_near(fx_from_double(0.5 * BJf[t - nq] * n_f[o], eG - n));
       }
   }
+}
+
+size_t fx_geometry_smem(const FxArgs &ka) {
+  const int d = ka.op.d, rows = ka.op.nq + ka.op.nf;
+  return (size_t)rows * (sizeof(double) + sizeof(int)) +
+         sizeof(float) * (size_t)d * (ka.op.nq * d + ka.op.nfac * ka.op.nq + ka.op.nf);
 }
 
 // ---------------------------------------------------------------------------
@@ -2461,8 +2492,12 @@ cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st) {
 
 cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st) {
-  if (ka.op.d == 2) fx_geometry_kernel<2><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
-  else fx_geometry_kernel<3><<<ka.ne, 128, 0, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
+  const size_t sm = fx_geometry_smem(ka);
+  const int tpb = std::min(256, (ka.op.nq + ka.op.nf + 31) / 32 * 32);
+  auto *kernel = ka.op.d == 2 ? fx_geometry_kernel<2> : fx_geometry_kernel<3>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  kernel<<<ka.ne, tpb, sm, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
   return cudaGetLastError();
 }
 

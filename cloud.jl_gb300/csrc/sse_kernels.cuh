@@ -228,6 +228,7 @@ cudaError_t launch_projection_of_one(const KernelArgs &ka, double *P1, double *R
 cudaError_t sse_set_smem_limits_mixed_a(const KernelArgs &ka);
 cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st);
 // the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG)
+size_t fx_geometry_smem(const FxArgs &ka);
 cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st);
 // the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW)
