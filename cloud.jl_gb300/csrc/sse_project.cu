@@ -13,201 +13,145 @@
 
 #include "../../include/sse_gb300.h"
 #include "sse_kernels.cuh"
-#include "sse_fixed_ops.cuh"
 
 namespace sse {
 namespace {
 
 struct ProjArgs {
   int np, nq, nc;
+  int64_t ne;
+  int epb;           // elements per block
+  int chunk;         // nodes staged at a time
+  const int *tri;    // r << 16 | c of the lower triangle's entries, rows in order
   const double *V, *W, *J, *uq;
-  Fx *Vf;  // V row i times 2^k_i times 2^-eV (at most 1/2), node-major; k_i <= 0
-  int *k;  // about the square root of the node's weight
-  int *eV;
   double *u0;
   int *flag;  // set when a mass matrix is not positive definite
 };
 
-// Vf, k and eV from V, by one block
-__global__ void __launch_bounds__(256) fix_vandermonde_kernel(ProjArgs a) {
-  __shared__ unsigned least, top;
-  const int np = a.np, nq = a.nq;
-  if (threadIdx.x == 0) {
-    least = 0x7ff00000u;
-    top = 0u;
-  }
-  __syncthreads();
-  // node i: its largest entry, brought down to the smallest such
-  auto largest = [&](int i) {
-    unsigned m = 0u;
-    for (int r = 0; r < np; ++r) m = max(m, (unsigned)__double2hiint(a.V[i + (size_t)nq * r]) & 0x7fffffffu);
-    return m;
-  };
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) atomicMin(&least, largest(i));
-  __syncthreads();
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) {
-    const unsigned m = largest(i);
-    const int k = max(-200, fx_exponent(least) - fx_exponent(m));
-    a.k[i] = k;
-    atomicMax(&top, m + ((unsigned)k << 20));
-  }
-  __syncthreads();
-  const int e = top >= 0x7ff00000u ? kFxBad : min(300, max(-300, fx_exponent(top) + 1));
-  if (threadIdx.x == 0) *a.eV = e;
-  for (int t = threadIdx.x; t < nq * np; t += blockDim.x) {
-    const int i = t / np, r = t - i * np;
-    a.Vf[t] = fo_from_double(a.V[i + (size_t)nq * r], e - a.k[i]);
-  }
-}
+constexpr int kThreads = 256;
 
-// 1/sqrt(x) for positive normal x: the hardware approximation (relative error
-// about 2^-22) and one third-order step y <- y (1 + e/2 + 3 e^2/8), e = 1 - x y^2
-__device__ __forceinline__ double rsqrt_step(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
-constexpr int kTile = 3;  // rows and columns of M a thread forms
-
-// Shared memory: WJ[nq], U[nc][nq], M[np][np] (lower triangle, overwritten by the
-// Cholesky factor), Y[nc][np], the factor's inverse diagonal [np].
+// Shared memory: of each element WJ[nq], U[nc][nq] (then W J u), M[np][np] (lower
+// triangle, overwritten by the Cholesky factor) and Y[nc][np]; then, STAGED,
+// chunk nodes of VDM and, of each element, of W J VDM, node-major.
 //
-// M = VDM' diag(W J) VDM is most of the work (630 sums of 125 terms at p = 4,
-// against 7 K FMAs of the factorisation).  In FP64 with an entry a thread it was
-// bound by the FP64 pipe, and the factorisation by one lane's chains of FMAs.  M
-// and the right-hand sides are formed in block fixed point (sse_fixed_ops.cuh)
-// with the rows of VDM scaled by 2^k_i, M in 3 x 3 entries a thread, the cross
-// products carried every four terms; the factorisation and the solves update
-// all remaining entries after each column.  10,368 p = 4 tets, the whole call: 5.79 -> 2.51 ms.
-__global__ void __launch_bounds__(128) project_function_kernel(ProjArgs a) {
+// Bound by the FP64 pipe (a warp instruction takes it for 16 cycles however few
+// lanes are live): the mass matrix is 630 sums of 125 terms at p = 4.  So the
+// products W J VDM are formed once a chunk rather than once a term, and the
+// factorisation updates all remaining entries after each column, with the
+// elements of a block sharing the warps of the square roots, divisions and
+// solves.  Each entry's sum keeps its order, so the results do not change.
+// 10,368 p = 4 tets, the whole call: 5.79 ms with a product a term, one element
+// a block and the factorisation by dot products; 3.20 ms.
+template <bool STAGED>
+__global__ void __launch_bounds__(kThreads) project_function_kernel(ProjArgs a) {
   extern __shared__ double sm[];
-  __shared__ unsigned key[2];
   __shared__ int bad;
-  const int64_t k = blockIdx.x;
-  const int np = a.np, nq = a.nq, nc = a.nc, eV = *a.eV;
-  double *WJ = sm, *U = WJ + nq, *M = U + (size_t)nc * nq, *Y = M + (size_t)np * np, *inv = Y + (size_t)nc * np;
-  Fx *wf = reinterpret_cast<Fx *>(WJ), *Uf = reinterpret_cast<Fx *>(U);
-  if (threadIdx.x == 0) {
-    bad = 0;
-    key[0] = key[1] = 0u;
+  const int np = a.np, nq = a.nq, nc = a.nc;
+  const int64_t k0 = (int64_t)blockIdx.x * a.epb;
+  const int live = (int)(a.ne - k0 < a.epb ? a.ne - k0 : a.epb);
+  const int per = nq + nc * nq + np * np + nc * np;  // doubles an element
+  const int oU = nq, oM = oU + nc * nq, oY = oM + np * np;
+  double *Vc = sm + (size_t)a.epb * per, *VWc = Vc + a.chunk * np;
+  if (threadIdx.x == 0) bad = 0;
+  for (int t = threadIdx.x; t < live * nq; t += kThreads) {
+    const int el = t / nq, i = t - el * nq;
+    double *E = sm + (size_t)el * per;
+    const double w = a.W[i] * a.J[(size_t)nq * k0 + t];
+    E[i] = w;
+    // lmul!(WJ, u_q): U <- WJ .* U
+    for (int e = 0; e < nc; ++e) E[oU + e * nq + i] = a.uq[((size_t)nc * (k0 + el) + e) * nq + i] * w;
   }
-  __syncthreads();
-  // W J 2^-2k and W J u_q 2^-k, in units small enough for sums of nq terms
-  unsigned m0 = 0u, m1 = 0u;
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) {
-    const double w = a.W[i] * a.J[(size_t)nq * k + i], up = fx_pow2(-a.k[i]);
-    WJ[i] = w * up * up;
-    m0 = max(m0, (unsigned)__double2hiint(WJ[i]) & 0x7fffffffu);
-    for (int e = 0; e < nc; ++e) {
-      const double u = a.uq[((size_t)nc * k + e) * nq + i] * w * up;
-      U[e * nq + i] = u;
-      m1 = max(m1, (unsigned)__double2hiint(u) & 0x7fffffffu);
-    }
-  }
-  fx_team_max(key, m0, threadIdx.x, blockDim.x);
-  fx_team_max(key + 1, m1, threadIdx.x, blockDim.x);
-  __syncthreads();
-  const int spare = 32 - __clz(nq);
-  auto unit_of = [&](unsigned m) { return m >= (1023u + 900u) << 20 ? kFxBad : max(-700, fx_exponent(m)) + spare; };
-  const int uW = unit_of(key[0]), uU = unit_of(key[1]);
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) {
-    wf[i] = fo_from_double(WJ[i], uW);
-    for (int e = 0; e < nc; ++e) Uf[e * nq + i] = fo_from_double(U[e * nq + i], uU);
-  }
-  __syncthreads();
-  // M[r][c] (r >= c) = sum_i (VDM[i, r] W J) VDM[i, c]
-  const int nt = (np + kTile - 1) / kTile, ntri = nt * (nt + 1) / 2;
-  for (int t = threadIdx.x; t < ntri; t += blockDim.x) {
-    // t -> (tr, tc) with tc <= tr, rows in order
-    int tr = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
-    while (tr * (tr + 1) / 2 > t) --tr;
-    while ((tr + 1) * (tr + 2) / 2 <= t) ++tr;
-    const int r0 = tr * kTile, c0 = (t - tr * (tr + 1) / 2) * kTile;
-    int rr[kTile], cc[kTile];
-#pragma unroll
-    for (int q = 0; q < kTile; ++q) {
-      rr[q] = min(r0 + q, np - 1);
-      cc[q] = min(c0 + q, np - 1);
-    }
-    FxSums<kTile> s[kTile];
-#pragma unroll 2
-    for (int i = 0; i < nq; ++i) {
-      const Fx w = wf[i];
-      Fx v[kTile];
-#pragma unroll
-      for (int q = 0; q < kTile; ++q) v[q] = a.Vf[i * np + cc[q]];
-#pragma unroll
-      for (int p = 0; p < kTile; ++p) {
-        FxSums<1> wv;
-        wv.add(a.Vf[i * np + rr[p]], &w, 0);
-        s[p].add(fo_split(wv.template value<0>(0)), v, 1);
+  const int ntri = np * (np + 1) / 2, tasks = ntri + nc * np;
+  for (int i0 = 0; i0 < nq; i0 += a.chunk) {
+    const int n = min(a.chunk, nq - i0);
+    __syncthreads();
+    if constexpr (STAGED) {
+      for (int t = threadIdx.x; t < n * np; t += kThreads) {
+        const int r = t / n, i = t - r * n;
+        const double v = a.V[i0 + i + (size_t)nq * r];
+        Vc[i * np + r] = v;
+        for (int el = 0; el < live; ++el) VWc[(el * a.chunk + i) * np + r] = v * sm[(size_t)el * per + i0 + i];
       }
-      if ((i & 3) == 3)
-#pragma unroll
-        for (int p = 0; p < kTile; ++p) s[p].fold();
+      __syncthreads();
     }
-#pragma unroll
-    for (int p = 0; p < kTile; ++p)
-#pragma unroll
-      for (int q = 0; q < kTile; ++q)
-        if (r0 + p < np && c0 + q <= r0 + p)
-          M[(r0 + p) * np + c0 + q] = fx_value(s[p].template value<0>(q), max(uW, eV) == kFxBad ? kFxBad : uW + 2 * eV);
-  }
-  // right-hand sides Y[e][r] = sum_i VDM[i, r] (WJ u_q)[e][i]
-  for (int t = threadIdx.x; t < nc * np; t += blockDim.x) {
-    const int e = t / np, r = t - e * np;
-    FxSums<1> s;
+    // M[r][c] (r >= c) = sum_i VDM[i, r] WJ[i] VDM[i, c] and
+    // Y[e][r] = sum_i VDM[i, r] (WJ u_q)[e][i]
+    for (int t = threadIdx.x; t < live * tasks; t += kThreads) {
+      const int el = t / tasks, q = t - el * tasks;
+      double *E = sm + (size_t)el * per;
+      if (q < ntri) {
+        const int rc = __ldg(a.tri + q), r = rc >> 16, c = rc & 0xffff;
+        double acc = i0 ? E[oM + r * np + c] : 0.0;
+        if constexpr (STAGED) {
+          const double *x = VWc + el * a.chunk * np + r, *y = Vc + c;
 #pragma unroll 4
-    for (int i = 0; i < nq; ++i) {
-      s.add(a.Vf[i * np + r], Uf + e * nq + i, 0);
-      if ((i & 3) == 3) s.fold();
+          for (int i = 0; i < n; ++i) acc = fma(x[i * np], y[i * np], acc);
+        } else {
+          const double *vr = a.V + i0 + (size_t)nq * r, *vc = a.V + i0 + (size_t)nq * c;
+          for (int i = 0; i < n; ++i) acc = fma(__ldg(vr + i) * E[i0 + i], __ldg(vc + i), acc);
+        }
+        E[oM + r * np + c] = acc;
+      } else {
+        const int e = (q - ntri) / np, r = q - ntri - e * np;
+        const double *u = E + oU + e * nq + i0;
+        double acc = i0 ? E[oY + e * np + r] : 0.0;
+        for (int i = 0; i < n; ++i)
+          acc = fma(STAGED ? Vc[i * np + r] : __ldg(a.V + i0 + i + (size_t)nq * r), u[i], acc);
+        E[oY + e * np + r] = acc;
+      }
     }
-    Y[t] = fx_value(s.template value<0>(0), max(uU, eV) == kFxBad ? kFxBad : uU + eV);
   }
   __syncthreads();
   // Cholesky M = L L' by columns (L overwrites the lower triangle), and L z = y
   // along with it
   for (int j = 0; j < np; ++j) {
-    if (threadIdx.x == 0) {
-      double d = M[j * np + j];
-      if (!(d > 0.0)) {
+    if (threadIdx.x < live) {
+      double *d = sm + (size_t)threadIdx.x * per + oM + j * np + j;
+      double v = *d;
+      if (!(v > 0.0)) {
         bad = 1;
-        d = 1.0;
+        v = 1.0;
       }
-      inv[j] = rsqrt_step(d);
+      *d = sqrt(v);
     }
     __syncthreads();
     const int below = np - 1 - j;
-    const double f = inv[j];
-    for (int t = threadIdx.x; t < below + nc; t += blockDim.x) {
-      double *x = t < below ? M + (j + 1 + t) * np + j : Y + (t - below) * np + j;
-      *x *= f;
+    for (int t = threadIdx.x; t < live * (below + nc); t += kThreads) {
+      const int el = t / (below + nc), q = t - el * (below + nc);
+      double *E = sm + (size_t)el * per;
+      double *x = q < below ? E + oM + (j + 1 + q) * np + j : E + oY + (q - below) * np + j;
+      *x /= E[oM + j * np + j];
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < below * (below + nc); t += blockDim.x) {
-      const int row = t / below, col = t - row * below + j + 1;
-      if (row < nc) {
-        Y[row * np + col] = fma(-M[col * np + j], Y[row * np + j], Y[row * np + col]);
+    const int rest = below * (below + 1) / 2, all = rest + nc * below;
+    for (int t = threadIdx.x; t < live * all; t += kThreads) {
+      const int el = t / all, q = t - el * all;
+      double *M = sm + (size_t)el * per + oM, *Y = M + np * np;
+      if (q < rest) {
+        const int rc = __ldg(a.tri + q), r = (rc >> 16) + j + 1, c = (rc & 0xffff) + j + 1;
+        M[r * np + c] = fma(-M[r * np + j], M[c * np + j], M[r * np + c]);
       } else {
-        const int r = row - nc + j + 1;
-        if (col <= r) M[r * np + col] = fma(-M[r * np + j], M[col * np + j], M[r * np + col]);
+        const int e = (q - rest) / below, r = q - rest - e * below + j + 1;
+        Y[e * np + r] = fma(-M[r * np + j], Y[e * np + j], Y[e * np + r]);
       }
     }
     __syncthreads();
   }
-  // L' x = z
-  for (int r = np - 1; r >= 0; --r) {
-    for (int e = threadIdx.x; e < nc; e += blockDim.x) Y[e * np + r] *= inv[r];
-    __syncthreads();
-    for (int t = threadIdx.x; t < nc * r; t += blockDim.x) {
-      const int e = t / r, q = t - e * r;
-      Y[e * np + q] = fma(-M[r * np + q], Y[e * np + r], Y[e * np + q]);
+  // L' x = z, one right-hand side per thread
+  for (int t = threadIdx.x; t < live * nc; t += kThreads) {
+    const double *M = sm + (size_t)(t / nc) * per + oM;
+    double *y = sm + (size_t)(t / nc) * per + oY + (t % nc) * np;
+    for (int r = np - 1; r >= 0; --r) {
+      double s = y[r];
+      for (int q = r + 1; q < np; ++q) s = fma(-M[q * np + r], y[q], s);
+      y[r] = s / M[r * np + r];
     }
-    __syncthreads();
   }
-  for (int t = threadIdx.x; t < nc * np; t += blockDim.x) a.u0[(size_t)nc * np * k + t] = Y[t];
+  __syncthreads();
+  for (int t = threadIdx.x; t < live * nc * np; t += kThreads) {
+    const int el = t / (nc * np);
+    a.u0[(size_t)nc * np * k0 + t] = sm[(size_t)el * per + oY + t - el * nc * np];
+  }
   if (threadIdx.x == 0 && bad) atomicExch(a.flag, 1);
 }
 
@@ -236,14 +180,23 @@ int project_function_run(int np, int nq, int nc, int64_t ne, const double *V, co
   if (np > nq) return bad("n_p must not exceed n_q");
   if (!V || !W || !J || !uq || !u0) return bad("null array");
   if (memory != SSE_HOST && memory != SSE_DEVICE) return bad("memory must be SSE_HOST or SSE_DEVICE");
-  const size_t smem = ((size_t)nq + (size_t)nc * nq + (size_t)np * np + (size_t)nc * np + np) * sizeof(double);
+  const size_t element = ((size_t)nq + (size_t)nc * nq + (size_t)np * np + (size_t)nc * np) * sizeof(double);
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (smem > (size_t)optin) {
+  const size_t static_bytes = 16;
+  if (element + static_bytes > (size_t)optin) {
     *err = "element too large for one CTA's shared memory";
     return SSE_ERR_UNSUPPORTED;
   }
+  // as many elements a block as leave room for three blocks on an SM; the chunk
+  // shrinks, and at last goes, where one element alone fills shared memory
+  int epb = 4, chunk = 16;
+  auto bytes = [&](int n, int ch) { return n * element + (size_t)(n + 1) * ch * np * sizeof(double); };
+  while (epb > 1 && bytes(epb, chunk) > (size_t)74 * 1024) epb /= 2;
+  while (chunk > 0 && bytes(epb, chunk) + static_bytes > (size_t)optin) --chunk;
+  const bool staged = chunk > 0;
+  const size_t smem = bytes(epb, chunk);
   Buffers buf;
   auto cuda = [&](cudaError_t e, const char *where) {
     *err = std::string(where) + ": " + cudaGetErrorString(e);
@@ -261,12 +214,18 @@ int project_function_run(int np, int nq, int nc, int64_t ne, const double *V, co
   if ((e = cudaMemcpy(p, V, (size_t)nq * np * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy((double *)p + (size_t)nq * np, W, nq * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess)
     return cuda(e, "upload VDM, W");
-  if ((e = buf.alloc((size_t)nq * np * sizeof(Fx) + (nq + 2) * sizeof(int), &p)) != cudaSuccess)
-    return cuda(e, "allocate");
-  a.Vf = (Fx *)p;
-  a.k = (int *)(a.Vf + (size_t)nq * np);
-  a.eV = a.k + nq;
-  a.flag = a.eV + 1;
+  std::vector<int> tri;
+  for (int r = 0; r < np; ++r)
+    for (int c = 0; c <= r; ++c) tri.push_back(r << 16 | c);
+  if ((e = buf.alloc(tri.size() * sizeof(int), &p)) != cudaSuccess) return cuda(e, "allocate");
+  a.tri = (const int *)p;
+  if ((e = cudaMemcpy(p, tri.data(), tri.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
+    return cuda(e, "upload triangle");
+  a.ne = ne;
+  a.epb = epb;
+  a.chunk = staged ? chunk : nq;
+  if ((e = buf.alloc(sizeof(int), &p)) != cudaSuccess) return cuda(e, "allocate");
+  a.flag = (int *)p;
   if ((e = cudaMemset(a.flag, 0, sizeof(int))) != cudaSuccess) return cuda(e, "memset");
   const size_t n_j = (size_t)nq * ne, n_u = (size_t)nq * nc * ne, n_o = (size_t)np * nc * ne;
   if (memory == SSE_DEVICE) {
@@ -283,9 +242,9 @@ int project_function_run(int np, int nq, int nc, int64_t ne, const double *V, co
     a.uq = d + n_j;
     a.u0 = d + n_j + n_u;
   }
-  cudaFuncSetAttribute(project_function_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  fix_vandermonde_kernel<<<1, 256>>>(a);
-  project_function_kernel<<<(unsigned)ne, 128, smem>>>(a);
+  auto *kernel = staged ? project_function_kernel<true> : project_function_kernel<false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<(unsigned)((ne + epb - 1) / epb), kThreads, smem>>>(a);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda(e, "projection kernel launch");
   if ((e = cudaDeviceSynchronize()) != cudaSuccess) return cuda(e, "projection kernel");
   int flag = 0;
