@@ -74,10 +74,10 @@ struct FxSums {
       x[e] &= (1LL << kFoLow) - 1;
     }
   }
-  // the sum, up by UP bits
+  // the sum, up by UP bits, rounded to nearest (FxDot)
   template <int UP>
   __device__ __forceinline__ long long value(int e) const {
-    return (long long)((unsigned long long)h[e] << UP) + (x[e] >> (kFoLow - UP));
+    return (long long)((unsigned long long)h[e] << UP) + ((x[e] + (1LL << (kFoLow - UP - 1))) >> (kFoLow - UP));
   }
   template <int UP>
   __device__ __forceinline__ void store(Fx *v, int stride) const {

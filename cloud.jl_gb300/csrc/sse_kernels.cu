@@ -123,10 +123,11 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
 // were 29 K of its 47 K FP64 instructions per p = 4 tet.  Here they are integer
 // multiply-adds and FP64 is left to the entropy-variable maps, about 19 K.  64
 // registers keep 32 warps on an SM (24 warps 1.63 ms, 40 with spills 1.53).
-// 24,576 p = 4 tets 2.69 -> 1.38 ms, 7,986 p = 5 tets 1.55 -> 0.76 ms, 13,182
-// p = 2 tets 0.383 -> 0.185 ms, 8,192 p = 4 triangles 0.149 -> 0.093 ms.  The
-// residual's error against extended precision falls to 0.4 to 0.8 of that
-// with the FP64 operators (40 modal configurations, p = 2 to 6).
+// 24,576 p = 4 tets 2.69 -> 1.28 ms, 7,986 p = 5 tets 1.55 -> 0.69 ms, 13,182
+// p = 2 tets 0.383 -> 0.170 ms, 8,192 p = 4 triangles 0.149 -> 0.086 ms: now the
+// FP64 pipe is 66 % busy, with the maps.  The residual's error against extended
+// precision falls to 0.4 to 0.8 of that with the FP64 operators (modal tensor-
+// product configurations, p = 2 to 6).
 // ---------------------------------------------------------------------------
 template <int D, int NC, int P1>
 __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_constant__ FxArgs ka) {
@@ -784,15 +785,15 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // the issue slots 10 %).  Here the pairs take none: node values are scaled to
 // integers once per element, the pair passes are integer multiply-adds and
 // FP32, and FP64 is left to the node values, the Lax-Friedrichs term and the
-// tail.  Metric terms are read through L1, which leaves shared memory for
-// three blocks of 256 threads on an SM (80 registers): while one block is in its
-// FP64 part the others keep the integer pipes busy (staged in shared memory,
-// two blocks: 3.58 ms against 2.48).  24,576 p = 4 tets: 8.86 -> 2.42 ms; 7,986
-// p = 5 tets 6.5 -> 1.92 ms; 13,182 p = 2 tets 0.96 -> 0.297 ms; 8,192 p = 4
-// triangles 0.365 -> 0.134 ms.  The tail in fixed point too measured 2.54 ms at
-// p = 4 (more barriers, and no FP64 part left to overlap) and, its inputs being
-// sums of all nodes, less exact; it stays in FP64.  The error against the
-// extended-precision residual is 0.81 to 1.00 of the FP64 passes' own on 60
+// last step of the tail (fx_tail).  Metric terms are read through L1, which
+// leaves shared memory for three blocks of 256 threads on an SM (80 registers):
+// while one block is in its FP64 part the others keep the integer pipes busy
+// (staged in shared memory, two blocks: 3.58 ms against 2.48).  24,576 p = 4
+// tets: 8.86 -> 2.17 ms; 7,986 p = 5 tets 6.5 -> 1.66 ms; 13,182 p = 2 tets 0.96
+// -> 0.276 ms; 8,192 p = 4 triangles 0.365 -> 0.117 ms.  The FP64 pipe is 19 %
+// busy and half the issue slots are taken; the rest is latency (barriers, loads
+// of metric terms).  The error against the extended-precision residual is 0.4
+// to 1.00 of the FP64 passes' own on 61
 // configurations (modal and nodal, p = 2 to 6, both metrics and interface
 // fluxes).
 // ---------------------------------------------------------------------------
@@ -1099,7 +1100,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
       FxDot s[D];
       long long h[D];
 #pragma unroll
-      for (int n = 0; n < D; ++n) { s[n].x = 0; h[n] = 0; }
+      for (int n = 0; n < D; ++n) h[n] = 0;
 #pragma unroll
       for (int m = 0; m < D; ++m) {
         const Fx S = fx.vp_S[(size_t)p * D + m];

@@ -117,3 +117,16 @@ def test_non_physical_states_are_reported(gpu_lib, value, variable):
     with pytest.raises(cases.PKG.SSEError) as err:
         cases.PKG.GB300Solver(host).residual(u)
     assert err.value.code == 4
+
+
+@pytest.mark.parametrize("p", [3, 4])
+def test_errors_have_no_direction(gpu_lib, p):
+    """Products are rounded to nearest, not down: over the elements of a mesh
+    the errors of each variable and mode have a mean within five standard
+    deviations of zero (some 175 means: chance exceeds that once in 10^4)."""
+    host = _host("Tet", p, 3, "ModalTensor")
+    u = S.initialize(_Flow(3, 1.4, 0.1, 0.02), host.sd)
+    u = u + 1e-3 * np.random.default_rng(p).standard_normal(u.shape)
+    d = cases.PKG.GB300Solver(host).residual(u) - ExtendedOracle(host).residual(u)
+    rms = np.sqrt((d * d).mean(axis=0))
+    assert np.all(np.abs(d.mean(axis=0)) <= 5.0 * rms / np.sqrt(len(d)))
