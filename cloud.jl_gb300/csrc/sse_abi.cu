@@ -481,15 +481,15 @@ int setup_fx_mass(sse_solver *s) {
   if (!ka.Ak) return SSE_OK;
   if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
   if (n * sizeof(Fx) > freeb / 4) return SSE_OK;
-  void *A, *eA, *eW;
-  if ((e = alloc(s, n * sizeof(Fx), &A)) || (e = alloc(s, ne * sizeof(int), &eA)) ||
-      (e = alloc(s, ne * sizeof(int), &eW)) ||
-      (e = launch_fx_mass_operators(ka, (Fx *)A, (int *)eA, (int *)eW, s->stream)) ||
-      (e = cudaStreamSynchronize(s->stream)))
+  void *p;
+  if ((e = alloc(s, n * sizeof(Fx) + 2 * ne * sizeof(int), &p))) return cuda_fail(s, e, "fixed-point mass operators");
+  Fx *A = (Fx *)p;
+  int *eA = (int *)(A + n), *eW = eA + ne;
+  if ((e = launch_fx_mass_operators(ka, A, eA, eW, s->stream)) || (e = cudaStreamSynchronize(s->stream)))
     return cuda_fail(s, e, "fixed-point mass operators");
-  ka.fx.A_k = (const Fx *)A;
-  ka.fx.eA = (const int *)eA;
-  ka.fx.eW = (const int *)eW;
+  ka.fx.A_k = A;
+  ka.fx.eA = eA;
+  ka.fx.eW = eW;
   ka.fx.on_a = 1;
   return SSE_OK;
 }
@@ -505,19 +505,20 @@ int setup_fx_geometry(sse_solver *s) {
   cudaError_t e;
   if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
   if ((nl + nh + 2 * nf) * sizeof(Fx) > freeb / 4 || fx_geometry_smem(ka) > (size_t)220 * 1024) return SSE_OK;
-  void *lam, *hnq, *hnf, *bn, *n, *eG;
-  if ((e = alloc(s, nl * sizeof(Fx), &lam)) || (e = alloc(s, nh * sizeof(Fx), &hnq)) ||
-      (e = alloc(s, nf * sizeof(Fx), &hnf)) || (e = alloc(s, nf * sizeof(Fx), &bn)) ||
-      (e = alloc(s, ne * (c.n_q + c.n_f), &n)) || (e = alloc(s, ne * sizeof(int), &eG)) ||
-      (e = launch_fx_geometry(ka, (Fx *)lam, (Fx *)hnq, (Fx *)hnf, (Fx *)bn, (signed char *)n, (int *)eG, s->stream)) ||
-      (e = cudaStreamSynchronize(s->stream)))
+  void *p;
+  if ((e = alloc(s, (nl + nh + 2 * nf) * sizeof(Fx) + ne * sizeof(int) + ne * (c.n_q + c.n_f), &p)))
     return cuda_fail(s, e, "fixed-point metric terms");
-  ka.fx.Lam = (const Fx *)lam;
-  ka.fx.hnq = (const Fx *)hnq;
-  ka.fx.hnf = (const Fx *)hnf;
-  ka.fx.bn = (const Fx *)bn;
-  ka.fx.n = (const signed char *)n;
-  ka.fx.eG = (const int *)eG;
+  Fx *lam = (Fx *)p, *hnq = lam + nl, *hnf = hnq + nh, *bn = hnf + nf;
+  int *eG = (int *)(bn + nf);
+  signed char *n = (signed char *)(eG + ne);
+  if ((e = launch_fx_geometry(ka, lam, hnq, hnf, bn, n, eG, s->stream)) || (e = cudaStreamSynchronize(s->stream)))
+    return cuda_fail(s, e, "fixed-point metric terms");
+  ka.fx.Lam = lam;
+  ka.fx.hnq = hnq;
+  ka.fx.hnf = hnf;
+  ka.fx.bn = bn;
+  ka.fx.n = n;
+  ka.fx.eG = eG;
   ka.fx.on = 1;
   return SSE_OK;
 }
