@@ -86,11 +86,11 @@ WORKLOADS = {
         "l2_policy": "inputs larger than L2: ~4 GB read per stage"},
 }
 
-# DRAM bytes (read + write) per element of one fd_time_derivative_kernel<3,5>
-# / nodal_values_kernel<3,5> launch at p = 4, from ncu captures of the same
-# kernels on the 8^3 x 6 = 3,072-tet case (145.7 MB and 37.9 MB per launch);
+# DRAM bytes (read + write) per element of one fd_time_derivative_fx_kernel<3,5,5>
+# / nodal_values_fx_kernel<3,5,5> launch at p = 4, from ncu captures of the same
+# kernels on the 8^3 x 6 = 3,072-tet case (154.3 MB and 37.9 MB per launch);
 # reads scale with the element count
-TRAFFIC_PER_ELEMENT = {"tgv_p4": {"B": 47_429, "A": 12_341}}
+TRAFFIC_PER_ELEMENT = {"tgv_p4": {"B": 50_235, "A": 12_335}}
 
 
 def env_rank():
@@ -485,6 +485,8 @@ def geometry_workload(pkg, pb, fp64_peak):
             "max_field_rel_err_vs_host": err,
             "roofline": {"kernel": kernel, "bound": "fp64", "achieved": tflops, "peak": fp64_peak,
                          "unit": "TFLOP/s", "frac": tflops / fp64_peak,
+                         "note": "FP64-equivalent: most products of tetrahedra are integer multiply-adds, which the "
+                                 "FP64 peak does not bound" if ra.d == 3 else "FP64",
                          "algorithmic_flops_per_element": flops / sd.N_e}}
 
 
@@ -606,12 +608,20 @@ def main():
     kernel_B = "fd_time_derivative_kernel" if fd else (
         "std_compact_kernel" if one_kernel else "std_time_derivative_kernel")
     traffic = TRAFFIC_PER_ELEMENT.get(args.workload) if not (args.cells or args.p) else None
-    roofline = {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp64_peak,
-                "kernel": kernel_B if dom == "B" else "nodal_values_kernel",
+    # the entropy-conservative Euler pair passes are integer multiply-adds: the
+    # FP64 peak does not bound them, HBM is the only roof left
+    fixed_point = (fd and host.cfg.law == pkg.abi.SSE_EULER and host.cfg.two_point_flux == pkg.abi.SSE_EC_FLUX
+                   and host.cfg.gamma <= 1.7)
+    dom_gbs = dom_bytes / (dom_ms * 1e-3) / 1e9
+    roofline = {"bound": "hbm" if fixed_point else "fp64", "achieved": dom_gbs if fixed_point else achieved,
+                "peak": hbm_peak if fixed_point else fp64_peak, "unit": "GB/s" if fixed_point else "TFLOP/s",
+                "frac": dom_gbs / hbm_peak if fixed_point else achieved / fp64_peak,
+                "kernel": (kernel_B if dom == "B" else "nodal_values_kernel").replace(
+                    "_kernel", "_fx_kernel" if fixed_point else "_kernel"),
+                "fp64_equivalent_tflops": achieved, "fp64_peak_tflops": fp64_peak,
                 "peak_source": "measured live: FP64 FMA-chain microbenchmark on this GPU",
-                "hbm_achieved_gbs": dom_bytes / (dom_ms * 1e-3) / 1e9,
-                "hbm_frac_of_measured": dom_bytes / (dom_ms * 1e-3) / 1e9 / hbm_peak,
+                "hbm_achieved_gbs": dom_gbs,
+                "hbm_frac_of_measured": dom_gbs / hbm_peak,
                 "traffic": traffic[dom] * ne if traffic else None,
                 "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on "
                                    "the 3,072-tet case, scaled by the element count") if traffic
@@ -620,7 +630,8 @@ def main():
                              "rk_stage_update": phases[2]},
                 "algorithmic_flops_per_element": {"nodal_values": work.flops_A,
                                                   "time_derivative": work.flops_B},
-                "whole_stage_frac": (work.flops * ne) / ((phases[0] + phases[1]) * 1e-3) / 1e12 / fp64_peak,
+                "whole_stage_frac": (work.bytes_A + work.bytes_B) * ne / ((phases[0] + phases[1]) * 1e-3) / 1e9 / hbm_peak
+                if fixed_point else (work.flops * ne) / ((phases[0] + phases[1]) * 1e-3) / 1e12 / fp64_peak,
                 "kernel_path": "one kernel per residual and per stage (std_compact_kernel)" if one_kernel
                 else "two phases (nodal values, time derivative)",
                 "fp32_peak_tflops": fp32_peak}

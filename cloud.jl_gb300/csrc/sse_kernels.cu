@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) nodal_values_kernel(KernelArgs ka) {
 // registers keep 32 warps on an SM (24 warps 1.63 ms, 40 with spills 1.53).
 // 24,576 p = 4 tets 2.69 -> 1.28 ms, 7,986 p = 5 tets 1.55 -> 0.69 ms, 13,182
 // p = 2 tets 0.383 -> 0.170 ms, 8,192 p = 4 triangles 0.149 -> 0.086 ms: now the
-// FP64 pipe is 66 % busy, with the maps.  The residual's error against extended
+// FP64 pipe is 65 % busy, with the maps.  The residual's error against extended
 // precision falls to 0.4 to 0.8 of that with the FP64 operators (modal tensor-
 // product configurations, p = 2 to 6).
 // ---------------------------------------------------------------------------
@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // while one block is in its FP64 part the others keep the integer pipes busy
 // (staged in shared memory, two blocks: 3.58 ms against 2.48).  24,576 p = 4
 // tets: 8.86 -> 2.17 ms; 7,986 p = 5 tets 6.5 -> 1.66 ms; 13,182 p = 2 tets 0.96
-// -> 0.276 ms; 8,192 p = 4 triangles 0.365 -> 0.117 ms.  The FP64 pipe is 19 %
+// -> 0.276 ms; 8,192 p = 4 triangles 0.365 -> 0.117 ms.  The FP64 pipe is 18 %
 // busy and half the issue slots are taken; the rest is latency (barriers, loads
 // of metric terms).  The error against the extended-precision residual is 0.4
 // to 1.00 of the FP64 passes' own on 61

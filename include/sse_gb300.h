@@ -145,7 +145,14 @@ int32_t sse_abi_version(void);
  * each element's mass operator V' diag(J^-1 W) V (N_p x N_p doubles per
  * element) when they take at most a quarter of the free device memory; the
  * mass solves are then dense products, otherwise two sum-factorised
- * applications of V.  Replaces Solver(...) + the Threaded/Serial parallelism
+ * applications of V.  For FluxDifferencingForm with the entropy-conservative
+ * Euler flux (1 < gamma <= 1.7) it keeps scaled 64-bit integer copies of the
+ * metric terms and of the mass operators (8 bytes a value, the size of
+ * Lambda_q, halfnJq, twice halfnJf and the mass operators; 36 KB per p = 4 tet),
+ * again each when it takes at most a quarter of the free device memory; without
+ * them the residual runs its FP64 kernels, as it does for a block of elements
+ * whose densities or enthalpies span more than a factor of 16 in an element.
+ * Replaces Solver(...) + the Threaded/Serial parallelism
  * tag (Solvers.jl:287-333, 429-452). */
 int32_t sse_create(const sse_config *cfg, const sse_operators *ops,
                    const sse_geometry *geo, sse_solver **out);

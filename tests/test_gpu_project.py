@@ -68,3 +68,26 @@ def test_sizes_and_units(gpu_lib, pkg, shape, p, scale):
     want = np.linalg.solve(mass, np.einsum("qa,keq->kae", V, uq * WJ[:, None, :])).transpose(0, 2, 1)
     assert np.all(got[0] == 0.0)
     assert np.abs(got - want).max() <= 1.0e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("N_p,N_q,N_c,N_e", [(1, 1, 1, 1), (10, 16, 4, 5), (35, 125, 5, 7), (84, 343, 5, 3), (120, 120, 8, 3),
+                                             (165, 166, 1, 2), (168, 168, 1, 2)])
+def test_partial_blocks_chunks_and_large_elements(gpu_lib, pkg, N_p, N_q, N_c, N_e):
+    """Element counts that do not fill a block, nodes that do not fill a chunk,
+    and elements whose mass matrix leaves shared memory for a part of a chunk or
+    none.  VDM has orthonormal columns and W J lies in [1/2, 3/2], so the mass
+    matrix has a condition of at most 3 and sums of N_q terms stay within
+    1e-12."""
+    rng = np.random.default_rng([N_p, N_q])
+
+    class Approximation:
+        V = np.linalg.qr(rng.standard_normal((N_q, N_p)))[0]
+        W = np.ones(N_q)
+
+    J = rng.uniform(0.5, 1.5, (N_e, N_q))
+    uq = rng.standard_normal((N_e, N_c, N_q))
+    got = pkg.gb300.project_function(Approximation, J, uq)
+    V = Approximation.V
+    mass = np.einsum("qa,kq,qb->kab", V, J, V)
+    want = np.linalg.solve(mass, np.einsum("qa,keq->kae", V, uq * J[:, None, :])).transpose(0, 2, 1)
+    assert np.abs(got - want).max() <= 1.0e-12 * np.abs(want).max()
