@@ -2,9 +2,9 @@
 //
 // project_function (src/Solvers/Solvers.jl:396-418): per element the mass
 // matrix M = VDM' diag(W J) VDM is formed, factorised by Cholesky and solved
-// against VDM' (W J u_q), all in one CTA: the weights, nodal data, mass
-// matrix, factor and right-hand sides live in shared memory; VDM is read
-// through L1/L2 by every CTA.
+// against VDM' (W J u_q), one to four elements in a CTA: the weights, nodal
+// data, mass matrix, factor and right-hand sides live in shared memory; VDM is
+// staged there a chunk of nodes at a time.
 #include <cmath>
 #include <string>
 #include <vector>
