@@ -444,7 +444,7 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
     for (int q = r.ptr[j]; q < r.ptr[j + 1]; ++q) row += std::ldexp(std::fabs(r.val[q]), -K[r.idx[q]]);
     if (!(row < 1e30)) return SSE_OK;
     if (!(row > 1e-30)) continue;
-    eR[j] = (signed char)(std::ilogb(row) + 1);
+    eR[j] = (signed char)fo_row_exponent(row);
     for (int q = r.ptr[j]; q < r.ptr[j + 1]; ++q) R[q] = fo_from_double(std::ldexp(r.val[q], -K[r.idx[q]]), eR[j]);
   }
   const CsrHost rt = csc_to_csr(ops->R, true);
@@ -455,7 +455,7 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
     for (int q = rt.ptr[i]; q < rt.ptr[i + 1]; ++q) row += std::ldexp(std::fabs(rt.val[q]), -K[i]);
     rows = std::max(rows, row);
   }
-  fx.eRt = rows > 1e-30 ? std::ilogb(rows) + 1 : 0;
+  fx.eRt = rows > 1e-30 ? fo_row_exponent(rows) : 0;
   fx.eRmin = *std::min_element(eR.begin(), eR.end());
   if (std::abs(fx.eRt - fx.eRmin) > 25) return SSE_OK;
   for (int i = 0; i < c.n_q; ++i)

@@ -17,6 +17,8 @@
 // hand.
 #pragma once
 
+#include <cmath>
+
 #include "sse_kernels.cuh"
 
 namespace sse {
@@ -48,6 +50,10 @@ __host__ __device__ __forceinline__ Fx fo_split(long long v) {
 __device__ __forceinline__ long long fo_join(Fx a) { return ((long long)a.hi << kFoLow) + a.lo; }
 // x 2^(62 - e)
 __host__ __device__ __forceinline__ Fx fo_from_double(double x, int e) { return fo_split(fx_from_double(x, e - 2)); }
+// Exponent e of an operator row with absolute sum `row` (positive and finite):
+// its entries stay below (1 - 2^-20) 2^e.  An entry of (1 - 2^-32) 2^e or more
+// would round to a high part of 2^31, beyond an int.
+inline int fo_row_exponent(double row) { return std::ilogb(row * (1.0 + 1e-6)) + 1; }
 
 // NC sums of products with one operator entry each
 template <int NC>
