@@ -471,7 +471,9 @@ int setup_fx_operators(sse_solver *s, const sse_operators *ops) {
   return SSE_OK;
 }
 
-// Fixed-point mass operators, by the same rule on memory as the metric terms
+// Fixed-point mass operators, by the same rule on memory as the metric terms.
+// Where an element's operator or weights are not finite or out of range, phase
+// A and the tail stay in FP64, which carries such values to the checks.
 int setup_fx_mass(sse_solver *s) {
   FxArgs &ka = s->ka;
   const sse_config &c = s->cfg;
@@ -482,11 +484,20 @@ int setup_fx_mass(sse_solver *s) {
   if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
   if (n * sizeof(Fx) > freeb / 4) return SSE_OK;
   void *p;
-  if ((e = alloc(s, n * sizeof(Fx) + 2 * ne * sizeof(int), &p))) return cuda_fail(s, e, "fixed-point mass operators");
+  if ((e = alloc(s, n * sizeof(Fx) + (2 * ne + 1) * sizeof(int), &p))) return cuda_fail(s, e, "fixed-point mass operators");
   Fx *A = (Fx *)p;
-  int *eA = (int *)(A + n), *eW = eA + ne;
-  if ((e = launch_fx_mass_operators(ka, A, eA, eW, s->stream)) || (e = cudaStreamSynchronize(s->stream)))
+  int *eA = (int *)(A + n), *eW = eA + ne, *bad = eW + ne;
+  int refused = 0;
+  if ((e = cudaMemsetAsync(bad, 0, sizeof(int), s->stream)) ||
+      (e = launch_fx_mass_operators(ka, A, eA, eW, bad, s->stream)) ||
+      (e = cudaMemcpyAsync(&refused, bad, sizeof(int), cudaMemcpyDeviceToHost, s->stream)) ||
+      (e = cudaStreamSynchronize(s->stream)))
     return cuda_fail(s, e, "fixed-point mass operators");
+  if (refused) {
+    s->allocations.pop_back();
+    cudaFree(p);
+    return SSE_OK;
+  }
   ka.fx.A_k = A;
   ka.fx.eA = eA;
   ka.fx.eW = eW;

@@ -254,11 +254,14 @@ __global__ void __launch_bounds__(256, 4) nodal_values_fx_kernel(const __grid_co
 }
 
 // Fixed-point mass operators of phase A: A_k scaled by 2^-eA so that the
-// absolute sums of its rows are at most 1, and eW with sum_i W J 2^-K_i < 2^eW
+// absolute sums of its rows are at most 1, and eW with sum_i W J 2^-K_i < 2^eW;
+// *bad is set where one of them is not finite or its exponent leaves
+// [-kFxMassExponent, kFxMassExponent]
+constexpr int kFxMassExponent = 400;
 __global__ void __launch_bounds__(128) fx_mass_operator_kernel(const double *__restrict__ Ak, const double *__restrict__ WJ,
                                                                const signed char *__restrict__ K,
                                                                const int *__restrict__ order, int np, int nq, Fx *oA,
-                                                               int *oeA, int *oeW) {
+                                                               int *oeA, int *oeW, int *bad) {
   __shared__ unsigned row;
   __shared__ double part[128];
   const size_t k = blockIdx.x;
@@ -274,12 +277,14 @@ __global__ void __launch_bounds__(128) fx_mass_operator_kernel(const double *__r
     atomicMax(&row, (unsigned)__double2hiint(s * (1.0 + 1e-6)));
   }
   __syncthreads();
-  const int e = min(400, max(-400, fx_exponent(row)));
+  const int e = fx_exponent(row);
   if (threadIdx.x == 0) {
     double s = 0.0;
     for (int t = 0; t < (int)blockDim.x; ++t) s += part[t];
+    const int w = fx_exponent((unsigned)__double2hiint(s * (1.0 + 1e-6)));
     oeA[k] = e;
-    oeW[k] = min(400, max(-400, fx_exponent((unsigned)__double2hiint(s * (1.0 + 1e-6)))));
+    oeW[k] = w;
+    if (abs(e) > kFxMassExponent || abs(w) > kFxMassExponent) *bad = 1;  // (not finite: at least 1025)
   }
   for (int t = threadIdx.x; t < np * np; t += blockDim.x) {
     const int b = t / np;
@@ -2502,8 +2507,8 @@ cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *
   return cudaGetLastError();
 }
 
-cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st) {
-  fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.fx.order, ka.op.np, ka.op.nq, A, eA, eW);
+cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, int *bad, cudaStream_t st) {
+  fx_mass_operator_kernel<<<ka.ne, 128, 0, st>>>(ka.Ak, ka.geo.WJ, ka.fx.K, ka.fx.order, ka.op.np, ka.op.nq, A, eA, eW, bad);
   return cudaGetLastError();
 }
 

@@ -231,8 +231,9 @@ cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st);
 size_t fx_geometry_smem(const FxArgs &ka);
 cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
                                cudaStream_t st);
-// the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW)
-cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, cudaStream_t st);
+// the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW); *bad is set when
+// an element's are not finite or out of range
+cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, int *bad, cudaStream_t st);
 cudaError_t launch_mass_operator(const KernelArgs &ka, double *Ak, cudaStream_t st);
 cudaError_t launch_energy(const KernelArgs &ka, const double *u, const double *dudt, double *partial,
                           cudaStream_t st);

@@ -48,3 +48,29 @@ def test_selection_rows_of_the_facet_interpolation(gpu_lib, shape, p):
     want = ExtendedOracle(host).residual(u)
     e64 = max(rel2(Oracle(host).residual(u), want), rel2(Oracle(host, variant="fma").residual(u), want))
     assert rel2(gpu.residual(u), want) <= 4.0 * e64 + 1.0e-14
+
+
+@pytest.mark.parametrize("field,value", [("JinvW", np.nan), ("JinvW", np.inf), ("WJ", np.nan), ("WJ", np.inf), ("J", 0.0)])
+def test_non_finite_geometry_is_reported(gpu_lib, field, value):
+    """One weight or mass entry of one element that is not finite, or a Jacobian
+    of zero, ends in SSE_ERR_NONPHYSICAL and not in numbers."""
+    host, u = _problem("Tet", 2)
+    if field == "J":
+        host.WJ[-1, 3], host.JinvW[-1, 3] = 0.0, np.inf
+    else:
+        getattr(host, field)[-1, 3] = value
+    with pytest.raises(cases.PKG.SSEError) as err:
+        cases.PKG.GB300Solver(host).residual(u)
+    assert err.value.code == cases.PKG.abi.SSE_ERR_NONPHYSICAL
+
+
+@pytest.mark.parametrize("unit", [1.0e-45, 1.0e45])
+def test_lengths_in_other_units(gpu_lib, unit):
+    """The same mesh with lengths of 1e-45 and 1e45: Jacobians of 1e-135 and 1e135
+    lie beyond the exponents of the scaled mass operators.  The residual is that
+    of unit lengths over the unit, to the parity tolerance of 1e-12."""
+    host, u = _problem("Tet", 2)
+    want = cases.PKG.GB300Solver(host).residual(u) / unit
+    for name, power in (("WJ", 3), ("JinvW", -3), ("BJf", 2), ("Lambda_q", 2), ("halfnJf", 2), ("halfnJq", 2)):
+        getattr(host, name)[...] *= unit ** power
+    assert rel2(cases.PKG.GB300Solver(host).residual(u) * unit, want * unit) <= 1.0e-12
