@@ -18,8 +18,11 @@
 // fixed point (sse_fixed_ops.cuh): in FP64 the curl kernel kept the FP64 pipe
 // 99 % busy.  A matrix is scaled so that its absolute row sums are at most 1, a
 // vector to at most 1/4, and the cross products are carried over every four
-// terms, so that no sum overflows.  Products and metrics at the nodes stay in
-// FP64.  10,368 p = 4 tets, curl form, the whole call: 4.80 -> 1.99 ms.
+// terms, so that no sum overflows.  Every coordinate, derivative, product and
+// metric term has a unit of its own, as the floating-point sums have: on
+// stretched or shifted elements they differ by orders of magnitude.  Products
+// and metrics at the nodes stay in FP64.  10,368 p = 4 tets, curl form, the
+// whole call: 4.80 -> 1.99 ms.
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -70,8 +73,9 @@ __global__ void __launch_bounds__(256) fix_matrices_kernel(FixGroups groups, int
     atomicMax(&row, (unsigned)__double2hiint(s * (1.0 + 1e-6)));
   }
   __syncthreads();
+  // (beyond 2^400, and where not finite, the results are NaN)
   const int e = min(400, max(-400, fx_exponent(row)));
-  if (threadIdx.x == 0) ex[blockIdx.x] = row >= 0x7ff00000u ? kFxBad : e;
+  if (threadIdx.x == 0) ex[blockIdx.x] = fx_exponent(row) > 400 ? kFxBad : e;
   for (int c = 0; c < f.count; ++c)
     for (int t = threadIdx.x; t < f.m * f.n; t += blockDim.x) f.out[c][t] = fo_from_double(f.in[c][t], e);
 }
@@ -81,24 +85,27 @@ __device__ __forceinline__ int vector_unit(unsigned key) {
   return key >= (1023u + 900u) << 20 ? kFxBad : max(-800, fx_exponent(key) + 2);
 }
 
-// x scaled in place to one unit, which is returned; *key: scratch in shared
-// memory, zero on entry.  Synchronises the block.
-__device__ __forceinline__ int fix_vectors(double *x, int count, unsigned *key) {
-  unsigned m = 0u;
-  for (int t = threadIdx.x; t < count; t += blockDim.x) m = max(m, (unsigned)__double2hiint(x[t]) & 0x7fffffffu);
-  fx_team_max(key, m, threadIdx.x, blockDim.x);
+// The nv vectors of n values at x scaled in place, each to a unit of its own
+// (unit, in shared memory), a warp per vector.  The values are complete on
+// entry (for the block); synchronises the block at the end.
+__device__ __forceinline__ void fix_vectors(double *x, int nv, int n, int *unit) {
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x >> 5; v < nv; v += blockDim.x >> 5) {
+    double *xv = x + (size_t)v * n;
+    unsigned m = 0u;
+    for (int t = lane; t < n; t += 32) m = max(m, (unsigned)__double2hiint(xv[t]) & 0x7fffffffu);
+    const int u = vector_unit(__reduce_max_sync(0xffffffffu, m));
+    Fx *f = reinterpret_cast<Fx *>(xv);
+    for (int t = lane; t < n; t += 32) f[t] = fo_from_double(xv[t], u);
+    if (lane == 0) unit[v] = u;
+  }
   __syncthreads();
-  const int unit = vector_unit(*key);
-  Fx *f = reinterpret_cast<Fx *>(x);
-  for (int t = threadIdx.x; t < count; t += blockDim.x) f[t] = fo_from_double(x[t], unit);
-  __syncthreads();
-  return unit;
 }
 
-// Row i of A applied to NV vectors; acc in FP64
+// Row i of A (times 2^-ex) applied to NV vectors in their units; acc in FP64
 template <int NV>
-__device__ __forceinline__ void fix_row(const Fx *__restrict__ A, int m, int n, int i, const Fx *x, int xs, int unit,
-                                        double *acc) {
+__device__ __forceinline__ void fix_row(const Fx *__restrict__ A, int m, int n, int i, const Fx *x, int xs, const int *unit,
+                                        int ex, double *acc) {
   FxSums<NV> s;
   int j = 0;
   for (; j + 4 <= n; j += 4) {
@@ -108,7 +115,7 @@ __device__ __forceinline__ void fix_row(const Fx *__restrict__ A, int m, int n, 
   }
   for (; j < n; ++j) s.add(A[i + (size_t)j * m], x + j, xs);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) acc[v] = fx_value(s.template value<0>(v), unit);
+  for (int v = 0; v < NV; ++v) acc[v] = fx_value(s.template value<0>(v), unit[v] + ex);
 }
 
 template <int NA>
@@ -237,35 +244,33 @@ __device__ __forceinline__ void load_xyz(const MetricArgs &g, int64_t k, int D, 
 template <int D>
 __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   extern __shared__ double sm[];
-  __shared__ unsigned key[3];
+  __shared__ int uX[D], uG[D * D], uJ[1];
   const int64_t k = blockIdx.x;
   double *X = sm;
   double *G = X + D * g.n_map;          // G[(a * D + c)] = D_a x_c
   double *Jq = G + D * D * g.n_map;
   load_xyz(g, k, D, X);
-  if (threadIdx.x < 3) key[threadIdx.x] = 0u;
   __syncthreads();
-  int uG = 0;
   if constexpr (D == 2) {
     matvecs<D, D>(Mats<D>{{g.Dr[0], g.Dr[1]}}, g.n_map, g.n_map, X, g.n_map, G, g.n_map);
     __syncthreads();
   } else {
-    const int uX = fix_vectors(X, D * g.n_map, key);
+    fix_vectors(X, D, g.n_map, uX);
     for (int t = threadIdx.x; t < D * g.n_map; t += blockDim.x) {
       const int a = t / g.n_map, i = t - a * g.n_map;
       double acc[D];
-      fix_row<D>(g.fDr[a], g.n_map, g.n_map, i, reinterpret_cast<const Fx *>(X), g.n_map, uX + g.ex[kExDr], acc);
+      fix_row<D>(g.fDr[a], g.n_map, g.n_map, i, reinterpret_cast<const Fx *>(X), g.n_map, uX, g.ex[kExDr], acc);
 #pragma unroll
       for (int c = 0; c < D; ++c) G[(a * D + c) * g.n_map + i] = acc[c];
     }
     __syncthreads();
-    uG = fix_vectors(G, D * D * g.n_map, key + 1);
+    fix_vectors(G, D * D, g.n_map, uG);
   }
   const Fx *Gf = reinterpret_cast<const Fx *>(G);
   for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
     double acc[D * D];
     if constexpr (D == 2) row_apply<D * D>(g.Vq, g.n_q, g.n_map, i, G, g.n_map, acc);
-    else fix_row<D * D>(g.fVq, g.n_q, g.n_map, i, Gf, g.n_map, uG + g.ex[kExVq], acc);
+    else fix_row<D * D>(g.fVq, g.n_q, g.n_map, i, Gf, g.n_map, uG, g.ex[kExVq], acc);
     double a[D][D], adj[D][D];
 #pragma unroll
     for (int m = 0; m < D; ++m)
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   for (int i = threadIdx.x; i < g.n_f; i += blockDim.x) {
     double acc[D * D];
     if constexpr (D == 2) row_apply<D * D>(g.Vf, g.n_f, g.n_map, i, G, g.n_map, acc);
-    else fix_row<D * D>(g.fVf, g.n_f, g.n_map, i, Gf, g.n_map, uG + g.ex[kExVf], acc);
+    else fix_row<D * D>(g.fVf, g.n_f, g.n_map, i, Gf, g.n_map, uG, g.ex[kExVf], acc);
     double a[D][D], adj[D][D];
 #pragma unroll
     for (int m = 0; m < D; ++m)
@@ -301,12 +306,11 @@ __global__ void __launch_bounds__(128) exact_metrics_kernel(MetricArgs g) {
   }
   if (g.project) {
     __syncthreads();
-    int uJ = 0;
-    if constexpr (D == 3) uJ = fix_vectors(Jq, g.n_q, key + 2);
+    if constexpr (D == 3) fix_vectors(Jq, 1, g.n_q, uJ);
     for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
       double acc[1];
       if constexpr (D == 2) row_apply<1>(g.P, g.n_q, g.n_q, i, Jq, g.n_q, acc);
-      else fix_row<1>(g.fP, g.n_q, g.n_q, i, reinterpret_cast<const Fx *>(Jq), 0, uJ + g.ex[kExP], acc);
+      else fix_row<1>(g.fP, g.n_q, g.n_q, i, reinterpret_cast<const Fx *>(Jq), 0, uJ, g.ex[kExP], acc);
       g.J_q[(size_t)g.n_q * k + i] = acc[0];
     }
   }
@@ -362,7 +366,7 @@ __global__ void __launch_bounds__(128) curl_metrics_2d_kernel(MetricArgs g) {
 // at p = 4, whose 56 nodes of degree 5 set the length of the large steps.
 __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
   extern __shared__ double sm[];
-  __shared__ unsigned key[3];
+  __shared__ int uJ[1], uF[9], uM[9];
   const int64_t k = blockIdx.x;
   const int nm = g.n_map, n1 = g.n1;
   double *X = sm;
@@ -372,7 +376,6 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
   double *G1 = X1 + 3 * n1;   // D1_a x1_c, later the metric terms M[m + 3 n]
   double *F = G1 + 9 * n1;    // F[p * 3 + a]
   load_xyz(g, k, 3, X);
-  if (threadIdx.x < 3) key[threadIdx.x] = 0u;
   __syncthreads();
   matvecs<3, 3>(Mats<3>{{g.Dr[0], g.Dr[1], g.Dr[2]}}, nm, nm, X, nm, G, nm);
   matvecs<1, 3>(Mats<1>{{g.N1}}, n1, nm, X, nm, X1, n1);
@@ -383,11 +386,12 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
     const double xt = G[6 * nm + i], yt = G[7 * nm + i], zt = G[8 * nm + i];
     Jm[i] = xr * (ys * zt - zs * yt) - yr * (xs * zt - zs * xt) + zr * (xs * yt - ys * xt);
   }
-  const int uJ = fix_vectors(Jm, nm, key);
+  __syncthreads();
+  fix_vectors(Jm, 1, nm, uJ);
   matvecs<3, 3>(Mats<3>{{g.D1[0], g.D1[1], g.D1[2]}}, n1, n1, X1, n1, G1, n1);
   for (int i = threadIdx.x; i < g.n_q; i += blockDim.x) {
     double acc[1];
-    fix_row<1>(g.fVq, g.n_q, nm, i, reinterpret_cast<const Fx *>(Jm), 0, uJ + g.ex[kExVq], acc);
+    fix_row<1>(g.fVq, g.n_q, nm, i, reinterpret_cast<const Fx *>(Jm), 0, uJ, g.ex[kExVq], acc);
     g.J_q[(size_t)g.n_q * k + i] = acc[0];
   }
   __syncthreads();
@@ -401,46 +405,54 @@ __global__ void __launch_bounds__(128) curl_metrics_3d_kernel(MetricArgs g) {
       for (int a = 0; a < 3; ++a) F[(p * 3 + a) * n1 + i] = G1[(a * 3 + dc[p]) * n1 + i] * X1[mc[p] * n1 + i];
   }
   __syncthreads();
-  const int uF = fix_vectors(F, 9 * n1, key + 1) + g.ex[kExD1];
+  fix_vectors(F, 9, n1, uF);
   const Fx *Ff = reinterpret_cast<const Fx *>(F);
   for (int t = threadIdx.x; t < 3 * n1; t += blockDim.x) {
-    // of pair p: D_t F_s - D_s F_t, D_r F_t - D_t F_r, D_s F_r - D_r F_s
+    // of pair p: D_t F_s - D_s F_t, D_r F_t - D_t F_r, D_s F_r - D_r F_s, each
+    // product in the unit of its F
     const int p = t / n1, i = t - p * n1;
-    const Fx *f = Ff + 3 * p * n1;
-    FxSums<1> c[3];
-    auto minus = [](Fx a) { return Fx{-a.lo, -a.hi}; };
-#pragma unroll 2
-    for (int j = 0; j < n1; ++j) {
+    const Fx *fr = Ff + 3 * p * n1, *fs = fr + n1, *ft = fs + n1;
+    FxSums<1> c[6];
+    auto add = [&](int j) {
       const size_t o = i + (size_t)j * n1;
-      if ((j & 1) == 0)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) c[q].fold();
       const Fx dr = g.fD1[0][o], ds = g.fD1[1][o], dt = g.fD1[2][o];
-      const Fx *fr = f + j, *fs = f + n1 + j, *ft = f + 2 * n1 + j;
-      c[0].add(dt, fs, 0);
-      c[0].add(minus(ds), ft, 0);
-      c[1].add(dr, ft, 0);
-      c[1].add(minus(dt), fr, 0);
-      c[2].add(ds, fr, 0);
-      c[2].add(minus(dr), fs, 0);
+      c[0].add(dt, fs + j, 0);
+      c[1].add(ds, ft + j, 0);
+      c[2].add(dr, ft + j, 0);
+      c[3].add(dt, fr + j, 0);
+      c[4].add(ds, fr + j, 0);
+      c[5].add(dr, fs + j, 0);
+    };
+    int j = 0;
+    for (; j + 4 <= n1; j += 4) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) add(j + q);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) c[q].fold();
     }
+    for (; j < n1; ++j) add(j);
+    // the difference of two sums in the larger of their units
+    const int u[6] = {uF[3 * p + 1], uF[3 * p + 2], uF[3 * p + 2], uF[3 * p], uF[3 * p], uF[3 * p + 1]};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double v = fx_value(c[q].template value<0>(0), uF);
-      G1[(q + 3 * p) * n1 + i] = p == 0 ? v : -v;
+      const int U = max(u[2 * q], u[2 * q + 1]);
+      const long long v = FxShift(min(62, U - u[2 * q]))(c[2 * q].template value<0>(0)) -
+                          FxShift(min(62, U - u[2 * q + 1]))(c[2 * q + 1].template value<0>(0));
+      const double d = fx_value(v, U, g.ex[kExD1]);
+      G1[(q + 3 * p) * n1 + i] = p == 0 ? d : -d;
     }
   }
   __syncthreads();
-  const int uM = fix_vectors(G1, 9 * n1, key + 2);
+  fix_vectors(G1, 9, n1, uM);
   const Fx *Mf = reinterpret_cast<const Fx *>(G1);
   for (int t = threadIdx.x; t < g.n_q + g.n_f; t += blockDim.x) {
     double L[9];
     if (t < g.n_q) {
-      fix_row<9>(g.fVq1, g.n_q, n1, t, Mf, n1, uM + g.ex[kExVq1], L);
+      fix_row<9>(g.fVq1, g.n_q, n1, t, Mf, n1, uM, g.ex[kExVq1], L);
       store_lambda<3>(g, k, t, L);
       write_nJq<3>(g, k, t, L);
     } else {
-      fix_row<9>(g.fVf1, g.n_f, n1, t - g.n_q, Mf, n1, uM + g.ex[kExVf1], L);
+      fix_row<9>(g.fVf1, g.n_f, n1, t - g.n_q, Mf, n1, uM, g.ex[kExVf1], L);
       write_nJf<3>(g, k, t - g.n_q, L);
     }
   }
