@@ -506,8 +506,9 @@ int setup_fx_mass(sse_solver *s) {
 }
 
 // Fixed-point metric terms, when the kernel that forms them fits in shared
-// memory and they take at most a quarter of the free
-// device memory; without them phase B runs in FP64.
+// memory, they take at most a quarter of the free device memory and at most
+// three quarters of the elements are without (stretched, kFxStretch); else phase
+// B is the FP64 kernel.
 int setup_fx_geometry(sse_solver *s) {
   FxArgs &ka = s->ka;
   const sse_config &c = s->cfg;
@@ -517,13 +518,22 @@ int setup_fx_geometry(sse_solver *s) {
   if ((e = cudaMemGetInfo(&freeb, &totalb))) return cuda_fail(s, e, "cudaMemGetInfo");
   if ((nl + nh + 2 * nf) * sizeof(Fx) > freeb / 4 || fx_geometry_smem(ka) > (size_t)220 * 1024) return SSE_OK;
   void *p;
-  if ((e = alloc(s, (nl + nh + 2 * nf) * sizeof(Fx) + ne * sizeof(int) + ne * (c.n_q + c.n_f), &p)))
+  if ((e = alloc(s, (nl + nh + 2 * nf) * sizeof(Fx) + (ne + 1) * sizeof(int) + ne * (c.n_q + c.n_f), &p)))
     return cuda_fail(s, e, "fixed-point metric terms");
   Fx *lam = (Fx *)p, *hnq = lam + nl, *hnf = hnq + nh, *bn = hnf + nf;
-  int *eG = (int *)(bn + nf);
-  signed char *n = (signed char *)(eG + ne);
-  if ((e = launch_fx_geometry(ka, lam, hnq, hnf, bn, n, eG, s->stream)) || (e = cudaStreamSynchronize(s->stream)))
+  int *eG = (int *)(bn + nf), *none = eG + ne;
+  signed char *n = (signed char *)(none + 1);
+  int without = 0;
+  if ((e = cudaMemsetAsync(none, 0, sizeof(int), s->stream)) ||
+      (e = launch_fx_geometry(ka, lam, hnq, hnf, bn, n, eG, none, s->stream)) ||
+      (e = cudaMemcpyAsync(&without, none, sizeof(int), cudaMemcpyDeviceToHost, s->stream)) ||
+      (e = cudaStreamSynchronize(s->stream)))
     return cuda_fail(s, e, "fixed-point metric terms");
+  if (without > (int)(ne - ne / 4)) {
+    s->allocations.pop_back();
+    cudaFree(p);
+    return SSE_OK;
+  }
   ka.fx.Lam = lam;
   ka.fx.hnq = hnq;
   ka.fx.hnf = hnf;

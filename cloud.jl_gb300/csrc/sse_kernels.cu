@@ -1211,9 +1211,18 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
 // which this kernel was 13.0 ms.
 constexpr float kFxNormError = 1.0f / 65536.0f;
 
+// Stretched elements get no fixed-point terms (kFxNone, counted in *none): the
+// components of a metric vector share a unit of 60 bits, so one 2^-m of the
+// largest keeps 60 - m bits, where FP64 keeps 53, and with it the momentum along
+// the long side.  The limit is on the ratio of the columns of Lambda_q (one per
+// direction) at any node.  Against extended precision, by variable, boxes 1 : 1 :
+// 1/A: A = 4 0.3 to 1.2 of the FP64 error, as at A = 1; A = 16 up to 2.1 (nodal p =
+// 3 tets, EC interface), A = 128 18, A = 1e4 690.
+constexpr double kFxStretch = 8.0;
+
 template <int D>
 __global__ void __launch_bounds__(256) fx_geometry_kernel(FxArgs ka, Fx *oLam, Fx *ohnq, Fx *ohnf, Fx *obn,
-                                                          signed char *on, int *oeG) {
+                                                          signed char *on, int *oeG, int *none) {
   extern __shared__ double smem[];
   __shared__ double sh[2][8];
   const DevOps &op = ka.op;
@@ -1246,8 +1255,25 @@ __global__ void __launch_bounds__(256) fx_geometry_kernel(FxArgs ka, Fx *oLam, F
   bool bad = !(lmax < 1e60) || !(hmax < 1e60);
   auto ex = [](double x) { return fx_exponent((unsigned)__double2hiint(x)); };
   const int eL = ex(fmax(lmax, 1e-60)), eH = ex(fmax(hmax, 1e-60));
+  bool thin = false;
+  for (int t = lane; t < nq; t += blockDim.x) {
+    double least = INFINITY, most = 0.0;
+#pragma unroll
+    for (int n = 0; n < D; ++n) {
+      double column = 0.0;
+#pragma unroll
+      for (int m = 0; m < D; ++m) column = fmax(column, fabs(Lam[t + nq * (m + D * n)]));
+      least = fmin(least, column);
+      most = fmax(most, column);
+    }
+    thin = thin || most > kFxStretch * least;
+  }
+  if (__syncthreads_or(thin)) bad = true;
   if (bad) {
-    if (lane == 0) oeG[k] = kFxNone;
+    if (lane == 0) {
+      oeG[k] = kFxNone;
+      atomicAdd(none, 1);
+    }
     return;
   }
   const double sL = fx_pow2(-eL), sH = fx_pow2(-eH);
@@ -1305,7 +1331,10 @@ __global__ void __launch_bounds__(256) fx_geometry_kernel(FxArgs ka, Fx *oLam, F
   int eG = ex(gmax * (1.0 + 1e-10));
   eG = max(eG, eL + 1 + fx.eS);
   if (op.nfp > 0) eG = max(eG, eH + 1 + fx.eC);
-  if (lane == 0) oeG[k] = bad ? kFxNone : eG;
+  if (lane == 0) {
+    oeG[k] = bad ? kFxNone : eG;
+    if (bad) atomicAdd(none, 1);
+  }
   if (bad) return;
   for (int t = lane; t < nl; t += blockDim.x) oLam[k * nl + t] = fx_split_near(fx_from_double(Lam[t], eG - fx.eS));
   for (int t = lane; t < nh; t += blockDim.x) {
@@ -2497,13 +2526,13 @@ cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st) {
 }
 
 cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
-                               cudaStream_t st) {
+                               int *none, cudaStream_t st) {
   const size_t sm = fx_geometry_smem(ka);
   const int tpb = std::min(256, (ka.op.nq + ka.op.nf + 31) / 32 * 32);
   auto *kernel = ka.op.d == 2 ? fx_geometry_kernel<2> : fx_geometry_kernel<3>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  kernel<<<ka.ne, tpb, sm, st>>>(ka, Lam, hnq, hnf, bn, n, eG);
+  kernel<<<ka.ne, tpb, sm, st>>>(ka, Lam, hnq, hnf, bn, n, eG, none);
   return cudaGetLastError();
 }
 

@@ -227,10 +227,11 @@ cudaError_t launch_nodal_values(const FxArgs &ka, cudaStream_t st);
 cudaError_t launch_projection_of_one(const KernelArgs &ka, double *P1, double *RP1, cudaStream_t st);
 cudaError_t sse_set_smem_limits_mixed_a(const KernelArgs &ka);
 cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st);
-// the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG)
+// the fixed-point metric terms of every element (ka.fx.Lam, hnq, hnf, bn, eG);
+// *none counts the elements without (eG = kFxNone)
 size_t fx_geometry_smem(const FxArgs &ka);
 cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *bn, signed char *n, int *eG,
-                               cudaStream_t st);
+                               int *none, cudaStream_t st);
 // the fixed-point mass operators of phase A (ka.fx.A_k, eA, eW); *bad is set when
 // an element's are not finite or out of range
 cudaError_t launch_fx_mass_operators(const FxArgs &ka, Fx *A, int *eA, int *eW, int *bad, cudaStream_t st);

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import cases
+from oracle.oracle import ExtendedOracle, Oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +72,48 @@ def test_geometric_factors(gpu_lib, pkg, metrics, p, aspect, offset):
         scale = np.abs(w).max()
         err, err64 = [float(np.abs(_component(gf, key) - w).max() / scale) for gf in (got, host)]
         assert err <= 2.0 * err64 + 4.0 * 2.0 ** -52, (key, err, err64)
+
+
+class _Shear:
+    """Smooth density and pressure, every velocity component ``speed[m]`` times a
+    periodic function of two coordinates."""
+
+    def __init__(self, lengths, speed):
+        self.k, self.speed = [2 * np.pi / L for L in lengths], speed
+
+    def evaluate(self, x, t=0.0):
+        k, d = self.k, len(self.k)
+        rho = 1.0 + 0.05 * np.sin(k[0] * x[0] + 0.3) * np.cos(k[-1] * x[-1])
+        p = (1.0 + 0.05 * np.cos(k[-1] * x[-1])) / 1.4
+        v = [self.speed[m] * np.cos(k[m] * x[m] + 0.5 * m) * np.sin(k[(m + 1) % d] * x[(m + 1) % d] + 0.7)
+             for m in range(d)]
+        E = p / 0.4 + 0.5 * rho * sum(w * w for w in v)
+        return np.stack([rho, *[rho * w for w in v], E], axis=-1)
+
+
+def _check_variables(basis, shape, p, lengths, speed, ec):
+    """Every variable of the residual no further from extended precision than
+    four times the FP64 oracle (as the residuals of other flows are held to)."""
+    ra, mesh = _mesh(basis, shape, p, 1 if shape == "Tet" else 2, lengths)
+    sd = M.spatial_discretization(mesh, ra, metrics="ChanWilcox")
+    nflux = S.EntropyConservativeNumericalFlux() if ec else S.LaxFriedrichsNumericalFlux()
+    host = S.HostArrays(S.EulerEquations(len(lengths), 1.4), sd, S.FluxDifferencingForm(inviscid_numerical_flux=nflux))
+    u = S.initialize(_Shear(lengths, speed), sd)
+    got, want = cases.PKG.GB300Solver(host).residual(u), ExtendedOracle(host).residual(u)
+    fp64 = [Oracle(host).residual(u), Oracle(host, variant="fma").residual(u)]
+    for e in range(host.N_c):
+        err, err64 = [max(float(np.linalg.norm(r[:, e] - want[:, e])) for r in rs) for rs in ([got], fp64)]
+        assert err <= 4.0 * err64 + 1.0e-14 * np.linalg.norm(want[:, e]), (e, err / err64)
+
+
+@pytest.mark.parametrize("basis,shape,p", [("ModalTensor", "Tri", 3), ("NodalTensor", "Tri", 4), ("ModalTensor", "Tet", 2),
+                                           ("ModalTensor", "Tet", 4), ("NodalTensor", "Tet", 3)])
+@pytest.mark.parametrize("aspect", [7.0, 9.0, 1.0e2, 1.0e4])
+@pytest.mark.parametrize("along", ["long", "short"])
+@pytest.mark.parametrize("ec", [True, False])
+def test_residual(gpu_lib, basis, shape, p, aspect, along, ec):
+    """Boxes with one short side, on both sides of the fixed-point terms' limit
+    and far beyond it, with flow along the long sides or across them."""
+    d = 2 if shape == "Tri" else 3
+    long, short = (0.3, 0.3 / aspect) if along == "long" else (0.3 / aspect, 0.3)
+    _check_variables(basis, shape, p, (2 * np.pi,) * (d - 1) + (2 * np.pi / aspect,), (long,) * (d - 1) + (short,), ec)
