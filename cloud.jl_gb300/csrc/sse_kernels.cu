@@ -843,11 +843,17 @@ __device__ __forceinline__ void fx_node_sums(const FxTables::Sums &S, int c, con
 // Exponents of an element's units from the extremes of its node values (upper
 // words of the largest density, enthalpy and |velocity component| and
 // 0x7fffffff less that of the smallest density and enthalpy); ok: positive,
-// finite and within a factor 2^4 to 2^5 of each other
+// finite and within a factor 2^4 to 2^5 of each other.
+// Velocities have units of at least 2^-20 of the speed of sound (fx_tail's
+// bounds), so those below 2^-23 of it have fewer bits than in FP64.  A Lax-
+// Friedrichs term (damped) adds 2^-53 of the speed of sound by itself; without
+// one, such elements are not ok unless the fluid is at rest (EC interface, Mach
+// 1e-10, p = 3 tets: density residual off by 130 times the FP64 error; Mach
+// 1e-7: 0.3 to 0.5).
 struct FxScale {
   int eR, eH, eV;
   bool ok;
-  __device__ __forceinline__ FxScale(const unsigned *key, int eG) {
+  __device__ __forceinline__ FxScale(const unsigned *key, int eG, bool damped) {
     ok = key[0] < 0x7ff00000u && key[1] < 0x7ff00000u && key[2] < 0x7ff00000u;
     const int r = fx_exponent(key[0]), h = fx_exponent(key[1]), v = fx_exponent(key[2]);
     ok = ok && r - fx_exponent(0x7fffffffu - key[3]) <= 4 && h - fx_exponent(0x7fffffffu - key[4]) <= 4;
@@ -855,7 +861,9 @@ struct FxScale {
     eR = r + 1;
     eV = v + 1;
     eH = max(h + 1, 2 * eV);
-    eV = max(eV, (eH - 40) >> 1);
+    const int least = (eH - 40) >> 1;
+    ok = ok && (damped || key[2] == 0u || eV + 4 > least);
+    eV = max(eV, least);
   }
 };
 
@@ -1064,7 +1072,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
   fx_team_max(key + 4, k4, lane, tpe);
   __syncthreads();
   const int eG = fx.eG[kk];
-  const FxScale sc(key, eG);
+  const FxScale sc(key, eG, ph.nflux == 0 && ph.half_lambda > 1e-6);
   // a block with an element out of range runs in FP64 as a whole
   if (!__syncthreads_and(sc.ok)) {
     fd_fp64<D, NC>(ka, smem + (size_t)team * ka.layB.team_doubles, kk, live, lane, tpe);

@@ -117,3 +117,12 @@ def test_residual(gpu_lib, basis, shape, p, aspect, along, ec):
     d = 2 if shape == "Tri" else 3
     long, short = (0.3, 0.3 / aspect) if along == "long" else (0.3 / aspect, 0.3)
     _check_variables(basis, shape, p, (2 * np.pi,) * (d - 1) + (2 * np.pi / aspect,), (long,) * (d - 1) + (short,), ec)
+
+
+@pytest.mark.parametrize("basis,shape,p", [("ModalTensor", "Tri", 4), ("NodalTensor", "Tet", 3)])
+@pytest.mark.parametrize("mach", [1.0e-6, 1.0e-7, 1.0e-9, 1.0e-12])
+def test_low_mach_without_dissipation(gpu_lib, basis, shape, p, mach):
+    """Velocities next to and below the smallest fixed-point unit, where no
+    Lax-Friedrichs term hides what they lose."""
+    d = 2 if shape == "Tri" else 3
+    _check_variables(basis, shape, p, (2 * np.pi,) * d, (mach,) * d, True)
