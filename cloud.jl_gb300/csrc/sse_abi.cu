@@ -270,6 +270,7 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return mask[a] > mask[b]; });
   std::vector<int> ij(nvp);
   std::vector<Fx> S((size_t)nvp * d), Cx(C.size());
+  std::vector<double> Sh((size_t)nvp * d);
   lists->vol.assign(nq, {});
   for (int t = 0; t < nvp; ++t) {
     const double *v = &vp_S[(size_t)order[t] * d];
@@ -277,7 +278,10 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
     ij[t] = vp_ij[order[t]];
     lists->vol[ij[t] & 0xffff].push_back(t << 8 | k << 1 | 1);
     lists->vol[ij[t] >> 16].push_back(t << 8 | k << 1);
-    for (int m = 0; m < d; ++m) S[(size_t)t * d + m] = fx_split_near(fx_from_double(0.5 * v[m], fx.eS - k));
+    for (int m = 0; m < d; ++m) {
+      Sh[(size_t)t * d + m] = 0.5 * v[m];
+      S[(size_t)t * d + m] = fx_split_near(fx_from_double(0.5 * v[m], fx.eS - k));
+    }
   }
   std::vector<int> kC(C.size());
   for (size_t t = 0; t < C.size(); ++t) {
@@ -288,7 +292,8 @@ int setup_fx_pairs(sse_solver *s, const std::vector<int> &vp_ij, const std::vect
   for (auto &l : lists->fac)
     for (int &v : l) v = v << 8 | kC[v] << 1;
   cudaError_t e;
-  if ((e = upload(s, ij.data(), ij.size(), &fx.vp_ij)) || (e = upload(s, S.data(), S.size(), &fx.vp_S)) ||
+  if ((e = upload(s, ij.data(), ij.size(), &fx.vp_ij)) || (e = upload(s, Sh.data(), Sh.size(), &fx.vp_Sh)) ||
+      (e = upload(s, S.data(), S.size(), &fx.vp_S)) ||
       (!C.empty() && (e = upload(s, Cx.data(), Cx.size(), &fx.fp_C))))
     return cuda_fail(s, e, "fixed-point pair tables");
   // P1 nodes a direction, P1^(d-1) a face, one face more than directions
@@ -1006,8 +1011,6 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
     for (; i < 12; ++i) L.off[i] = off;
     L.team_doubles = off;
   };
-  Layout fx_layB{};     // FP64 passes inside the fixed-point kernel: layout and chunk
-  int fx_fd_chunk = 0;
   // phase-A layout: X, Y, Z, W, F, lane partials; F holds NC x max(N_p, N_q,
   // N_f) (modal scratch, facet values, or V dudt in the conservation kernel)
   finish(ka.layA, {nc * std::max(np, nq), nc * nq, zsz, wsz, nc * std::max({np, nq, nf}), tpe * (nc + 1)});
@@ -1083,14 +1086,6 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
       layout_x(n);
       // no room for the node values: the FP64 passes
       if ((size_t)epb_x * ka.layBx.team_doubles * 8 > (size_t)220 * 1024) ka.fx = FxTables{};
-      // the FP64 passes of blocks that leave the fixed-point ones fit in the
-      // same shared memory where chunks of at least one pass of the threads do
-      const Layout one = ka.layB;
-      const int room = (ka.layBx.team_doubles - (layout(0) - ((std::max(0, final_scratch) + 1) & ~1)) - 1) / nc;
-      fx_fd_chunk = std::min(chunk, room >= tpe_x ? room / tpe_x * tpe_x : std::min(tpe_x, max_pairs));
-      layout(fx_fd_chunk);
-      fx_layB = ka.layB;
-      ka.layB = one;
     }
     // the interface flux of one facet node costs about 0.8 of a volume pair
     // (block timings at p = 4): balance lanes when all pairs are one chunk.
@@ -1160,8 +1155,6 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   // opt in to large dynamic shared memory for every kernel instantiation used
   size_t smA = (size_t)std::max(epb, ka.epb_a) * ka.layA.team_doubles * 8,
          smB = (size_t)epb * ka.layB.team_doubles * 8;
-  if (ka.fx.vp_ij)
-    smB = std::max(smB, (size_t)ka.epb_bx * std::max(fx_layB.team_doubles, ka.layBx.team_doubles) * 8);
   if ((e = sse_set_smem_limits(ka, smA, smB)) != cudaSuccess) return cuda_fail(s, e, "cudaFuncSetAttribute");
 
   // the weight-adjusted mass operator V' diag(J^-1 W) V of every element,
@@ -1183,11 +1176,6 @@ int build(sse_solver *s, const sse_config *cfg, const sse_operators *ops, const 
   if (ka.fx.vp_ij && (rc = setup_fx_sums(s, fx_lists))) return rc;
   if (ka.fx.vp_ij && (rc = setup_fx_geometry(s))) return rc;
   if (ka.fx.T && (rc = setup_fx_mass(s))) return rc;
-  if (ka.fx.on) {
-    ka.layB = fx_layB;
-    ka.fd_chunk = fx_fd_chunk;
-    ka.vp_split = 0;
-  }
   return setup_compact(s, ops, mapP);
 }
 

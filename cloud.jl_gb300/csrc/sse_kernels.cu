@@ -14,6 +14,7 @@
 // Phase B  fd_time_derivative_kernel   time_derivative! FD (flux_differencing_form.jl:294-347)
 //          std_time_derivative_kernel  time_derivative! StandardForm (standard_form_first_order.jl:16-63)
 #include <algorithm>
+#include <type_traits>
 
 #include "sse_device.cuh"
 #include "sse_kernels.cuh"
@@ -803,35 +804,41 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // fluxes).
 // ---------------------------------------------------------------------------
 
-// Each node's sum of its pairs' contributions (at diff + NC pair), shifted to
-// the node's unit, handed to sink(node, sums).  A list longer than the others is
-// summed by two or four adjacent lanes (a p = 4 tet's facet lists have 5 entries
-// but 25 on the collapsed face: 13 steps instead of 25; 24,576 tets 2.52 ->
-// 2.42 ms, 7,986 p = 5 tets 2.05 -> 1.92 ms).
-template <int NC, typename Sink>
-__device__ __forceinline__ void fx_node_sums(const FxTables::Sums &S, int c, const long long *diff, const signed char *ns,
-                                             int lane, int tpe, Sink sink) {
+// Each node's sum of its pairs' contributions (at diff + NC pair), integers
+// shifted to the node's unit or FP64 values, handed to sink(node, sums).  A list
+// longer than the others is summed by two or four adjacent lanes (a p = 4 tet's
+// facet lists have 5 entries but 25 on the collapsed face: 13 steps instead of
+// 25; 24,576 tets 2.52 -> 2.42 ms, 7,986 p = 5 tets 2.05 -> 1.92 ms).
+template <int NC, typename T, typename Sink>
+__device__ __forceinline__ void fx_node_sums(const FxTables::Sums &S, int c, const T *diff, const signed char *ns, int lane,
+                                             int tpe, Sink sink) {
+  constexpr bool fixed = !std::is_same<T, double>::value;
   for (int t = lane; t < S.tasks; t += tpe) {
     const int2 task = S.task[(size_t)c * S.tasks + t];
     const int node = task.y & 0xffff, len = (task.y >> 16) & 0xfff, g = task.y >> 28;
-    const int n = ns[node];
-    long long acc[NC];
+    const int n = fixed ? ns[node] : 0;
+    T acc[NC];
 #pragma unroll
     for (int e = 0; e < NC; ++e) acc[e] = 0;
 #pragma unroll 2
     for (int q = task.x; q < task.x + len; ++q) {
       const int inc = S.inc[q];
-      const FxShift down((inc >> 1 & 127) - n);
-      const long long *dp = diff + (size_t)(inc >> 8) * NC;
+      const T *dp = diff + (size_t)(inc >> 8) * NC;
+      if constexpr (fixed) {
+        const FxShift down((inc >> 1 & 127) - n);
 #pragma unroll
-      for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
+        for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -down(dp[e]) : down(dp[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) acc[e] += (inc & 1) ? -dp[e] : dp[e];
+      }
     }
     if (__any_sync(0xffffffffu, g > 0)) {
 #pragma unroll
       for (int o = 1; o <= 2; o <<= 1)
 #pragma unroll
         for (int e = 0; e < NC; ++e) {
-          const long long other = __shfl_xor_sync(0xffffffffu, acc[e], o);
+          const T other = __shfl_xor_sync(0xffffffffu, acc[e], o);
           if (g > o >> 1) acc[e] += other;
         }
     }
@@ -949,13 +956,93 @@ __device__ __forceinline__ void fx_tail(const FxArgs &ka, const long long *rqi, 
   }
 }
 
-// the FP64 passes for a block that leaves the fixed-point ones: out of line, so
-// that their registers are not the kernel's
+// The FP64 passes of a block that leaves the fixed-point ones, in their chunks
+// and node lists and on the node values they started from; f_f holds the Lax-
+// Friedrichs term.  Out of line, so that their registers are not the kernel's,
+// and for this flux alone: the 80 registers of the kernel hold it without spills
+// (fd_fluxes with its other fluxes spilled 624 bytes).  With every block out of
+// range, against fd_time_derivative_kernel: 24,576 p = 4 tets 8.38 ms (9.07),
+// 7,986 p = 5 tets 6.42 (7.23), 13,182 p = 2 tets 0.99 (1.02), 8,192 p = 4 triangles
+// 0.366 (0.379); 10,368 p = 3 tets 1.78 (1.70) and 1,458 p = 3 triangles 0.065
+// (0.059), where the node values of the range test weigh most.
 template <int D, int NC>
-__device__ __noinline__ void fd_fp64(const KernelArgs &ka, double *base, int kk, bool live, int lane, int tpe) {
-  const Layout &L = ka.layB;
-  fd_fluxes<D, NC>(ka, base, kk, lane, tpe);
-  fd_tail<D, NC>(ka, base + L.off[3], base + L.off[2], base + L.off[4], kk, live, lane, tpe);
+__device__ __noinline__ void fd_fp64(const FxArgs &ka, double *ff, double *rq, double *diff, double *node, int kk, bool live,
+                                     int lane, int tpe) {
+  const DevOps &op = ka.op;
+  const Physics &ph = ka.ph;
+  const FxTables &fx = ka.fx;
+  constexpr int PS = kFxStride<D>;
+  const int nq = op.nq, nf = op.nf, nfac = op.nfac, CH = ka.fx_chunk;
+  const float rnpf = qrcp(op.npf > 0 ? op.npf : 1);
+  const double *Lam = ka.geo.Lambda_q + (size_t)kk * nq * D * D, *hnq = ka.geo.halfnJq + (size_t)kk * D * nfac * nq,
+               *hnf = ka.geo.halfnJf + (size_t)kk * D * nf;
+  fx_prefetch(Lam, nq * D * D * sizeof(double), lane, tpe);
+  if (op.nfp > 0) fx_prefetch(hnq, D * nfac * nq * sizeof(double), lane, tpe);
+  fx_prefetch(hnf, D * nf * sizeof(double), lane, tpe);
+  // [rho, p, beta, V]
+  for (int i = lane; i < nq + 2 * nf; i += tpe) node[(size_t)i * PS + 2] = node[(size_t)i * PS] * sse_rcp(node[(size_t)i * PS + 1]);
+  __syncthreads();
+  for (int c = 0; c < fx.vol.chunks; ++c) {
+    const int c0 = c * CH, c1 = min(op.nvp, c0 + CH);
+    for (int p = c0 + lane; p < c1; p += tpe) {
+      const int ij = fx.vp_ij[p], i = ij & 0xffff, j = ij >> 16;
+      const double *S = fx.vp_Sh + (size_t)p * D;
+      double G[D];
+#pragma unroll
+      for (int n = 0; n < D; ++n) G[n] = 0.0;
+#pragma unroll
+      for (int m = 0; m < D; ++m) {
+        if (S[m] == 0.0) continue;
+#pragma unroll
+        for (int n = 0; n < D; ++n) G[n] = fma(S[m], Lam[i + nq * (m + D * n)] + Lam[j + nq * (m + D * n)], G[n]);
+      }
+      ec_flux_dot_half<D>(ph.igm1, ph.ilm_q, node + (size_t)i * PS, node + (size_t)j * PS, G, diff + (size_t)(p - c0) * NC);
+    }
+    __syncthreads();
+    fx_node_sums<NC>(fx.vol, c, diff - (size_t)c0 * NC, nullptr, lane, tpe, [&](int i, const double *acc) {
+#pragma unroll
+      for (int e = 0; e < NC; ++e) rq[e * nq + i] = c == 0 ? acc[e] : rq[e * nq + i] + acc[e];
+    });
+    __syncthreads();
+  }
+  const int nall = op.nfp + nf;
+  for (int c = 0; c < fx.fac.chunks; ++c) {
+    const int c0 = c * CH, c1 = min(nall, c0 + CH);
+    for (int p = c0 + lane; p < c1; p += tpe) {
+      double G[D];
+      int i, j;
+      if (p < op.nfp) {
+        const int ij = op.fp_ij[p], jf = ij >> 16, f = qdiv(jf, rnpf);
+        i = ij & 0xffff;
+        j = nq + jf;
+        const double C = op.fp_Ch[p];
+#pragma unroll
+        for (int m = 0; m < D; ++m) G[m] = C * (hnf[m + D * jf] + hnq[m + D * (f + nfac * i)]);
+      } else {
+        i = nq + p - op.nfp;
+        j = i + nf;
+        const double b = 0.5 * ka.geo.BJf[(size_t)kk * nf + i - nq];
+#pragma unroll
+        for (int m = 0; m < D; ++m) G[m] = b * ka.geo.n_f[m + D * ((i - nq) + (size_t)nf * kk)];
+      }
+      ec_flux_dot_half<D>(ph.igm1, ph.ilm_q, node + (size_t)i * PS, node + (size_t)j * PS, G, diff + (size_t)(p - c0) * NC);
+    }
+    __syncthreads();
+    fx_node_sums<NC>(fx.fac, c, diff - (size_t)c0 * NC, nullptr, lane, tpe, [&](int t, const double *acc) {
+      if (t < nq) {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) rq[e * nq + t] -= acc[e];
+      } else {
+        const int r = t - nq, p = op.nfp + r;
+        const bool own = p >= c0 && p < c1;
+        const double *dp = diff + (size_t)(own ? p - c0 : 0) * NC;
+#pragma unroll
+        for (int e = 0; e < NC; ++e) ff[e * nf + r] += (own ? dp[e] : 0.0) - acc[e];
+      }
+    });
+    __syncthreads();
+  }
+  fd_tail<D, NC>(ka, rq, ff, diff, kk, live, lane, tpe);
 }
 
 template <int D, int NC, int P1>
@@ -1075,7 +1162,7 @@ __global__ void __launch_bounds__(256, 3) fd_time_derivative_fx_kernel(const __g
   const FxScale sc(key, eG, ph.nflux == 0 && ph.half_lambda > 1e-6);
   // a block with an element out of range runs in FP64 as a whole
   if (!__syncthreads_and(sc.ok)) {
-    fd_fp64<D, NC>(ka, smem + (size_t)team * ka.layB.team_doubles, kk, live, lane, tpe);
+    fd_fp64<D, NC>(ka, ff, rq, reinterpret_cast<double *>(diff), noded, kk, live, lane, tpe);
     return;
   }
   const int kappa = sc.eH - 2 * sc.eV, eP = sc.eR + sc.eH - 2;
@@ -2401,7 +2488,7 @@ cudaError_t sse_set_smem_limits(const FxArgs &ka, size_t smA, size_t smB) {
     if (!ka.fd) set((const void *)std_time_derivative_kernel<D, NC>, smB);
   });
   if (ka.fx.T) set(fx_kernel_a(ka), (size_t)ka.epb_ax * ka.layAx.team_doubles * sizeof(double));
-  if (ka.fx.vp_ij) set(fx_kernel_b(ka), smB);
+  if (ka.fx.vp_ij) set(fx_kernel_b(ka), (size_t)ka.epb_bx * ka.layBx.team_doubles * sizeof(double));
   return e;
 }
 
@@ -2522,7 +2609,7 @@ cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st) {
     FxArgs kx = ka;
     kx.epb = ka.epb_bx;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;
-    sm = (size_t)kx.epb * std::max(ka.layB.team_doubles, ka.layBx.team_doubles) * sizeof(double);
+    sm = (size_t)kx.epb * ka.layBx.team_doubles * sizeof(double);
     void *args[] = {&kx};
     return cudaLaunchKernel(fx_kernel_b(ka), dim3(gridx), dim3(ka.tpb_bx), args, sm, st);
   } else if (ka.fd) {

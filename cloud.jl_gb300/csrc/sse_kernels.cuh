@@ -34,6 +34,7 @@ struct Layout {
 struct FxTables {
   int on;             // 0: no fixed-point tables, phase B runs in FP64
   const int *vp_ij;   // i | j << 16
+  const double *vp_Sh;  // nvp x d: S / 2
   const Fx *vp_S;     // nvp x d: S / 2 in units 2^(eS - k)
   const Fx *fp_C;     // C / 2 in units 2^(eC - k)
   // Node sums of the volume pairs, and of the facet-correction pairs (followed
