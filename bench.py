@@ -608,18 +608,18 @@ def main():
     kernel_B = "fd_time_derivative_kernel" if fd else (
         "std_compact_kernel" if one_kernel else "std_time_derivative_kernel")
     traffic = TRAFFIC_PER_ELEMENT.get(args.workload) if not (args.cells or args.p) else None
-    # the entropy-conservative Euler pair passes are integer multiply-adds: the
-    # FP64 peak does not bound them, HBM is the only roof left
-    fixed_point = (fd and host.cfg.law == pkg.abi.SSE_EULER and host.cfg.two_point_flux == pkg.abi.SSE_EC_FLUX
-                   and host.cfg.gamma <= 1.7)
+    # a fixed-point phase is integer multiply-adds, which the FP64 peak does not
+    # bound: instruction issue and latency do, and the fraction given is HBM's
+    fixed_point = gpu.fixed_point_phases() & (pkg.abi.SSE_FIXED_POINT_B if dom == "B" else pkg.abi.SSE_FIXED_POINT_A) != 0
+    kernel = kernel_B if dom == "B" else "nodal_values_kernel"
     dom_gbs = dom_bytes / (dom_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm" if fixed_point else "fp64", "achieved": dom_gbs if fixed_point else achieved,
+    roofline = {"bound": "issue and latency" if fixed_point else "fp64", "achieved": dom_gbs if fixed_point else achieved,
                 "peak": hbm_peak if fixed_point else fp64_peak, "unit": "GB/s" if fixed_point else "TFLOP/s",
                 "frac": dom_gbs / hbm_peak if fixed_point else achieved / fp64_peak,
-                "kernel": (kernel_B if dom == "B" else "nodal_values_kernel").replace(
-                    "_kernel", "_fx_kernel" if fixed_point else "_kernel"),
+                "kernel": kernel.replace("_kernel", "_fx_kernel") if fixed_point else kernel,
                 "fp64_equivalent_tflops": achieved, "fp64_peak_tflops": fp64_peak,
-                "peak_source": "measured live: FP64 FMA-chain microbenchmark on this GPU",
+                "peak_source": ("MEASURED_PEAKS.json: device copy" if peaks else "fallback copy rate") if fixed_point
+                else "measured live: FP64 FMA-chain microbenchmark on this GPU",
                 "hbm_achieved_gbs": dom_gbs,
                 "hbm_frac_of_measured": dom_gbs / hbm_peak,
                 "traffic": traffic[dom] * ne if traffic else None,

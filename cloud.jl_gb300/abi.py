@@ -32,6 +32,9 @@ SSE_FP64 = 0
 SSE_MIXED = 1
 SSE_PATH_TWO_PHASE = 0
 SSE_PATH_ONE_KERNEL = 1
+
+SSE_FIXED_POINT_A = 1
+SSE_FIXED_POINT_B = 2
 SSE_HOST = 0
 SSE_DEVICE = 1
 SSE_CARPENTER_KENNEDY_2N54 = 0

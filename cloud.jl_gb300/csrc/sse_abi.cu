@@ -2756,6 +2756,11 @@ int32_t sse_kernel_path(const sse_solver *s) {
   return s->ka.compact ? SSE_PATH_ONE_KERNEL : SSE_PATH_TWO_PHASE;
 }
 
+int32_t sse_fixed_point_phases(const sse_solver *s) {
+  if (!s) return SSE_ERR_INVALID_ARGUMENT;
+  return (s->ka.fx.on_a ? SSE_FIXED_POINT_A : 0) + (s->ka.fx.on ? SSE_FIXED_POINT_B : 0);
+}
+
 int32_t sse_set_kernel_path(sse_solver *s, int32_t path) {
   if (!s) return SSE_ERR_INVALID_ARGUMENT;
   if (path == SSE_PATH_TWO_PHASE) {

@@ -28,7 +28,8 @@ EXPORTED = ["sse_abi_version", "sse_create", "sse_destroy", "sse_residual",
             "sse_conservation_residual", "sse_set_precision", "sse_set_stream",
             "sse_phase_timings", "sse_struct_sizes", "sse_measure_fma_peaks", "sse_last_error",
             "sse_create_error", "sse_geometric_factors", "sse_project_function",
-            "sse_energy_residual", "sse_kernel_path", "sse_set_kernel_path"]
+            "sse_energy_residual", "sse_kernel_path", "sse_set_kernel_path",
+            "sse_fixed_point_phases"]
 
 _lib = None
 
@@ -86,6 +87,8 @@ def load_library(path: str | None = None):
     L.sse_phase_timings.restype = i32
     L.sse_kernel_path.argtypes = [vp]
     L.sse_kernel_path.restype = i32
+    L.sse_fixed_point_phases.argtypes = [vp]
+    L.sse_fixed_point_phases.restype = i32
     L.sse_set_kernel_path.argtypes = [vp, i32]
     L.sse_set_kernel_path.restype = i32
     L.sse_measure_fma_peaks.argtypes = [vp]
@@ -265,6 +268,13 @@ class GB300Solver:
     def kernel_path(self) -> int:
         """SSE_PATH_TWO_PHASE or SSE_PATH_ONE_KERNEL (sse_kernel_path)."""
         r = self.L.sse_kernel_path(self.h)
+        if r < 0:
+            self._check(r)
+        return r
+
+    def fixed_point_phases(self) -> int:
+        """Sum of SSE_FIXED_POINT_A and SSE_FIXED_POINT_B (sse_fixed_point_phases)."""
+        r = self.L.sse_fixed_point_phases(self.h)
         if r < 0:
             self._check(r)
         return r

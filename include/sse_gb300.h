@@ -348,6 +348,12 @@ int32_t sse_kernel_path(const sse_solver *s);
  * outside its scope; the handle's path is then unchanged. */
 int32_t sse_set_kernel_path(sse_solver *s, int32_t path);
 
+/* Which phases of the FP64 residual run the fixed-point kernels on this handle
+ * (see sse_create): a sum of SSE_FIXED_POINT_A and SSE_FIXED_POINT_B, negative:
+ * error.  No counterpart in the reference. */
+enum sse_fixed_point_phase { SSE_FIXED_POINT_A = 1, SSE_FIXED_POINT_B = 2 };
+int32_t sse_fixed_point_phases(const sse_solver *s);
+
 /* ---- Geometric factors on the device -------------------------------------
  *
  * Drop-in for the constructor GeometricFactors(mesh, reference_element,

@@ -42,3 +42,29 @@ def test_blocks_out_of_range(gpu_lib, shape, p, cells, basis, most):
     scale = np.abs(before).max(axis=(0, 2))
     for e in changed:
         assert np.all(np.abs(after[e] - before[e]).max(axis=1) <= 1.0e-12 * scale)
+
+
+def _phases(basis="ModalTensor", shape="Tet", aspect=1.0, form=None, law=None, multi=False):
+    d = 2 if shape == "Tri" else 3
+    if multi:
+        sd = cases._disc_multi(basis, shape, 3, 2, 2 * np.pi, 0.05, "ChanWilcox")
+    else:
+        ra = cases.R.reference_approximation(basis, shape, 3, mapping_degree=3)
+        box = (2 * np.pi,) * (d - 1) + (2 * np.pi / aspect,)
+        mesh = cases.M.uniform_periodic_mesh(ra, tuple((0.0, L) for L in box), (2,) * d)
+        sd = cases.M.spatial_discretization(cases.M.warp_mesh(mesh, ra, "Chan", 0.05, box), ra, metrics="ChanWilcox")
+    form = form or S.FluxDifferencingForm(inviscid_numerical_flux=S.LaxFriedrichsNumericalFlux())
+    return cases.PKG.GB300Solver(S.HostArrays(law or S.EulerEquations(d, 1.4), sd, form)).fixed_point_phases()
+
+
+def test_reported_phases(gpu_lib):
+    """What a handle says of its phases: A needs a modal tensor-product basis, B the
+    entropy-conservative flux, gamma of at most 1.7 and elements not stretched."""
+    A, B = cases.PKG.abi.SSE_FIXED_POINT_A, cases.PKG.abi.SSE_FIXED_POINT_B
+    lf = S.LaxFriedrichsNumericalFlux()
+    assert _phases() == _phases(shape="Tri") == A + B
+    assert _phases("NodalTensor") == _phases("ModalMulti", multi=True) == B
+    assert _phases(aspect=1.0e3) == A
+    assert _phases(law=S.EulerEquations(3, 2.0)) == 0
+    assert _phases(form=S.StandardForm(inviscid_numerical_flux=lf)) == 0
+    assert _phases(form=S.FluxDifferencingForm(inviscid_numerical_flux=lf, two_point_flux=S.ChandrashekarFlux())) == 0
