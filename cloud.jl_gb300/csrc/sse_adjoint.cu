@@ -1320,8 +1320,7 @@ cudaError_t sse_set_smem_limits_adjoint(const KernelArgs &ka) {
   cudaError_t e = cudaSuccess;
   auto set = [&](const void *f, const Layout &L) {
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)((size_t)ka.epb * L.team_doubles * sizeof(double)));
+      e = raise_smem_limit(f, (size_t)ka.epb * L.team_doubles * sizeof(double));
   };
   if (!ka.fd) {
 #define SSE_STD_ADJ_LIMITS(DD, NN)                                  \
@@ -1371,8 +1370,7 @@ cudaError_t sse_set_smem_limits_adjoint_mixed(const KernelArgs &ka) {
   cudaError_t e = cudaSuccess;
   auto set = [&](const void *f, const Layout &L) {
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)((size_t)ka.epb * L.team_doubles * sizeof(float)));
+      e = raise_smem_limit(f, (size_t)ka.epb * L.team_doubles * sizeof(float));
   };
   if (ka.op.d == 2 && ka.op.nc == 4) {
     set((const void *)adj_lift_mixed_kernel<2, 4>, ka.layAdjB1m);

@@ -369,8 +369,7 @@ __global__ void __launch_bounds__(128) dense_vdm_kernel(KernelArgs ka, double *o
 
 cudaError_t sse_set_smem_limit_compact(const KernelArgs &ka, size_t bytes) {
   cudaError_t e = cudaSuccess;
-  SSE_COMPACT_DISPATCH((e = cudaFuncSetAttribute((const void *)std_compact_kernel<D, NC>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)));
+  SSE_COMPACT_DISPATCH((e = raise_smem_limit((const void *)std_compact_kernel<D, NC>, bytes)));
   return e;
 }
 
@@ -385,14 +384,10 @@ cudaError_t launch_dense_vdm(const KernelArgs &ka, double *out, cudaStream_t s) 
   const size_t sm = (size_t)ka.layA.team_doubles * sizeof(double);
   cudaError_t e;
   if (ka.op.d == 2) {
-    if ((e = cudaFuncSetAttribute((const void *)dense_vdm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm)))
-      return e;
+    if ((e = raise_smem_limit((const void *)dense_vdm_kernel<2>, sm))) return e;
     dense_vdm_kernel<2><<<ka.op.np, 128, sm, s>>>(ka, out);
   } else {
-    if ((e = cudaFuncSetAttribute((const void *)dense_vdm_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm)))
-      return e;
+    if ((e = raise_smem_limit((const void *)dense_vdm_kernel<3>, sm))) return e;
     dense_vdm_kernel<3><<<ka.op.np, 128, sm, s>>>(ka, out);
   }
   return cudaGetLastError();

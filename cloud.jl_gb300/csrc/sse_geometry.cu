@@ -634,17 +634,17 @@ int geometric_factors_run(const sse_metric_operators *ops, int64_t n_e, const do
   const dim3 grid((unsigned)n_e);
   if (ops->metrics == SSE_EXACT_METRICS) {
     if (d == 2) {
-      cudaFuncSetAttribute(exact_metrics_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_smem_limit((const void *)exact_metrics_kernel<2>, smem);
       exact_metrics_kernel<2><<<grid, threads, smem>>>(g);
     } else {
-      cudaFuncSetAttribute(exact_metrics_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_smem_limit((const void *)exact_metrics_kernel<3>, smem);
       exact_metrics_kernel<3><<<grid, threads, smem>>>(g);
     }
   } else if (d == 2) {
-    cudaFuncSetAttribute(curl_metrics_2d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit((const void *)curl_metrics_2d_kernel, smem);
     curl_metrics_2d_kernel<<<grid, threads, smem>>>(g);
   } else {
-    cudaFuncSetAttribute(curl_metrics_3d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit((const void *)curl_metrics_3d_kernel, smem);
     curl_metrics_3d_kernel<<<grid, threads, smem>>>(g);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda(e, "metric kernel launch");

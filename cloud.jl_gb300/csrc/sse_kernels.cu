@@ -14,6 +14,7 @@
 // Phase B  fd_time_derivative_kernel   time_derivative! FD (flux_differencing_form.jl:294-347)
 //          std_time_derivative_kernel  time_derivative! StandardForm (standard_form_first_order.jl:16-63)
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "sse_device.cuh"
@@ -2476,10 +2477,19 @@ static const void *fx_kernel(const FxArgs &ka, bool a, int p1) {
 static const void *fx_kernel_a(const FxArgs &ka) { return fx_kernel(ka, true, ka.fx.p1_a); }
 static const void *fx_kernel_b(const FxArgs &ka) { return fx_kernel(ka, false, ka.fx.p1_b); }
 
+cudaError_t raise_smem_limit(const void *kernel, size_t bytes) {
+  static std::mutex mutex;  // between the query and the setting
+  std::lock_guard<std::mutex> lock(mutex);
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 cudaError_t sse_set_smem_limits(const FxArgs &ka, size_t smA, size_t smB) {
   cudaError_t e = cudaSuccess;
   auto set = [&](const void *f, size_t bytes) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) e = raise_smem_limit(f, bytes);
   };
   SSE_DISPATCH(D, NC, {
     set((const void *)nodal_values_kernel<D, NC>, smA);
@@ -2539,18 +2549,15 @@ cudaError_t sse_set_smem_limits_mixed_a(const KernelArgs &ka) {
   const int am = (int)((size_t)ka.epb_am * ka.layAm.team_doubles * sizeof(double));
   const int p1 = (int)((size_t)ka.epb * ka.layP1.team_doubles * sizeof(double));
   if (ka.op.d == 2 && ka.op.nc == 4) {
-    e = cudaFuncSetAttribute((const void *)nodal_values_mixed_kernel<2, 4>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, am);
+    e = raise_smem_limit((const void *)nodal_values_mixed_kernel<2, 4>, am);
   } else if (ka.op.d == 3 && ka.op.nc == 5) {
-    e = cudaFuncSetAttribute((const void *)nodal_values_mixed_kernel<3, 5>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, am);
+    e = raise_smem_limit((const void *)nodal_values_mixed_kernel<3, 5>, am);
   } else {
     return cudaErrorInvalidValue;
   }
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ka.op.d == 2 ? (const void *)projection_of_one_kernel<2>
-                                          : (const void *)projection_of_one_kernel<3>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, p1);
+    e = raise_smem_limit(ka.op.d == 2 ? (const void *)projection_of_one_kernel<2>
+                                      : (const void *)projection_of_one_kernel<3>, p1);
   return e;
 }
 
@@ -2570,7 +2577,7 @@ static const void *mixed_b_kernel(const KernelArgs &ka) {
 cudaError_t sse_mixed_b_blocks_per_sm(const KernelArgs &ka, size_t smBm, int *blocks) {
   const void *f = mixed_b_kernel(ka);
   if (!f) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  cudaError_t e = raise_smem_limit(f, 220 * 1024);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, f, ka.tpb, smBm);
 }
@@ -2578,7 +2585,7 @@ cudaError_t sse_mixed_b_blocks_per_sm(const KernelArgs &ka, size_t smBm, int *bl
 cudaError_t sse_set_smem_limit_mixed(const KernelArgs &ka, size_t smBm) {
   const void *f = mixed_b_kernel(ka);
   if (!f) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smBm);
+  return raise_smem_limit(f, smBm);
 }
 
 cudaError_t launch_time_derivative(const FxArgs &ka, cudaStream_t st) {
@@ -2625,7 +2632,7 @@ cudaError_t launch_fx_geometry(const FxArgs &ka, Fx *Lam, Fx *hnq, Fx *hnf, Fx *
   const size_t sm = fx_geometry_smem(ka);
   const int tpb = std::min(256, (ka.op.nq + ka.op.nf + 31) / 32 * 32);
   auto *kernel = ka.op.d == 2 ? fx_geometry_kernel<2> : fx_geometry_kernel<3>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = raise_smem_limit((const void *)kernel, sm);
   if (e != cudaSuccess) return e;
   kernel<<<ka.ne, tpb, sm, st>>>(ka, Lam, hnq, hnf, bn, n, eG, none);
   return cudaGetLastError();
@@ -2640,8 +2647,7 @@ cudaError_t launch_mass_operator(const KernelArgs &ka, double *Ak, cudaStream_t 
   int grid = (ka.ne + ka.epb - 1) / ka.epb;
   size_t sm = (size_t)ka.epb * ka.layA.team_doubles * sizeof(double);
   cudaError_t e = cudaSuccess;
-  SSE_DISPATCH(D, NC, (e = cudaFuncSetAttribute(mass_operator_kernel<D, NC>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
+  SSE_DISPATCH(D, NC, (e = raise_smem_limit((const void *)mass_operator_kernel<D, NC>, sm)));
   if (e != cudaSuccess) return e;
   SSE_DISPATCH(D, NC, (mass_operator_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka, Ak)));
   return cudaGetLastError();
@@ -2652,8 +2658,7 @@ cudaError_t launch_energy(const KernelArgs &ka, const double *u, const double *d
   int grid = (ka.ne + ka.epb - 1) / ka.epb;
   size_t sm = (size_t)ka.epb * ka.layE.team_doubles * sizeof(double);
   cudaError_t e = cudaSuccess;
-  SSE_DISPATCH(D, NC, (e = cudaFuncSetAttribute(energy_kernel<D, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sm)));
+  SSE_DISPATCH(D, NC, (e = raise_smem_limit((const void *)energy_kernel<D, NC>, sm)));
   if (e != cudaSuccess) return e;
   SSE_DISPATCH(D, NC, (energy_kernel<D, NC><<<grid, ka.tpb, sm, st>>>(ka, u, dudt, partial)));
   return cudaGetLastError();
@@ -2783,8 +2788,7 @@ cudaError_t launch_tail_operators(const KernelArgs &ka, const double *Vd, double
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const size_t sm = (size_t)np * np * sizeof(double);
-  if ((e = cudaFuncSetAttribute((const void *)tail_operator_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sm)))
+  if ((e = raise_smem_limit((const void *)tail_operator_kernel, sm)))
     return e;
   tail_operator_kernel<<<ka.ne, 256, sm, st>>>(ka.Ak, M, reinterpret_cast<float4 *>(E), np, quads);
   return cudaGetLastError();

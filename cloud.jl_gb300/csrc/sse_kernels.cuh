@@ -192,6 +192,10 @@ struct CompactStage {
   double *out;
 };
 
+// Let a kernel have `bytes` of dynamic shared memory.  The limit belongs to the
+// kernel and not to a handle: it is only ever raised, so that the launches of
+// larger elements' handles still fit after a smaller one is created.
+cudaError_t raise_smem_limit(const void *kernel, size_t bytes);
 cudaError_t sse_set_smem_limits(const FxArgs &ka, size_t smA, size_t smB);
 cudaError_t sse_set_smem_limit_compact(const KernelArgs &ka, size_t bytes);
 cudaError_t launch_std_compact(const KernelArgs &ka, const CompactStage &st, cudaStream_t s);

@@ -243,7 +243,7 @@ int project_function_run(int np, int nq, int nc, int64_t ne, const double *V, co
     a.u0 = d + n_j + n_u;
   }
   auto *kernel = staged ? project_function_kernel<true> : project_function_kernel<false>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void *)kernel, smem);
   kernel<<<(unsigned)((ne + epb - 1) / epb), kThreads, smem>>>(a);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda(e, "projection kernel launch");
   if ((e = cudaDeviceSynchronize()) != cudaSuccess) return cuda(e, "projection kernel");
