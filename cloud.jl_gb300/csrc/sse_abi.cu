@@ -549,6 +549,16 @@ int setup_fx_mass(sse_solver *s) {
   ka.fx.eA = eA;
   ka.fx.eW = eW;
   ka.fx.on_a = 1;
+  // Where neither the FP64 pipe nor the SMs are full, phase A is its own chain,
+  // and the fixed-point one is longer at the lowest degrees, and on triangles of
+  // degree 7, where many short steps meet sizes taken from the operators: FP64 up
+  // to 30,000 nodes (p = 1 triangles: 512 21.6 us against 25.4, 1,458 27.1 / 28.1,
+  // 3,200 35.0 / 32.7; p = 2: 512 23.5 / 26.0, 1,458 29.4 / 31.9, 3,200 37.7 / 37.9; p
+  // = 1 tets: 162 27.4 / 34.2, 750 32.9 / 33.8, 3,072 70.9 / 46.2).  At the other
+  // degrees fixed point is at least as fast at any size.
+  const int p1 = ka.op.p1;
+  const bool short_chain = c.d == 2 ? p1 > 3 && p1 < 8 : p1 > 2;
+  ka.fx.run_a = short_chain || ne * (size_t)(c.n_q + c.n_f) > 30000;
   return SSE_OK;
 }
 
@@ -2807,7 +2817,7 @@ int32_t sse_kernel_path(const sse_solver *s) {
 
 int32_t sse_fixed_point_phases(const sse_solver *s) {
   if (!s) return SSE_ERR_INVALID_ARGUMENT;
-  return (s->ka.fx.on_a ? SSE_FIXED_POINT_A : 0) + (s->ka.fx.on ? SSE_FIXED_POINT_B : 0);
+  return (s->ka.fx.run_a ? SSE_FIXED_POINT_A : 0) + (s->ka.fx.on ? SSE_FIXED_POINT_B : 0);
 }
 
 int32_t sse_set_kernel_path(sse_solver *s, int32_t path) {

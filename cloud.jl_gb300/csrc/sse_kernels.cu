@@ -2516,9 +2516,9 @@ cudaError_t launch_nodal_values(const FxArgs &ka, cudaStream_t st) {
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
   }
-  // the fixed-point operators wherever their tables exist (EC flux, modal
-  // tensor-product basis)
-  if (ka.fx.on_a) {
+  // the fixed-point operators where their tables exist (EC flux, modal tensor-
+  // product basis) and the mesh is not too small for them
+  if (ka.fx.run_a) {
     FxArgs kx = ka;
     kx.epb = ka.epb_ax;
     const int gridx = (ka.ne + kx.epb - 1) / kx.epb;

@@ -60,7 +60,8 @@ struct FxTables {
   // scaled per node (2^K_i) and mode (2^T_l); R times 2^-K_q, row j in units
   // 2^eR_j (absolute row sums at most 1; CSR values); the mass operators in
   // units 2^eA (absolute row sums at most 1) and 2^eW > sum of W J 2^-K
-  int on_a;
+  int on_a;           // the tables are there (phase B's tail reads them too)
+  int run_a;          // phase A runs on them
   const Fx *A, *B, *C, *R, *A_k;
   const signed char *T, *K, *eR;
   const int *eA, *eW;

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import cases
+from oracle.oracle import Oracle, rel2
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +69,26 @@ def test_reported_phases(gpu_lib):
     assert _phases(law=S.EulerEquations(3, 2.0)) == 0
     assert _phases(form=S.StandardForm(inviscid_numerical_flux=lf)) == 0
     assert _phases(form=S.FluxDifferencingForm(inviscid_numerical_flux=lf, two_point_flux=S.ChandrashekarFlux())) == 0
+
+
+@pytest.mark.parametrize("shape,p,fp64,fixed", [("Tri", 1, 38, 39), ("Tri", 2, 28, 29), ("Tri", 7, 13, 14), ("Tet", 1, 5, 6),
+                                                ("Tri", 3, None, 2), ("Tet", 2, None, 1)])
+def test_size_where_phase_a_turns_to_fixed_point(gpu_lib, shape, p, fp64, fixed):
+    """The meshes (cells a side) on both sides of the line, or the smallest where
+    there is none: the phase that runs, and its nodal values to the parity
+    tolerance."""
+    d = 2 if shape == "Tri" else 3
+    for cells, want in ((fp64, 0), (fixed, cases.PKG.abi.SSE_FIXED_POINT_A)):
+        if cells is None:
+            continue
+        sd = cases._disc("ModalTensor", shape, p, cells, 2 * np.pi, 0.05, "ChanWilcox")
+        host = S.HostArrays(S.EulerEquations(d, 1.4), sd,
+                            S.FluxDifferencingForm(inviscid_numerical_flux=S.LaxFriedrichsNumericalFlux()))
+        rng = np.random.default_rng(cells)
+        u = np.zeros((host.N_e, host.N_c, host.N_p))
+        u[:, 0, 0], u[:, 1, 0], u[:, -1, 0] = 1.0, 0.3, 2.5
+        u += 1.0e-3 * rng.standard_normal(u.shape)
+        solver = cases.PKG.GB300Solver(host)
+        assert solver.fixed_point_phases() & cases.PKG.abi.SSE_FIXED_POINT_A == want
+        for got, ref in zip(solver.nodal_values(u), Oracle(host).nodal_values(u)):
+            assert rel2(got, ref) <= 1.0e-12
