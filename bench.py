@@ -88,9 +88,9 @@ WORKLOADS = {
 
 # DRAM bytes (read + write) per element of one fd_time_derivative_fx_kernel<3,5,5>
 # / nodal_values_fx_kernel<3,5,5> launch at p = 4, from ncu captures of the same
-# kernels on the 8^3 x 6 = 3,072-tet case (154.3 MB and 37.9 MB per launch);
+# kernels on the 8^3 x 6 = 3,072-tet case (153.8 MB and 37.8 MB per launch);
 # reads scale with the element count
-TRAFFIC_PER_ELEMENT = {"tgv_p4": {"B": 50_235, "A": 12_335}}
+TRAFFIC_PER_ELEMENT = {"tgv_p4": {"B": 50_081, "A": 12_318}}
 
 
 def env_rank():

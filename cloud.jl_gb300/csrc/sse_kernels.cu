@@ -800,9 +800,10 @@ __global__ void __launch_bounds__(256) fd_time_derivative_kernel(KernelArgs ka) 
 // -> 0.276 ms; 8,192 p = 4 triangles 0.365 -> 0.117 ms.  The FP64 pipe is 18 %
 // busy and half the issue slots are taken; the rest is latency (barriers, loads
 // of metric terms).  The error against the extended-precision residual is 0.4
-// to 1.00 of the FP64 passes' own on 61
-// configurations (modal and nodal, p = 2 to 6, both metrics and interface
-// fluxes).
+// to 1.00 of the FP64 passes' own on 61 configurations (modal and nodal, p = 2 to
+// 6, both metrics and interface fluxes), by variable 0.2 to 0.7 (modal) and 0.3 to
+// 1.4 (nodal).  Blocks with an element that would lose more take fd_fp64: a range
+// beyond 2^4 (FxScale), stretched (kFxStretch).
 // ---------------------------------------------------------------------------
 
 // Each node's sum of its pairs' contributions (at diff + NC pair), integers

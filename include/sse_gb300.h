@@ -150,8 +150,12 @@ int32_t sse_abi_version(void);
  * metric terms and of the mass operators (8 bytes a value, the size of
  * Lambda_q, halfnJq, twice halfnJf and the mass operators; 36 KB per p = 4 tet),
  * again each when it takes at most a quarter of the free device memory; without
- * them the residual runs its FP64 kernels, as it does for a block of elements
- * whose densities or enthalpies span more than a factor of 16 in an element.
+ * them the residual runs its FP64 kernels.  So does a block of elements with one
+ * whose densities or enthalpies have exponents more than 4 apart (a factor of 16
+ * to 32), or that is stretched (columns of Lambda_q more than a factor of 8
+ * apart at a node), or, without a Lax-Friedrichs term, whose velocities are below
+ * 2^-23 of the speed of sound and not zero; and phase A on meshes of at most
+ * 30,000 nodes at p = 1 and on triangles of p = 2 and 7.
  * Replaces Solver(...) + the Threaded/Serial parallelism
  * tag (Solvers.jl:287-333, 429-452). */
 int32_t sse_create(const sse_config *cfg, const sse_operators *ops,
